@@ -394,7 +394,7 @@ void require_pair_index(Ctx* c, int64_t n) {
 }
 
 // Explicit tet pair batches of at least this many pairs run through the
-// early-out pass and the index clipper (work counters: misc ints 24-29).
+// early-out pass and the tet clipper (work counters: misc ints 24-29).
 constexpr int64_t kPairsPipelineMin = 2048;
 unsigned long long* pairs_work(Ctx* c) { return reinterpret_cast<unsigned long long*>(bad_flag(c) + 24); }
 

@@ -15,16 +15,18 @@
 //   K5  k_clip_tris     one candidate pair per thread, polygon in shared
 //                       memory, FP64 Sutherland-Hodgman
 //   K6  k_prefilter_tets two exact early-outs and the no-op plane mask;
-//                       k_clip_tets_ix depth-first clipping over point
-//                       indices with a refill pipeline, templated on what it
-//                       does with the kept tets (measures; explicit pairs'
-//                       output tets; the supermesh's tets at their offsets;
-//                       the P1 quadrature) and on the plane count (4: tets,
-//                       6: hexahedra)
+//                       k_clip_tets_bf breadth-first clipping, a warp per
+//                       batch of pairs, templated on what it does with the
+//                       kept tets (measures of small and medium passes;
+//                       explicit pairs' output tets; the supermesh's tets at
+//                       their offsets; the P1 quadrature);
+//                       k_clip_tets_ix depth-first clipping, a lane per pair,
+//                       over point indices with a refill pipeline (measures
+//                       of large passes; six planes: hexahedra)
 //   K7  compensated reductions (per-block (sum, err), then final; per mesh
 //                       pair for the batched path)
 //   K8  P1-P1 mixed mass blocks + u^T M v: 2D k_p1_mass; 3D the early-out
-//                       pass and k_clip_tets_ix with the quadrature sink;
+//                       pass and k_clip_tets_bf with the quadrature sink;
 //                       k_p2_inner  P2 inner product
 //   K9  1D sort finder  k_prep_1d, 64-bit stable sort, max segment tree,
 //                       k_rows_1d, k_sweep_1d, k_emit_1d;  k_clip_intervals
@@ -1583,7 +1585,20 @@ __host__ __device__ inline int64_t seg_per(int64_t npairs, int grid) {
   return ((npairs + grid - 1) / grid + 255) / 256 * 256;
 }
 
-template <bool kSettle, int NP = 4, bool kSeg = false>
+// Last word of a survivor record for k_clip_tets_bf (kCode; otherwise just the
+// no-op mask): the no-op mask in bits 0-3, then
+// the signs of A's vertices at B's planes (plane l, vertex v at bit 4 +
+// 4 (3-l) + 3-v, as the pass shifts them in), and in bit 30 whether some
+// distance is neither clearly positive nor clearly negative to the clipper
+// (|d| < eps, infinite or NaN; the clipper then classifies A itself).  irr is
+// the largest 2 * (high word of |d|) - 2 * kEpsHi, modulo 2^32: it reaches
+// 2 * (0x7ff00000 - kEpsHi) exactly for such distances.
+constexpr unsigned kEpsHi = 0x3cb00000u;  // high word of eps = 2^-52
+__device__ __forceinline__ int surv_code(int noop, unsigned neg, unsigned irr) {
+  return noop | (int)(neg << 4) | (irr >= 2u * (0x7ff00000u - kEpsHi) ? 1 << 30 : 0);
+}
+
+template <bool kSettle, int NP, bool kSeg, bool kCode>
 __global__ void __launch_bounds__(256, LSM_PREFILTER_BPS) k_prefilter_tets(int64_t npairs, const int32_t* __restrict__ order,
                                                         const int32_t* __restrict__ pa,
                                                         const int32_t* __restrict__ pb,
@@ -1623,7 +1638,7 @@ __global__ void __launch_bounds__(256, LSM_PREFILTER_BPS) k_prefilter_tets(int64
     bool live = false;
     const int64_t i = ni;
     const int a = na, b = nb;
-    int noop = 0;
+    int noop = 0, code = 0;
     {
       const int64_t jn = j + blockDim.x;
       if (jn < end) {
@@ -1640,6 +1655,7 @@ __global__ void __launch_bounds__(256, LSM_PREFILTER_BPS) k_prefilter_tets(int64
 #pragma unroll
       for (int k = 0; k < 4; ++k) M = fmax(M, fmax(fabs(t.x[k]), fmax(fabs(t.y[k]), fabs(t.z[k]))));
       bool reject = false;
+      unsigned neg = 0, irr = 0;  // sign bits of the distances, and the clipper's class test (surv_code)
 #pragma unroll
       for (int L = 0; L < NP; ++L) {
         double nx, ny, nz, c;
@@ -1649,12 +1665,18 @@ __global__ void __launch_bounds__(256, LSM_PREFILTER_BPS) k_prefilter_tets(int64
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const double d = ((nx * t.x[k] + ny * t.y[k]) + nz * t.z[k]) - c;
+          if (kCode) {
+            const unsigned hi = (unsigned)__double2hiint(d);
+            neg = __funnelshift_l(hi, neg, 1);
+            irr = max(irr, 2u * hi - 2u * kEpsHi);
+          }
           dmin = fmin(dmin, d);
           dmax = fmax(dmax, d);
         }
         reject = reject || dmin >= thr;
         noop |= dmax <= -thr ? 1 << L : 0;
       }
+      code = kCode ? surv_code(noop, neg, irr) : noop;
       if (NP == 4 && !reject && faces_a) {
         const double2* sb = reinterpret_cast<const double2*>(screen_b + (int64_t)b * kScreen3);
         const double2 gt = __ldg(sb + 6), mz = __ldg(sb + 7);
@@ -1704,7 +1726,7 @@ __global__ void __launch_bounds__(256, LSM_PREFILTER_BPS) k_prefilter_tets(int64
       off = __shfl_sync(0xffffffffu, off, leader);
       if (live) {
         const int64_t o = (int64_t)off + __popc(mask & lt);
-        reinterpret_cast<int4*>(survivors)[o] = make_int4((int)i, a, b, noop);
+        reinterpret_cast<int4*>(survivors)[o] = make_int4((int)i, a, b, code);
       }
     }
   }
@@ -1798,7 +1820,7 @@ inline const unsigned long long* seg_nlist(const SegList* seg, const unsigned lo
   return seg_on(seg) ? work + 2 : work;
 }
 inline const int4* seg_table(const SegList* seg) { return seg_on(seg) ? seg->table : nullptr; }
-template <bool kSettle, int NP>
+template <bool kSettle, int NP, bool kCode>
 void run_prefilter(int64_t n, const int32_t* order, const int32_t* pa, const int32_t* pb, const double* coords_a,
                    const double* tol_a, const double* setup, double* measure, int32_t* nout, int32_t* survivors,
                    unsigned long long* work, const double* faces_a, const double* screen_b, const int64_t* n_dev,
@@ -1806,12 +1828,12 @@ void run_prefilter(int64_t n, const int32_t* order, const int32_t* pa, const int
   const int gp = grid_for(n, 256, 8);
   if (seg_on(seg)) {
     count_launch(2);
-    k_prefilter_tets<kSettle, NP, true><<<gp, 256, 0, s>>>(n, order, pa, pb, coords_a, tol_a, setup, measure, nout,
+    k_prefilter_tets<kSettle, NP, true, kCode><<<gp, 256, 0, s>>>(n, order, pa, pb, coords_a, tol_a, setup, measure, nout,
                                                            survivors, work, faces_a, screen_b, n_dev, seg->count);
     k_seg_chunks<<<gp, 256, 0, s>>>(n, n_dev, seg->count, seg->table, work);
   } else {
     count_launch();
-    k_prefilter_tets<kSettle, NP><<<gp, 256, 0, s>>>(n, order, pa, pb, coords_a, tol_a, setup, measure, nout,
+    k_prefilter_tets<kSettle, NP, false, kCode><<<gp, 256, 0, s>>>(n, order, pa, pb, coords_a, tol_a, setup, measure, nout,
                                                      survivors, work, faces_a, screen_b, n_dev);
   }
 }
@@ -1951,12 +1973,10 @@ constexpr int kIxChunk = 64;
 // tet is A itself), which the supermesh's early-out pass settles itself.
 struct IxMeasureSink {
   static constexpr bool kInside = false;
-  static constexpr int kLaneDoubles = 0;  // shared memory per lane behind the point pool
   double* pair_measure;
   int32_t* pair_nout;
   double m;
   int kept;
-  __device__ __forceinline__ void bind(double*) {}
   __device__ __forceinline__ void begin(const int4&) {
     m = 0.0;
     kept = 0;
@@ -1969,25 +1989,21 @@ struct IxMeasureSink {
     pair_measure[p] = m;
     pair_nout[p] = kept;
   }
-  template <int BLOCK>
-  __device__ __forceinline__ void finish() {}
 };
 
 // Measure and count per pair and, for explicit pairs, the output tets:
 // elems (optional) [n][kCap][4][3] in the reference's order (tets beyond
-// kCap are counted, not stored: 81 for tet-tet, 729 for tet-hex).  The list
-// includes pairs with every plane a no-op.
+// kCap are counted, not stored: 729 for tet-hex).  The list includes pairs
+// with every plane a no-op.
 template <int kCap>
 struct IxElemSinkT {
   static constexpr bool kInside = true;
-  static constexpr int kLaneDoubles = 0;
   double* pair_measure;
   int32_t* pair_nout;
   double* elems;
   double m;
   int kept;
   int pid;
-  __device__ __forceinline__ void bind(double*) {}
   __device__ __forceinline__ void begin(const int4& r) {
     m = 0.0;
     kept = 0;
@@ -2010,11 +2026,13 @@ struct IxElemSinkT {
     pair_measure[p] = m;
     pair_nout[p] = kept;
   }
-  template <int NT>
-  __device__ __forceinline__ void finish() {}
 };
 
-using IxElemSink = IxElemSinkT<81>;
+// As IxMeasureSink, for a list that also holds the pairs with every plane a
+// no-op.
+struct IxInsideSink : IxMeasureSink {
+  static constexpr bool kInside = true;
+};
 
 // As IxElemSinkT, but a pair's sum, count and output tets continue from
 // what an earlier launch left in pair_measure / pair_nout / elems: the
@@ -2023,14 +2041,12 @@ using IxElemSink = IxElemSinkT<81>;
 template <int kCap>
 struct IxCarrySinkT {
   static constexpr bool kInside = true;
-  static constexpr int kLaneDoubles = 0;
   double* pair_measure;
   int32_t* pair_nout;
   double* elems;
   double m;
   int kept;
   int pid;
-  __device__ __forceinline__ void bind(double*) {}
   __device__ __forceinline__ void begin(const int4& r) {
     pid = r.x;
     m = pair_measure[pid];
@@ -2053,44 +2069,8 @@ struct IxCarrySinkT {
     pair_measure[p] = m;
     pair_nout[p] = kept;
   }
-  template <int NT>
-  __device__ __forceinline__ void finish() {}
 };
 constexpr int kHexHexCap = 5 * 729;  // output tets per hexahedron pair
-
-// The supermesh's tets, written where the scan of the per-pair counts puts
-// them: tet j of pair p at elems[pair_off[p] + j], with its parents.
-struct IxEmitSink {
-  static constexpr bool kInside = true;
-  static constexpr int kLaneDoubles = 0;
-  const int64_t* pair_off;
-  double* elems;
-  int64_t* parent_a;
-  int64_t* parent_b;
-  int64_t at;
-  int a, b;
-  __device__ __forceinline__ void bind(double*) {}
-  __device__ __forceinline__ void begin(const int4& r) {
-    at = pair_off[r.x];
-    a = r.y;
-    b = r.z;
-  }
-  __device__ __forceinline__ void tet(const Tet& o, double) {
-    double2* e = reinterpret_cast<double2*>(elems + at * 12);
-    e[0] = make_double2(o.x[0], o.y[0]);
-    e[1] = make_double2(o.z[0], o.x[1]);
-    e[2] = make_double2(o.y[1], o.z[1]);
-    e[3] = make_double2(o.x[2], o.y[2]);
-    e[4] = make_double2(o.z[2], o.x[3]);
-    e[5] = make_double2(o.y[3], o.z[3]);
-    if (parent_a) parent_a[at] = a;
-    if (parent_b) parent_b[at] = b;
-    ++at;
-  }
-  __device__ __forceinline__ void end(int64_t) {}
-  template <int NT>
-  __device__ __forceinline__ void finish() {}
-};
 
 // Points in a lane's pool for NP planes: A's 4 vertices + 4 per plane.
 __host__ __device__ constexpr int ix_points(int np) { return 4 + 4 * np; }
@@ -2105,7 +2085,6 @@ __global__ void __launch_bounds__(BLOCK, BPS) k_clip_tets_ix(
   static_assert(ix_points(NP) <= 32, "pool indices are 5 bits");
   extern __shared__ double ix_mem[];
   IxPool<BLOCK> pool{ix_mem + threadIdx.x};
-  sk.bind(ix_mem + 3 * ix_points(NP) * BLOCK + threadIdx.x);
   // pending tets (at most 2 per plane but the last): a shift register of
   // 20-bit index tuples over kW words (stk[kW-1]:...:stk[0], newest in the
   // low bits) and their planes, kLB bits each (stk_lv)
@@ -2263,7 +2242,698 @@ __global__ void __launch_bounds__(BLOCK, BPS) k_clip_tets_ix(
     sk.end(p);
     p = -1;
   }
-  sk.template finish<BLOCK>();
+}
+
+// ----------------------------------------------------------------------
+// K6: breadth-first tet clipper, a warp per batch of pairs
+// ----------------------------------------------------------------------
+// Split table: for the 2-bit classes of a tet's vertices (0 zero, 1 negative,
+// 2 positive) the order in which to gather them (their roles), and each child
+// as a byte permute of (old tet, new points).  In role order the interpolated
+// edges are the same for all cases: (0,3), (1,3), (2,3), except that ++-- takes
+// (0,2) third and (1,2) fourth; interp_edge is symmetric in its ends, so a
+// role's sign does not matter, and the edges that a case does not have give
+// points nothing refers to.
+// Byte permute: byte i of the result is byte s_i of (b : a), s_i the i-th
+// nibble of s; with s_i's top bit set, that byte's sign instead (0 or 0xff).
+__device__ __forceinline__ unsigned prmt(unsigned a, unsigned b, unsigned s) {
+  unsigned r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(s));
+  return r;
+}
+
+struct ClipTable {
+  uint2 e[256];
+};
+
+// Entry for classes c: x = child 0 | child 1 << 16, y = child 2 | roles << 16,
+// each four nibbles (vertex i of the child: 0-3 old vertex, 4-7 new point;
+// roles: old vertex).  Bit 2 of the roles' nibbles 0-3: ++--, two or more
+// children, three, a split (Tetrahedron_Intersection.F90:290-434: the same
+// cases, interpolation and child order as split_tet).
+constexpr ClipTable make_clip_table() {
+  ClipTable T{};
+  for (unsigned c = 0; c < 256; ++c) {
+    unsigned neg[4] = {}, pos[4] = {}, zer[4] = {};
+    unsigned nn = 0, np = 0, nz = 0;
+    bool ok = true;
+    for (unsigned v = 0; v < 4; ++v) {
+      const unsigned k = (c >> (2 * v)) & 3u;
+      if (k == 0) zer[nz++] = v;
+      if (k == 1) neg[nn++] = v;
+      if (k == 2) pos[np++] = v;
+      if (k == 3) ok = false;
+    }
+    unsigned role[4] = {0, 1, 2, 3}, ch[3][4] = {{0, 1, 2, 3}, {0, 1, 2, 3}, {0, 1, 2, 3}};
+    unsigned kids = 1;
+    bool two = false;
+    if (ok && nn > 0 && np > 0) {
+      if (nn == 1) {  // +++-, ++-0, +-00: the r-th positive vertex becomes new point r
+        for (unsigned r = 0; r < 3; ++r) role[r] = r < np ? pos[r] : zer[r - np];
+        role[3] = neg[0];
+        for (unsigned r = 0; r < np; ++r) ch[0][pos[r]] = 4 + r;
+      } else if (np == 2) {  // ++--
+        two = true;
+        kids = 3;
+        role[0] = pos[0];
+        role[1] = pos[1];
+        role[2] = neg[1];
+        role[3] = neg[0];
+        ch[0][pos[0]] = 6;
+        ch[0][pos[1]] = 5;
+        const unsigned a[4] = {neg[1], 7, 6, 5}, b[4] = {neg[0], 4, 5, 6};
+        for (unsigned i = 0; i < 4; ++i) {
+          ch[1][i] = a[i];
+          ch[2][i] = b[i];
+        }
+      } else {  // +---, +--0
+        role[0] = neg[0];
+        role[1] = neg[1];
+        role[2] = nn == 3 ? neg[2] : zer[0];
+        role[3] = pos[0];
+        ch[0][pos[0]] = 4;
+        kids = nn;
+        const unsigned a3[4] = {4, neg[1], neg[2], 5}, b3[4] = {neg[2], 5, 6, 4}, a2[4] = {5, zer[0], neg[1], 4};
+        for (unsigned i = 0; i < 4; ++i) {
+          ch[1][i] = nn == 3 ? a3[i] : a2[i];
+          if (nn == 3) ch[2][i] = b3[i];
+        }
+      }
+    }
+    unsigned w[4] = {};
+    for (unsigned i = 0; i < 4; ++i) {
+      for (unsigned j = 0; j < 3; ++j) w[j] |= ch[j][i] << (4 * i);
+      w[3] |= role[i] << (4 * i);
+    }
+    if (ok && nn > 0 && np > 0) w[3] |= 1u << 14;
+    if (two) w[3] |= 1u << 2;
+    if (kids >= 2) w[3] |= 1u << 6;
+    if (kids == 3) w[3] |= 1u << 10;
+    T.e[c].x = w[0] | w[1] << 16;
+    T.e[c].y = w[2] | w[3] << 16;
+  }
+  return T;
+}
+__device__ const ClipTable g_clip_table = make_clip_table();
+constexpr int kClipTableBytes = sizeof(ClipTable);
+
+// The point where edge (X, Y) meets the plane, dx and dy the ends' distances
+// (of opposite sign).  With i = 1/(dx - dy) it is (-dy i) X + (dx i) Y: for
+// X positive exactly the reference's w0, w1; for X negative both the
+// difference and the reciprocal change sign, which negates nothing in the
+// products, and the sum's two terms change places.
+__device__ __forceinline__ V3 interp_edge(const V3& X, const V3& Y, double dx, double dy) {
+  const double i = __drcp_rn(dx - dy);
+  const double wx = -dy * i, wy = dx * i;
+  return V3{wx * X.x + wy * Y.x, wx * X.y + wy * Y.y, wx * X.z + wy * Y.z};
+}
+
+// Class bits of a distance at plane q (zero if |d| < eps; NaN is neither):
+// bit q negative, bit 4 + q positive.
+__device__ __forceinline__ unsigned class_bits(double d, unsigned neg_bit) {
+  const unsigned hi = (unsigned)__double2hiint(d);
+  const unsigned lim = 0x7ff00000u - kEpsHi;
+  unsigned w = 0;
+  if (hi - kEpsHi <= lim) w = neg_bit << 4;
+  if ((hi ^ 0x80000000u) - kEpsHi <= lim) w = neg_bit;
+  return w;
+}
+
+// A pair whose distances are not all finite, by visits as in k_clip_tets_ix
+// (A's vertices in the pool): a vertex with a NaN distance belongs to none of
+// the reference's three lists, which class bits cannot say.
+template <class Pool, class Sink>
+__device__ __forceinline__ void clip_nonfinite(const Pool& pool, const double* planes, unsigned act, double tol,
+                                               unsigned (&st)[8], Sink& sk) {
+  const int last = 31 - __clz(act);
+  unsigned cur = ix_pack(0, 1, 2, 3), lv = 0;  // lv: 2 bits per pending tet
+  int L = __ffs(act) - 1, sp = 0;
+  for (;;) {
+    Tet t;
+    ix_gather(pool, cur, t);
+    double nx, ny, nz, c;
+    load_plane(planes, L, nx, ny, nz, c);
+    TetClass cls;
+    classify_tet(t, nx, ny, nz, c, cls);
+    int k = 0;
+    unsigned ch[3] = {cur, 0, 0};
+    if (cls.nn > 0) k = cls.np == 0 ? 1 : ix_split(cur, cls, pool, 4 + 4 * L, ch[0], ch[1], ch[2]);
+    if (L == last) {
+#pragma unroll 1
+      for (int j = 0; j < k; ++j) {
+        ix_gather(pool, j == 0 ? ch[0] : (j == 1 ? ch[1] : ch[2]), t);
+        double v1;
+        if (final_tet_keep(t, tol, v1)) sk(t, v1);
+      }
+      k = 0;
+    }
+    const int next = __ffs(act & (~0u << (L + 1))) - 1;
+#pragma unroll
+    for (int j = 2; j > 0; --j)
+      if (j < k) {
+#pragma unroll
+        for (int i = 7; i > 0; --i) st[i] = st[i - 1];
+        st[0] = ch[j];
+        lv = lv << 2 | (unsigned)next;
+        ++sp;
+      }
+    if (k > 0) {
+      cur = ch[0];
+      L = next;
+      continue;
+    }
+    if (sp == 0) break;
+    cur = st[0];
+    L = (int)(lv & 3u);
+#pragma unroll
+    for (int i = 0; i < 7; ++i) st[i] = st[i + 1];
+    lv >>= 2;
+    --sp;
+  }
+}
+
+// Depth-first clipping by one lane per pair (k_clip_tets_ix) leaves half the
+// lanes idle: they keep, drop or split at different moments, and at the last
+// plane up to three volumes run in a row while the others wait.  Where a final
+// tet costs more than its volume (the P1 quadrature, the stores of the
+// supermesh's tets), or where there are too few pairs for a lane each to fill
+// the chip and the longest pair's serial walk is the time (a hundred visits of
+// about 1000 instructions), the whole warp works on the tets of a batch of
+// pairs instead, breadth first: one list of tets per generation (the number of
+// the pair's active planes left), one round at a time over up to 32 tets of
+// one generation, children appended in order.  Every list keeps a pair's tets
+// together and in the reference's breadth-first order, so the last
+// generation's children come out in output order; a lane per pair then adds
+// its volumes up.
+// A point carries one byte with its class at the pair's planes (bits 0-3
+// negative, 4-7 positive, in the order of the generations), evaluated once,
+// when the point is created; a list entry carries its four vertices' bytes,
+// and the same byte permute that makes a child's vertex indices out of the old
+// tet's and the new points' makes its classes.
+// Measured (tet3d_27x32 unless said): P1 mass 12.8 -> 5.9 ms; supermesh elements 4.47 ->
+// 4.04 ms; measures of 330 thousand candidates (10^3 x 6 against 12^3 x 6
+// tets), early-out pass included, 0.212 -> 0.136 ms.  On the large measure
+// passes the two are level (1.38 against 1.34 ms; tet3d_graded_55x51 6.3
+// against 6.8 ms: as many instructions go into the lists and rounds as into
+// the idle lanes of the other), so those stay with k_clip_tets_ix.
+//
+// Shared memory of a warp: the point pool (groups of four points: point i of
+// group q at index 4 q + (i ^ (q >> 2 & 3)), so that the i-th points of
+// sixteen consecutive groups fall into different banks; a split's new points
+// are a group, and so are A's vertices), the planes of each slot's pair in the order
+// of the generations, the lists, and the final tets of one round.
+constexpr int kBfRow = 18;     // doubles per slot: four planes, tolerance, pad
+constexpr int kBfRing = 128;   // entries in the list of generations 1-3
+constexpr int kBfFinals = 96;  // final tets of one round, at most
+template <int Q>
+struct BfPool {
+  static_assert(Q <= 128, "nine index bits");
+  double* x;
+  __device__ __forceinline__ V3 get(unsigned j) const { return V3{x[j], x[4 * Q + j], x[8 * Q + j]}; }
+  __device__ __forceinline__ void put(unsigned j, const V3& v) const {
+    x[j] = v.x;
+    x[4 * Q + j] = v.y;
+    x[8 * Q + j] = v.z;
+  }
+  static __device__ __forceinline__ unsigned at(unsigned q, unsigned i) { return 4 * q + (i ^ (q >> 2 & 3u)); }
+  // A tet's point indices: their low bytes in one word, their high bits in
+  // the bytes of another.  Those of group q:
+  static __device__ __forceinline__ unsigned lo(unsigned q) {
+    return (4 * q & 255u) * 0x01010101u + (0x03020100u ^ (q >> 2 & 3u) * 0x01010101u);
+  }
+  static __device__ __forceinline__ unsigned hi(unsigned q) { return (q >> 6) * 0x01010101u; }
+};
+template <int V>
+__device__ __forceinline__ unsigned bf_vert(unsigned lo, unsigned hi) {
+  return prmt(lo, hi, V | (4 + V) << 4 | (12 + V) << 8 | (12 + V) << 12);
+}
+template <class Pool>
+__device__ __forceinline__ void bf_gather(const Pool& pool, unsigned lo, unsigned hi, V3 (&v)[4]) {
+  v[0] = pool.get(bf_vert<0>(lo, hi));
+  v[1] = pool.get(bf_vert<1>(lo, hi));
+  v[2] = pool.get(bf_vert<2>(lo, hi));
+  v[3] = pool.get(bf_vert<3>(lo, hi));
+}
+template <class Pool>
+__device__ __forceinline__ void bf_tet(const Pool& pool, unsigned lo, unsigned hi, Tet& t) {
+  V3 v[4];
+  bf_gather(pool, lo, hi, v);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    t.x[i] = v[i].x;
+    t.y[i] = v[i].y;
+    t.z[i] = v[i].z;
+  }
+}
+template <int P, int Q>
+__host__ __device__ constexpr int bf_warp_bytes() {
+  return 8 * (12 * Q + P * kBfRow + kBfFinals) + 12 * (3 * kBfRing + 32) + 4 * 32;
+}
+__device__ __forceinline__ void store_tet(double* at, const Tet& o) {
+  double2* e = reinterpret_cast<double2*>(at);
+  e[0] = make_double2(o.x[0], o.y[0]);
+  e[1] = make_double2(o.z[0], o.x[1]);
+  e[2] = make_double2(o.y[1], o.z[1]);
+  e[3] = make_double2(o.x[2], o.y[2]);
+  e[4] = make_double2(o.z[2], o.x[3]);
+  e[5] = make_double2(o.y[3], o.z[3]);
+}
+
+// What is done with a pair's kept output tets.  kSum: their vertex-1 volumes
+// are added up in the reference's order, stored with their count; kStore: the
+// tets are written, the k-th of the pair in slot s at place(s) + k; kP1: the
+// P1 quadrature.  kSlots: pairs per batch; kWarps: warps per SM; kQuads:
+// groups of points; kKeep: groups left to every deeper generation; kRoom:
+// groups a generation must be able to take for its next round to come before
+// a deeper partial one; kExtra: bytes of shared memory per warp beyond the
+// clipper's own.
+struct BfMeasureSink {
+  static constexpr bool kSum = true, kStore = false, kP1 = false;
+  static constexpr int kSlots = 32, kWarps = 10, kQuads = 128, kRoom = 24, kKeep = 8, kExtra = 0;
+  double* pair_measure;
+  int32_t* pair_nout;
+};
+
+// Explicit pairs' output tets: elems [n][81][4][3] (tets beyond 81 are
+// counted, not stored).
+struct BfElemSink {
+  static constexpr bool kSum = true, kStore = true, kP1 = false;
+  static constexpr int kSlots = 32, kWarps = 9, kQuads = 128, kRoom = 24, kKeep = 8, kExtra = 32 * 20;
+  double* pair_measure;
+  int32_t* pair_nout;
+  double* elems;
+  __device__ __forceinline__ int64_t place(const int4& rec) const { return (int64_t)rec.x * 81; }
+  __device__ __forceinline__ void store(const Tet& o, int64_t base, int k, int2) const {
+    if (k < 81) store_tet(elems + (base + k) * 12, o);
+  }
+};
+
+// The supermesh's tets, written where the scan of the per-pair counts puts
+// them, with their parents.
+struct BfEmitSink {
+  static constexpr bool kSum = false, kStore = true, kP1 = false;
+  static constexpr int kSlots = 32, kWarps = 9, kQuads = 128, kRoom = 24, kKeep = 8, kExtra = 32 * 20;
+  const int64_t* pair_off;
+  double* elems;
+  int64_t* parent_a;
+  int64_t* parent_b;
+  __device__ __forceinline__ int64_t place(const int4& rec) const { return pair_off[rec.x]; }
+  __device__ __forceinline__ void store(const Tet& o, int64_t base, int k, int2 ab) const {
+    store_tet(elems + (base + k) * 12, o);
+    if (parent_a) parent_a[base + k] = ab.x;
+    if (parent_b) parent_b[base + k] = ab.y;
+  }
+};
+
+template <class Sink>
+__host__ __device__ constexpr int bf_bytes() {
+  return bf_warp_bytes<Sink::kSlots, Sink::kQuads>() + Sink::kExtra;
+}
+
+template <class Sink>
+__global__ void __launch_bounds__(Sink::kWarps * 32, 1) k_clip_tets_bf(
+    const int4* __restrict__ list, const unsigned long long* __restrict__ nlist, const double* __restrict__ coords_a,
+    const double* __restrict__ tol_a, const double* __restrict__ setup_b, Sink sk, unsigned long long* work,
+    const int4* __restrict__ chunks) {
+  constexpr int P = Sink::kSlots, Q = Sink::kQuads;
+  extern __shared__ double ix_mem[];
+  uint2* table = reinterpret_cast<uint2*>(ix_mem);
+  for (int i = threadIdx.x; i < 256; i += Sink::kWarps * 32) table[i] = g_clip_table.e[i];
+  __syncthreads();
+  char* wm = reinterpret_cast<char*>(ix_mem) + kClipTableBytes + (threadIdx.x >> 5) * bf_bytes<Sink>();
+  BfPool<Q> pool{reinterpret_cast<double*>(wm)};
+  double* rows = pool.x + 12 * Q;
+  uint2* fin = reinterpret_cast<uint2*>(rows + P * kBfRow);  // {low bytes, high bits | slot << 27}
+  // lists of generations 1-3 (kBfRing entries each), then 0 (32)
+  unsigned* llo = reinterpret_cast<unsigned*>(fin + kBfFinals);
+  unsigned* lhi = llo + 3 * kBfRing + 32;
+  unsigned* lcl = lhi + 3 * kBfRing + 32;
+  unsigned short* seg = reinterpret_cast<unsigned short*>(lcl + 3 * kBfRing + 32);  // [2][32]
+  char* extra = wm + bf_warp_bytes<P, Q>();
+  // a final tet's volume takes the place of its indices, except where those
+  // are needed again
+  double* vol = Sink::kP1 ? reinterpret_cast<double*>(extra) : reinterpret_cast<double*>(fin);
+  int64_t* s_base = reinterpret_cast<int64_t*>(extra);         // kStore: [32]
+  int2* s_ab = reinterpret_cast<int2*>(extra + 32 * 8);        // kStore: [32]
+  int* s_run = reinterpret_cast<int*>(extra + 32 * 16);        // kStore: [32] tets stored so far
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const int64_t npairs = (int64_t)*nlist;
+  int64_t cbeg = 0, cend = 0;
+  // the next batch's records, fetched while the current one is clipped
+  int nnext = 0;
+  int4 nrec = make_int4(0, -1, 0, 0);
+  bool done = false;
+  auto fetch = [&] {
+    nnext = 0;
+    if (cbeg >= cend && !done) {
+      unsigned long long base = 0;
+      if (lane == 0) base = atomicAdd(work, chunks ? 1ull : (unsigned long long)kIxChunk);
+      base = __shfl_sync(full, base, 0);
+      if ((int64_t)base >= npairs) {
+        done = true;
+      } else if (chunks) {
+        const int4 ch = chunks[base];
+        cbeg = ch.x;
+        cend = ch.y;
+      } else {
+        cbeg = (int64_t)base;
+        cend = cbeg + kIxChunk < npairs ? cbeg + kIxChunk : npairs;
+      }
+    }
+    if (cbeg < cend) {
+      nnext = cend - cbeg < P ? (int)(cend - cbeg) : P;
+      if (lane < nnext) nrec = list[cbeg + lane];
+      cbeg += nnext;
+    }
+  };
+  fetch();
+  while (nnext) {
+    // ---- a batch of up to P pairs, slot = lane; neighbours with the same A
+    // share its points
+    const int n = nnext;
+    const bool mine = lane < n;
+    const int4 rec = nrec;
+    const int prev = __shfl_up_sync(full, rec.y, 1);
+    const bool fresh = mine && (lane == 0 || prev != rec.y);
+    const unsigned fm = __ballot_sync(full, fresh);
+    const unsigned aq = __popc(fm & (lt | 1u << lane)) - 1u;
+    const unsigned act = ~(unsigned)rec.w & 15u;
+    const int gen = mine ? 4 - __popc(act) : -1;  // generation the pair enters at
+    unsigned x = 0;
+    bool odd = false;
+    if (mine) {
+      const double* row = setup_b + (int64_t)rec.z * clip_row(4);
+      const unsigned w = (unsigned)rec.w;
+      Tet t;
+      if (fresh || (w >> 30)) load_tet(coords_a + (int64_t)rec.y * 12, t);
+      double* o = rows + lane * kBfRow;
+      st2(o + 16, fmin(tol_a[rec.y], row[16]), 0.0);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (act >> q & 1u) {
+          const int h = 4 - __popc(act >> q);
+          double nx, ny, nz, c;
+          load_plane(row, q, nx, ny, nz, c);
+          st2(o + 4 * h, nx, ny);
+          st2(o + 4 * h + 2, nz, c);
+          if (w >> 30) {
+            int bad = 0, nan = 0;
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const double d = ((nx * t.x[v] + ny * t.y[v]) + nz * t.z[v]) - c;
+              x |= class_bits(d, 1u << h) << (8 * v);
+              bad += !isfinite(d);
+              nan += isnan(d);
+            }
+            // (a plane of a degenerate B is NaN at every vertex and drops every tet)
+            odd = odd || (bad > 0 && nan < 4);
+          } else {
+            x |= (((w >> (4 + 4 * (3 - q))) & 15u) * 0x00204081u & 0x01010101u) << h;
+          }
+        }
+      }
+      if (!(w >> 30)) {
+        x = prmt(x, 0, 0x0123);
+        x |= (~x & 0x0f0f0f0fu) << 4;
+      }
+      if (fresh) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) pool.put(pool.at(aq, v), V3{t.x[v], t.y[v], t.z[v]});
+      }
+      if constexpr (Sink::kStore) {
+        s_base[lane] = sk.place(rec);
+        s_ab[lane] = make_int2(rec.y, rec.z);
+        s_run[lane] = 0;
+      }
+      if constexpr (Sink::kP1) sk.begin(extra, lane, rec);
+    }
+    fetch();
+    if (lane < nnext) {  // the next batch's rows into L2
+      const double* ca = coords_a + (int64_t)nrec.y * 12;
+      const double* row = setup_b + (int64_t)nrec.z * clip_row(4);
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(ca));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(row));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(row + 16));
+    }
+    double m = 0.0;
+    int kept = 0;
+    // lists: counts and heads, 8 bits per generation; groups in use below
+    // each generation's own
+    unsigned cnt = 0, head = 0, mark = (unsigned)__popc(fm) * 0x01010101u;
+    int nf = 0;  // final tets to take
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const bool in = gen == g && !odd && (x & (0x01010101u << g));
+      const unsigned b = __ballot_sync(full, in);
+      if (in) {
+        const int at = (g == 0 ? 3 : g - 1) * kBfRing + __popc(b & lt);
+        llo[at] = pool.lo(aq);
+        lhi[at] = pool.hi(aq) | (unsigned)lane << 27;
+        lcl[at] = x;
+      }
+      cnt |= (unsigned)__popc(b) << (8 * g);
+    }
+    {  // pairs whose every plane is a no-op: A itself is the final tet
+      const unsigned b = __ballot_sync(full, gen == 4);
+      nf = __popc(b);
+      if (nf) {
+        const int at = __popc(b & lt);
+        if (gen == 4) fin[at] = make_uint2(pool.lo(aq), pool.hi(aq) | (unsigned)lane << 27);
+        seg[lane] = (unsigned short)at;
+        seg[32 + lane] = (unsigned short)(at + (gen == 4));
+      }
+    }
+    __syncwarp();
+    for (;;) {
+      if (nf) {
+        // ---- final tets, in the pairs' order
+        for (int f0 = 0; f0 < nf; f0 += 32) {
+          const int f = f0 + lane;
+          const bool on = f < nf;
+          uint2 t = make_uint2(0, 0xffffffffu);
+          Tet o;
+          double v1 = 0.0;
+          bool keep = false;
+          if (on) {
+            t = fin[f];
+            bf_tet(pool, t.x, t.y & 0x03030303u, o);
+            keep = final_tet_keep(o, rows[(t.y >> 27) * kBfRow + 16], v1);
+          }
+          if constexpr (Sink::kStore) {
+            // rank among the pair's kept tets: those stored so far, and those
+            // of this step's lanes from the pair's first one on
+            const unsigned slot = t.y >> 27;
+            const unsigned before = __shfl_up_sync(full, slot, 1), after = __shfl_down_sync(full, slot, 1);
+            const unsigned km = __ballot_sync(full, keep);
+            const unsigned hm = __ballot_sync(full, lane == 0 || before != slot);
+            const unsigned first = 31 - __clz(hm & (lt | 1u << lane));
+            const int k = on ? s_run[slot] + __popc(km & lt & ~((1u << first) - 1u)) : 0;
+            if (keep) sk.store(o, s_base[slot], k, s_ab[slot]);
+            __syncwarp();
+            if (on && (lane == 31 || f + 1 == nf || after != slot)) s_run[slot] = k + keep;
+            __syncwarp();
+          }
+          if (on && (Sink::kSum || Sink::kP1)) vol[f] = keep ? v1 : -1.0;
+        }
+        __syncwarp();
+        if constexpr (Sink::kSum) {
+          int f = seg[lane];
+          const int fe = seg[32 + lane];
+#pragma unroll 1
+          for (; f < fe; f += 4) {
+            double v1[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v1[i] = f + i < fe ? vol[f + i] : -1.0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (__double2hiint(v1[i]) >= 0) {
+                m = m + v1[i];
+                ++kept;
+              }
+          }
+        }
+        if constexpr (Sink::kP1) sk.integrate(extra, pool, fin, vol, nf, lane);
+        nf = 0;
+        __syncwarp();
+      }
+      if (!cnt) break;
+      // ---- a round: the deepest generation with tets; with fewer than a warp
+      // of them, the one before it first, if its new points still fit
+      int g = (31 - __clz(cnt)) >> 3;
+      {
+        const unsigned here = (cnt >> (8 * g)) & 255u;
+        if (g > 0 && here < 32 && ((cnt >> (8 * (g - 1))) & 255u) &&
+            ((mark >> (8 * g)) & 255u) + Sink::kRoom <= Q - Sink::kKeep * (4 - g))
+          --g;
+      }
+      // new points go behind those that tets in the lists still refer to
+      const unsigned deeper = cnt >> (8 * g) >> 8;
+      unsigned top = (mark >> (8 * (g + (deeper != 0)))) & 255u;
+      const unsigned room = Q - Sink::kKeep * (3 - g) - top;
+      unsigned r = min((cnt >> (8 * g)) & 255u, 32u);
+      const int src =
+          (g == 0 ? 3 : g - 1) * kBfRing + ((((head >> (8 * g)) & 255u) + lane) & (g == 0 ? 31 : kBfRing - 1));
+      const unsigned lo = llo[src], hs = lhi[src];
+      x = lcl[src];
+      const unsigned slot = hs >> 27, hi = hs & 0x03030303u;
+      const unsigned cls = ((x >> g) & 0x01010101u) | ((x >> (g + 3)) & 0x02020202u);
+      const uint2 e = table[(cls * 0x01041040u) >> 24];
+      bool split = lane < (int)r && (e.y >> 30 & 1u);
+      unsigned sm = __ballot_sync(full, split);
+      if (__popc(sm) > (int)room) {  // the round ends before the first split that finds no room
+        const unsigned over = __ballot_sync(full, split && __popc(sm & lt) >= (int)room);
+        r = __ffs(over) - 1;
+        sm &= (1u << r) - 1u;
+        split = split && lane < (int)r;
+      }
+      const bool on = lane < (int)r;
+      const unsigned quad = top + __popc(sm & lt);
+      unsigned nm = 0;
+      if (split) {
+        const double* pr = rows + slot * kBfRow;
+        V3 v[4];
+        bf_gather(pool, prmt(lo, lo, e.y >> 16), prmt(hi, hi, e.y >> 16), v);
+        double d[4];
+        {
+          const double2 n01 = *reinterpret_cast<const double2*>(pr + 4 * g);
+          const double2 n2c = *reinterpret_cast<const double2*>(pr + 4 * g + 2);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) d[i] = ((n01.x * v[i].x + n01.y * v[i].y) + n2c.x * v[i].z) - n2c.y;
+        }
+        const bool two = (e.y >> 18) & 1u;
+        V3 T[4];
+        T[0] = interp_edge(v[0], v[3], d[0], d[3]);
+        T[1] = interp_edge(v[1], v[3], d[1], d[3]);
+        T[2] = interp_edge(v[2], two ? v[0] : v[3], d[2], two ? d[0] : d[3]);
+        T[3] = V3{0.0, 0.0, 0.0};
+        if (two) T[3] = interp_edge(v[1], v[2], d[1], d[2]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) pool.put(pool.at(quad, i), T[i]);
+        // classes of the new points: negative up to this plane (it keeps what
+        // is left of the tet), evaluated at those after it
+        nm = ((2u << g) - 1u) * 0x01010101u;
+#pragma unroll 1
+        for (int h = g + 1; h < 4; ++h) {
+          const double2 n01 = *reinterpret_cast<const double2*>(pr + 4 * h);
+          const double2 n2c = *reinterpret_cast<const double2*>(pr + 4 * h + 2);
+          double q[4];
+          unsigned neg = 0, irr = 0;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            q[i] = ((n01.x * T[i].x + n01.y * T[i].y) + n2c.x * T[i].z) - n2c.y;
+            const unsigned qh = (unsigned)__double2hiint(q[i]);
+            neg = __funnelshift_l(qh, neg, 1);
+            irr = max(irr, 2u * qh - 2u * kEpsHi);
+          }
+          if (irr < 2u * (0x7ff00000u - kEpsHi)) {
+            const unsigned nb = prmt(neg * 0x00204081u & 0x01010101u, 0, 0x0123);
+            nm |= (nb | (nb ^ 0x01010101u) << 4) << h;
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) nm |= class_bits(q[i], 1u << h) << (8 * i);
+          }
+        }
+      }
+      const unsigned nlo = pool.lo(quad), nhi = pool.hi(quad), sl = slot << 27;
+      const bool k2 = on && (e.y >> 22 & 1u), k3 = on && (e.y >> 26 & 1u);
+      const unsigned sel1 = e.x >> 16;
+      // this round's tets leave the list
+      top += __popc(sm);
+      cnt -= r << (8 * g);
+      head = (head & ~(255u << (8 * g))) | (((((head >> (8 * g)) & 255u) + r) & (kBfRing - 1)) << (8 * g));
+      if (g < 3) {
+        // children without a negative vertex at the next plane are dropped
+        const unsigned nb = 0x01010101u << (g + 1);
+        const unsigned x0 = prmt(x, nm, e.x), x1 = prmt(x, nm, sel1), x2 = prmt(x, nm, e.y);
+        const bool f0 = on && (x0 & nb), f1 = k2 && (x1 & nb), f2 = k3 && (x2 & nb);
+        const unsigned b0 = __ballot_sync(full, f0), b1 = __ballot_sync(full, f1), b2 = __ballot_sync(full, f2);
+        unsigned at = ((head >> (8 * g + 8)) & 255u) + ((cnt >> (8 * g + 8)) & 255u) + __popc(b0 & lt) +
+                      __popc(b1 & lt) + __popc(b2 & lt);
+        auto put = [&](unsigned sel, unsigned xc) {
+          const int l = g * kBfRing + (at++ & (kBfRing - 1));
+          llo[l] = prmt(lo, nlo, sel);
+          lhi[l] = prmt(hi, nhi, sel) | sl;
+          lcl[l] = xc;
+        };
+        if (f0) put(e.x, x0);
+        if (f1) put(sel1, x1);
+        if (f2) put(e.y, x2);
+        cnt += (unsigned)(__popc(b0) + __popc(b1) + __popc(b2)) << (8 * g + 8);
+        mark = (mark & ~(255u << (8 * g + 8))) | top << (8 * g + 8);
+      } else {
+        // the children are final tets
+        const unsigned b0 = __ballot_sync(full, on), b1 = __ballot_sync(full, k2), b2 = __ballot_sync(full, k3);
+        unsigned at = __popc(b0 & lt) + __popc(b1 & lt) + __popc(b2 & lt);
+        nf = __popc(b0) + __popc(b1) + __popc(b2);
+        if (Sink::kSum) {
+          seg[lane] = 0;
+          seg[32 + lane] = 0;
+        }
+        const unsigned before = __shfl_up_sync(full, slot, 1), after = __shfl_down_sync(full, slot, 1);
+        __syncwarp();
+        if (on) {
+          if (Sink::kSum && (lane == 0 || before != slot)) seg[slot] = (unsigned short)at;
+          fin[at++] = make_uint2(prmt(lo, nlo, e.x), prmt(hi, nhi, e.x) | sl);
+          if (k2) fin[at++] = make_uint2(prmt(lo, nlo, sel1), prmt(hi, nhi, sel1) | sl);
+          if (k3) fin[at++] = make_uint2(prmt(lo, nlo, e.y), prmt(hi, nhi, e.y) | sl);
+          if (Sink::kSum && (lane == (int)r - 1 || after != slot)) seg[32 + slot] = (unsigned short)at;
+        }
+      }
+      __syncwarp();
+    }
+    // ---- pairs with distances that are not finite, one at a time
+    for (unsigned om = __ballot_sync(full, odd); om; om &= om - 1u) {
+      if (lane == __ffs(om) - 1) {
+        Tet t;
+        load_tet(coords_a + (int64_t)rec.y * 12, t);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) pool.put(v, V3{t.x[v], t.y[v], t.z[v]});
+        unsigned st[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) st[i] = 0;
+        auto each = [&](const Tet& o, double v1) {
+          if constexpr (Sink::kStore) sk.store(o, s_base[lane], kept, s_ab[lane]);
+          if constexpr (Sink::kP1) sk.tet(extra, lane, o, v1);
+          m = m + v1;
+          ++kept;
+        };
+        clip_nonfinite(pool, setup_b + (int64_t)rec.z * clip_row(4), act, rows[lane * kBfRow + 16], st, each);
+      }
+      __syncwarp();
+    }
+    if constexpr (Sink::kSum) {
+      if (mine) {
+        sk.pair_measure[rec.x] = m;
+        sk.pair_nout[rec.x] = kept;
+      }
+    }
+    if constexpr (Sink::kP1) sk.end(extra, n, rec, lane);
+    __syncwarp();
+  }
+}
+
+// Measure passes of fewer candidate pairs than this go through
+// k_clip_tets_bf.  Early-out pass and clipper, k_clip_tets_ix against it:
+// 330 thousand candidates 0.212 / 0.136 ms, 1.05 million explicit pairs (whole call) 0.757 /
+// 0.699 ms, 10 million 1.83 / 1.80 ms, 56 million (graded) 8.67 / 9.14 ms.
+constexpr int64_t kBfMeasureMax = 4 << 20;
+
+template <class Sink>
+size_t bf_smem_bytes() {
+  return kClipTableBytes + (size_t)Sink::kWarps * bf_bytes<Sink>();
+}
+template <class Sink>
+cudaError_t bf_attributes() {
+  return cudaFuncSetAttribute(k_clip_tets_bf<Sink>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)bf_smem_bytes<Sink>());
+}
+template <class Sink>
+void run_bf(const int4* list, const unsigned long long* nlist, const double* coords_a, const double* tol_a,
+            const double* setup_b, const Sink& sk, unsigned long long* work, const int4* chunks, cudaStream_t s) {
+  k_clip_tets_bf<Sink><<<sm_count(), Sink::kWarps * 32, bf_smem_bytes<Sink>(), s>>>(list, nlist, coords_a, tol_a,
+                                                                                    setup_b, sk, work, chunks);
 }
 
 size_t ix_smem_bytes() { return (size_t)kIxBlock * 3 * kIxPoints * sizeof(double); }
@@ -2361,13 +3031,13 @@ cudaError_t launch_tet_hex_pairs(int64_t n, const double* tet_a, const double* h
   const int4* list = reinterpret_cast<const int4*>(survivors);
   const int g = sm_count();
   if (elems) {
-    run_prefilter<false, 6>(n, nullptr, iota, iota, tet_a, tol_a, setup, measure, nout, survivors, work, nullptr,
+    run_prefilter<false, 6, false>(n, nullptr, iota, iota, tet_a, tol_a, setup, measure, nout, survivors, work, nullptr,
                             nullptr, nullptr, seg, s);
     k_clip_tets_ix<IxElemSinkT<729>, kIxHexBlock, 1, 6><<<g, kIxHexBlock, ix_hex_smem_bytes(), s>>>(
         list, seg_nlist(seg, work), tet_a, tol_a, setup, IxElemSinkT<729>{measure, nout, elems}, work + 1,
         seg_table(seg));
   } else {
-    run_prefilter<true, 6>(n, nullptr, iota, iota, tet_a, tol_a, setup, measure, nout, survivors, work, nullptr,
+    run_prefilter<true, 6, false>(n, nullptr, iota, iota, tet_a, tol_a, setup, measure, nout, survivors, work, nullptr,
                            nullptr, nullptr, seg, s);
     k_clip_tets_ix<IxMeasureSink, kIxHexBlock, 1, 6><<<g, kIxHexBlock, ix_hex_smem_bytes(), s>>>(
         list, seg_nlist(seg, work), tet_a, tol_a, setup, IxMeasureSink{measure, nout, 0.0, 0}, work + 1,
@@ -2435,7 +3105,7 @@ cudaError_t launch_hex_hex_pairs(int64_t n, const double* hex_a, const double* h
     const double* tk = sub + (int64_t)k * n * 12;
     const double* lk = tol + (int64_t)k * n;
     cudaMemsetAsync(work, 0, 2 * sizeof(unsigned long long), s);
-    run_prefilter<false, 6>(n, nullptr, iota, iota, tk, lk, setup, nullptr, nullptr, survivors, work, nullptr,
+    run_prefilter<false, 6, false>(n, nullptr, iota, iota, tk, lk, setup, nullptr, nullptr, survivors, work, nullptr,
                             nullptr, nullptr, seg, s);
     count_launch();
     k_clip_tets_ix<IxCarrySinkT<kHexHexCap>, kIxHexBlock, 1, 6><<<sm_count(), kIxHexBlock, ix_hex_smem_bytes(), s>>>(
@@ -2451,12 +3121,20 @@ cudaError_t launch_clip_elems(int64_t n, const int32_t* pair_a, const int32_t* p
                               const double* screen_b, cudaStream_t s, const SegList* seg) {
   cudaMemsetAsync(work, 0, 2 * sizeof(unsigned long long), s);
   if (n <= 0) return cudaGetLastError();
-  run_prefilter<false, 4>(n, nullptr, pair_a, pair_b, tet_a, tol_a, setup, measure, nout, survivors, work, faces_a,
+  run_prefilter<false, 4, true>(n, nullptr, pair_a, pair_b, tet_a, tol_a, setup, measure, nout, survivors, work, faces_a,
                           screen_b, nullptr, seg, s);
   count_launch();
-  k_clip_tets_ix<IxElemSink, kIxBlock, kIxBlocksPerSm><<<sm_count() * kIxBlocksPerSm, kIxBlock, ix_smem_bytes(), s>>>(
-      reinterpret_cast<const int4*>(survivors), seg_nlist(seg, work), tet_a, tol_a, setup,
-      IxElemSink{measure, nout, elems}, work + 1, seg_table(seg));
+  const int4* list = reinterpret_cast<const int4*>(survivors);
+  if (elems)
+    run_bf(list, seg_nlist(seg, work), tet_a, tol_a, setup, BfElemSink{measure, nout, elems}, work + 1, seg_table(seg),
+           s);
+  else if (n < kBfMeasureMax)
+    run_bf(list, seg_nlist(seg, work), tet_a, tol_a, setup, BfMeasureSink{measure, nout}, work + 1, seg_table(seg), s);
+  else
+    k_clip_tets_ix<IxInsideSink, kIxBlock, kIxBlocksPerSm>
+        <<<sm_count() * kIxBlocksPerSm, kIxBlock, ix_smem_bytes(), s>>>(list, seg_nlist(seg, work), tet_a, tol_a, setup,
+                                                                        IxInsideSink{{measure, nout, 0.0, 0}}, work + 1,
+                                                                        seg_table(seg));
   return cudaGetLastError();
 }
 
@@ -2506,7 +3184,9 @@ cudaError_t launch_clip(int dim, int64_t npairs, const int32_t* pair_a, const in
     // the binned orders read one list: with bin->flat the segments are
     // gathered into it first
     const SegList sg = (bin && !bin->flat) ? SegList{} : (seg ? *seg : SegList{});
-    run_prefilter<true, 4>(npairs, order, pair_a, pair_b, coords_a, tol_a, setup_b, pair_measure, pair_nout,
+    const bool bf = !bin && npairs < kBfMeasureMax;
+    const auto early = bf ? run_prefilter<true, 4, true> : run_prefilter<true, 4, false>;
+    early(npairs, order, pair_a, pair_b, coords_a, tol_a, setup_b, pair_measure, pair_nout,
                            overflow_list, work, faces_a, screen_b, n_dev, &sg, s);
     const int4* list = reinterpret_cast<const int4*>(overflow_list);
     if (bin) {
@@ -2520,9 +3200,14 @@ cudaError_t launch_clip(int dim, int64_t npairs, const int32_t* pair_a, const in
       if (e != cudaSuccess) return e;
       list = bin->out;
     }
-    k_clip_tets_ix<IxMeasureSink, kIxBlock, kIxBlocksPerSm><<<sm_count() * kIxBlocksPerSm, kIxBlock, ix_smem_bytes(), s>>>(
-        list, bin ? work : seg_nlist(&sg, work), coords_a, tol_a, setup_b,
-        IxMeasureSink{pair_measure, pair_nout, 0.0, 0}, work + 1, bin ? nullptr : seg_table(&sg));
+    if (bf)
+      run_bf(list, seg_nlist(&sg, work), coords_a, tol_a, setup_b, BfMeasureSink{pair_measure, pair_nout}, work + 1,
+             seg_table(&sg), s);
+    else
+      k_clip_tets_ix<IxMeasureSink, kIxBlock, kIxBlocksPerSm>
+          <<<sm_count() * kIxBlocksPerSm, kIxBlock, ix_smem_bytes(), s>>>(
+              list, bin ? work : seg_nlist(&sg, work), coords_a, tol_a, setup_b,
+              IxMeasureSink{pair_measure, pair_nout, 0.0, 0}, work + 1, bin ? nullptr : seg_table(&sg));
   }
   if (ev_end) cudaEventRecord(ev_end, s);
   return cudaGetLastError();
@@ -2584,9 +3269,8 @@ cudaError_t launch_emit_elements(int dim, int64_t npairs, const int32_t* pair_a,
   // the survivors of the counting pass again (work[0] holds their number);
   // only the clipper's pair counter starts over
   cudaMemsetAsync(work + 1, 0, sizeof(unsigned long long), s);
-  k_clip_tets_ix<IxEmitSink, kIxBlock, kIxBlocksPerSm><<<sm_count() * kIxBlocksPerSm, kIxBlock, ix_smem_bytes(), s>>>(
-      reinterpret_cast<const int4*>(survivors), seg_nlist(seg, work), coords_a, tol_a, setup_b,
-      IxEmitSink{pair_off, elems, parent_a, parent_b}, work + 1, seg_table(seg));
+  run_bf(reinterpret_cast<const int4*>(survivors), seg_nlist(seg, work), coords_a, tol_a, setup_b,
+         BfEmitSink{pair_off, elems, parent_a, parent_b}, work + 1, seg_table(seg), s);
   return cudaGetLastError();
 }
 
@@ -2596,11 +3280,11 @@ cudaError_t init_device_attributes() {
   cudaError_t e = cudaFuncSetAttribute(k_clip_tets_ix<IxMeasureSink, kIxBlock, kIxBlocksPerSm>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ix_smem_bytes());
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_clip_tets_ix<IxElemSink, kIxBlock, kIxBlocksPerSm>,
+    e = cudaFuncSetAttribute(k_clip_tets_ix<IxInsideSink, kIxBlock, kIxBlocksPerSm>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ix_smem_bytes());
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_clip_tets_ix<IxEmitSink, kIxBlock, kIxBlocksPerSm>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ix_smem_bytes());
+  if (e == cudaSuccess) e = bf_attributes<BfMeasureSink>();
+  if (e == cudaSuccess) e = bf_attributes<BfElemSink>();
+  if (e == cudaSuccess) e = bf_attributes<BfEmitSink>();
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_clip_tets_ix<IxMeasureSink, kIxHexBlock, 1, 6>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ix_hex_smem_bytes());
@@ -3658,7 +4342,8 @@ __device__ __forceinline__ int64_t node_of(const void* en, int64_t e, int loc, i
 // row swaps (row exchanged with row 0 in bits 0-1, with row 1 in bits 2-3).
 // p1_apply_3d applies to the point's right-hand side exactly the operations
 // the elimination applies to the augmented column, in the same order.
-constexpr int kP1Fac3 = 12;
+// Entries 12-14 hold the pivots' reciprocals, for div_by.
+constexpr int kP1Fac3 = 15;
 
 template <int S>
 __device__ __forceinline__ int p1_factor_3d(const double* cc, double* F) {
@@ -3694,6 +4379,7 @@ __device__ __forceinline__ int p1_factor_3d(const double* cc, double* F) {
     sw |= j << (2 * i);
     const double piv = m[i][i];
     F[(3 + i) * S] = piv;
+    F[(12 + i) * S] = __drcp_rn(piv);
 #pragma unroll
     for (int c = 0; c < 3; ++c) m[i][c] = m[i][c] / piv;
 #pragma unroll
@@ -3717,8 +4403,31 @@ __device__ __forceinline__ int p1_factor_3d(const double* cc, double* F) {
   return sw;
 }
 
-template <int S>
-__device__ __forceinline__ void p1_apply_3d(const double* F, int sw, double x, double y, double z, double f[4]) {
+// a / b, correctly rounded, for a divisor whose correctly rounded reciprocal
+// y is at hand.  Markstein (IBM J. Res. Dev. 34, 1990): if q is within one ulp
+// of a/b and y = RN(1/b), then r = a - b q is exact and RN(q + r y) = RN(a/b).
+// a y is within 1.5 ulp, so a first such step brings q within one ulp and the
+// second gives the quotient.  Holds while nothing underflows or overflows:
+// div_range keeps the largest 2 * (high word of |v|) - 2 * high(2^-400), modulo
+// 2^32, of the operands; div_ok(max) is false as soon as one lies outside
+// [2^-400, 2^400] (zero, infinity and NaN included), and the caller then
+// divides.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  double q = a * y;
+  q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+constexpr unsigned kDivLo = (1023u - 400u) << 20, kDivHi = (1023u + 400u) << 20;
+__device__ __forceinline__ unsigned div_range(unsigned range, double v) {
+  return max(range, 2u * (unsigned)__double2hiint(v) - 2u * kDivLo);
+}
+__device__ __forceinline__ bool div_ok(unsigned range) { return range <= 2u * (kDivHi - kDivLo); }
+
+// FAST: the three divisions through the stored reciprocals; range gathers
+// their numerators.
+template <int S, bool FAST>
+__device__ __forceinline__ void p1_apply_3d(const double* F, int sw, double x, double y, double z, double f[4],
+                                            unsigned& range) {
   double r0 = x - F[0], r1 = y - F[S], r2 = z - F[2 * S];
   const int j0 = sw & 3, j1 = (sw >> 2) & 3;
   {
@@ -3727,7 +4436,8 @@ __device__ __forceinline__ void p1_apply_3d(const double* F, int sw, double x, d
     r1 = j0 == 1 ? t0 : r1;
     r2 = j0 == 2 ? t0 : r2;
   }
-  r0 = r0 / F[3 * S];
+  if (FAST) range = div_range(range, r0);
+  r0 = FAST ? div_by(r0, F[3 * S], F[12 * S]) : r0 / F[3 * S];
   r1 = r1 - F[6 * S] * r0;
   r2 = r2 - F[7 * S] * r0;
   {
@@ -3735,9 +4445,11 @@ __device__ __forceinline__ void p1_apply_3d(const double* F, int sw, double x, d
     r1 = j1 == 2 ? r2 : r1;
     r2 = j1 == 2 ? t1 : r2;
   }
-  r1 = r1 / F[4 * S];
+  if (FAST) range = div_range(range, r1);
+  r1 = FAST ? div_by(r1, F[4 * S], F[13 * S]) : r1 / F[4 * S];
   r2 = r2 - F[8 * S] * r1;
-  r2 = r2 / F[5 * S];
+  if (FAST) range = div_range(range, r2);
+  r2 = FAST ? div_by(r2, F[5 * S], F[14 * S]) : r2 / F[5 * S];
   r1 = r1 - F[9 * S] * r2;
   r0 = r0 - F[10 * S] * r2;
   r0 = r0 - F[11 * S] * r1;
@@ -3750,14 +4462,20 @@ __device__ __forceinline__ void p1_apply_3d(const double* F, int sw, double x, d
 // P1-P1 mixed mass block of a pair (test_parallel_p1_inner_product_3d.F90:
 // four-point rule, P1 bases of A and B by elimination at each point), per
 // kept output tet in the reference's order; at the end of the pair the block
-// is stored and u^T M v written per pair (lanes take pairs in a dynamic order;
-// the caller sums them in pair order).  The per-element part of
-// both eliminations is done once per pair (p1_factor_3d) into the lane's
-// slice of shared memory behind the point pool (kLaneDoubles per lane).
-template <typename IDX, int BLOCK>
-struct IxP1Sink {
-  static constexpr bool kInside = true;
-  static constexpr int kLaneDoubles = 2 * kP1Fac3;
+// is stored and u^T M v written per pair (the caller sums them in pair order).
+// The per-element part of both eliminations is done once per pair
+// (p1_factor_3d).  Sixteen final tets at a time: two lanes evaluate a tet's
+// bases, two points each, into shared memory; then sixteen lanes, one per
+// entry of the block, add the products up, tet by tet (the other sixteen take
+// the tets from the first pair boundary after the eighth on).
+template <typename IDX>
+struct BfP1Sink {
+  static constexpr bool kSum = false, kStore = false, kP1 = true;
+  static constexpr int kSlots = 16, kWarps = 8, kQuads = 64, kRoom = 12, kKeep = 4;
+  static constexpr int kLane = 18;  // doubles per lane: w phi_A, then phi_B, of two points interleaved; pad
+  static constexpr int kVol = 0, kFac = kVol + 8 * kBfFinals, kBlk = kFac + 8 * 2 * kP1Fac3 * kSlots,
+                       kBuf = kBlk + 8 * 16 * kSlots, kMeta = kBuf + 8 * 32 * kLane,
+                       kExtra = kMeta + 8 * kSlots;
   const double* coords_a;
   const double* coords_b;
   const void* en_a;
@@ -3766,60 +4484,185 @@ struct IxP1Sink {
   const double* v_b;
   double* blocks;
   double* pair_uv;  // u^T M v per pair (when u_a and v_b are given), summed in pair order afterwards
-  double blk[16];
-  double* fac;  // this lane's factors: A's at fac, B's at fac + kP1Fac3 * BLOCK
-  int a, b, swa, swb;
-  __device__ __forceinline__ void bind(double* lane_mem) { fac = lane_mem; }
-  __device__ __forceinline__ void begin(const int4& r) {
-    a = r.y;
-    b = r.z;
-    swa = p1_factor_3d<BLOCK>(coords_a + (int64_t)a * 12, fac);
-    swb = p1_factor_3d<BLOCK>(coords_b + (int64_t)b * 12, fac + kP1Fac3 * BLOCK);
+  __device__ __forceinline__ void begin(char* mem, int slot, const int4& r) const {
+    double* fa = reinterpret_cast<double*>(mem + kFac) + slot;
+    double* fb = fa + kP1Fac3 * kSlots;
+    double* blk = reinterpret_cast<double*>(mem + kBlk) + 16 * slot;
+    const int swa = p1_factor_3d<kSlots>(coords_a + (int64_t)r.y * 12, fa);
+    const int swb = p1_factor_3d<kSlots>(coords_b + (int64_t)r.z * 12, fb);
+    unsigned range = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      range = div_range(range, fa[(3 + i) * kSlots]);
+      range = div_range(range, fb[(3 + i) * kSlots]);
+    }
+    reinterpret_cast<uint2*>(mem + kMeta)[slot] = make_uint2((unsigned)((swa & 15) | swb << 4), range);
 #pragma unroll
     for (int j = 0; j < 16; ++j) blk[j] = 0.0;
   }
-  __device__ __forceinline__ void tet(const Tet& o, double v1) {
+  // Quadrature point qq of tet o, in the reference's order of operations.
+  static __device__ __forceinline__ V3 point(const Tet& o, int qq) {
     const double qa = 5.8541019662496852e-1, qb = 1.3819660112501050e-1;
+    V3 p{0.0, 0.0, 0.0};
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const double wv = v == qq ? qa : qb;
+      p.x = p.x + wv * o.x[v];
+      p.y = p.y + wv * o.y[v];
+      p.z = p.z + wv * o.z[v];
+    }
+    return p;
+  }
+  // One tet of one lane's pair (pairs with distances that are not finite).
+  __device__ __forceinline__ void tet(char* mem, int slot, const Tet& o, double v1) const {
+    const double* fac = reinterpret_cast<const double*>(mem + kFac) + slot;
+    double* blk = reinterpret_cast<double*>(mem + kBlk) + 16 * slot;
+    const unsigned sw = reinterpret_cast<const uint2*>(mem + kMeta)[slot].x;
     const double w = 0.25 * v1;
-#pragma unroll
+    unsigned range = 0;
+#pragma unroll 1
     for (int qq = 0; qq < 4; ++qq) {
-      double x = 0.0, y = 0.0, z = 0.0;
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const double wv = v == qq ? qa : qb;
-        x = x + wv * o.x[v];
-        y = y + wv * o.y[v];
-        z = z + wv * o.z[v];
-      }
+      const V3 p = point(o, qq);
       double fa[4], fb[4];
-      p1_apply_3d<BLOCK>(fac, swa, x, y, z, fa);
-      p1_apply_3d<BLOCK>(fac + kP1Fac3 * BLOCK, swb, x, y, z, fb);
+      p1_apply_3d<kSlots, false>(fac, sw & 15, p.x, p.y, p.z, fa, range);
+      p1_apply_3d<kSlots, false>(fac + kP1Fac3 * kSlots, sw >> 4, p.x, p.y, p.z, fb, range);
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int c = 0; c < 4; ++c) blk[r * 4 + c] += w * fa[r] * fb[c];
     }
   }
-  __device__ __forceinline__ void end(int64_t p) {
-    if (blocks) {
+  template <class Pool>
+  __device__ __forceinline__ void integrate(char* mem, const Pool& pool, const uint2* fin, const double* vol, int nf,
+                                            int lane) const {
+    const unsigned full = 0xffffffffu;
+    double* buf = reinterpret_cast<double*>(mem + kBuf);
+    double* blk = reinterpret_cast<double*>(mem + kBlk);
+#pragma unroll 1
+    for (int f0 = 0; f0 < nf; f0 += 16) {
+      const int nt = nf - f0 < 16 ? nf - f0 : 16;
+      const int t = lane >> 1;
+      uint2 id = make_uint2(0, 0xffffffffu);
+      double v1 = -1.0;
+      if (t < nt) {
+        id = fin[f0 + t];
+        v1 = vol[f0 + t];
+      }
+      const unsigned slot = id.y >> 27;
+      if (v1 >= 0.0) {
+        Tet o;
+        bf_tet(pool, id.x, id.y & 0x03030303u, o);
+        const double* fac = reinterpret_cast<const double*>(mem + kFac) + slot;
+        const uint2 meta = reinterpret_cast<const uint2*>(mem + kMeta)[slot];
+        const double w = 0.25 * v1;
+        double fa[2][4], fb[2][4];
+        unsigned range = meta.y;
+        // this lane's points 0 and 1, or 2 and 3: the vertices' weights
+        const bool second = lane & 1;
+        V3 p[2];
+        {
+          const double qa = 5.8541019662496852e-1, qb = 1.3819660112501050e-1;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) blocks[p * 16 + j] = blk[j];
+          for (int j = 0; j < 2; ++j) {
+            p[j] = V3{0.0, 0.0, 0.0};
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const double wv = (v & 1) == j && (v >> 1) == (int)second ? qa : qb;
+              p[j].x = p[j].x + wv * o.x[v];
+              p[j].y = p[j].y + wv * o.y[v];
+              p[j].z = p[j].z + wv * o.z[v];
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          p1_apply_3d<kSlots, true>(fac, meta.x & 15, p[j].x, p[j].y, p[j].z, fa[j], range);
+          p1_apply_3d<kSlots, true>(fac + kP1Fac3 * kSlots, meta.x >> 4, p[j].x, p[j].y, p[j].z, fb[j], range);
+        }
+        if (!div_ok(range)) {
+#pragma unroll 1
+          for (int j = 0; j < 2; ++j) {
+            const V3 pj = point(o, 2 * (int)second + j);
+            double ga[4], gb[4];
+            p1_apply_3d<kSlots, false>(fac, meta.x & 15, pj.x, pj.y, pj.z, ga, range);
+            p1_apply_3d<kSlots, false>(fac + kP1Fac3 * kSlots, meta.x >> 4, pj.x, pj.y, pj.z, gb, range);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              if (j == 0) {
+                fa[0][i] = ga[i];
+                fb[0][i] = gb[i];
+              } else {
+                fa[1][i] = ga[i];
+                fb[1][i] = gb[i];
+              }
+            }
+          }
+        }
+        double* out = buf + lane * kLane;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          st2(out + 2 * i, w * fa[0][i], w * fa[1][i]);
+          st2(out + 8 + 2 * i, fb[0][i], fb[1][i]);
+        }
+      } else {  // (a sum is not changed by adding +0)
+        double* out = buf + lane * kLane;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) st2(out + 2 * i, 0.0, 0.0);
+      }
+      // pair boundaries among the sixteen tets
+      const unsigned before = __shfl_up_sync(full, slot, 2);
+      const unsigned heads = __ballot_sync(full, t < nt && (t == 0 || before != slot));
+      __syncwarp();
+      const int h = lane >> 4;
+      const unsigned late = heads >> 16;  // boundaries from the eighth tet on
+      const int mid = late ? 8 + ((__ffs(late) - 1) >> 1) : nt;
+      int i = h ? mid : 0;
+      const int ie = h ? nt : mid;
+      const double* q = buf + 2 * i * kLane + 2 * ((lane >> 2) & 3);
+      const int cb = 8 + 2 * ((lane & 3) - ((lane >> 2) & 3));
+      while (i < ie) {  // one pair's tets (the first of the sixteen go on from the ones before)
+        double* at = blk + 16 * (fin[f0 + i].y >> 27) + (lane & 15);
+        const unsigned next = heads & ~((4u << (2 * i)) - 1u);
+        const int end = next ? min(ie, (__ffs(next) - 1) >> 1) : ie;
+        double acc = *at;
+#pragma unroll 2
+        for (; i < end; ++i) {
+          const double2 a0 = *reinterpret_cast<const double2*>(q), b0 = *reinterpret_cast<const double2*>(q + cb);
+          const double2 a1 = *reinterpret_cast<const double2*>(q + kLane);
+          const double2 b1 = *reinterpret_cast<const double2*>(q + kLane + cb);
+          acc = acc + a0.x * b0.x;
+          acc = acc + a0.y * b0.y;
+          acc = acc + a1.x * b1.x;
+          acc = acc + a1.y * b1.y;
+          q += 2 * kLane;
+        }
+        *at = acc;
+      }
+      __syncwarp();
     }
-    if (u_a && v_b) {
+  }
+  __device__ __forceinline__ void end(char* mem, int n, const int4& rec, int lane) const {
+    const double* blk = reinterpret_cast<const double*>(mem + kBlk);
+    __syncwarp();
+    if (blocks) {
+      for (int s = lane >> 4; s < ((n + 1) & ~1); s += 2) {
+        const int64_t p = __shfl_sync(0xffffffffu, rec.x, s);
+        if (s < n) blocks[p * 16 + (lane & 15)] = blk[16 * s + (lane & 15)];
+      }
+    }
+    if (u_a && v_b && lane < n) {
+      blk += 16 * lane;
       double sv = 0.0;
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        const double ur = u_a[node_of<IDX>(en_a, a, 4, r)];
+        const double ur = u_a[node_of<IDX>(en_a, rec.y, 4, r)];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) sv += ur * blk[r * 4 + c] * v_b[node_of<IDX>(en_b, b, 4, c)];
+        for (int c = 0; c < 4; ++c) sv += ur * blk[r * 4 + c] * v_b[node_of<IDX>(en_b, rec.z, 4, c)];
       }
-      pair_uv[p] = sv;
+      pair_uv[rec.x] = sv;
     }
   }
-  template <int NT>
-  __device__ __forceinline__ void finish() {}
 };
-
 
 // 2D: one pair per thread, clipped with the triangle clipper; per supermesh
 // triangle the degree-2 rule (three points), P1 bases of A and B, 3x3 block.
@@ -4036,20 +4879,6 @@ cudaError_t launch_p2_inner(int64_t npairs, const int32_t* pair_a, const int32_t
   return cudaGetLastError();
 }
 
-// 3D: the index clipper with the P1 sink, one block per SM.  The sink's
-// 4x4 block accumulator and the quadrature raise the register need to about
-// 250: 8 warps (2 per SM sub-partition) can hold them without spilling,
-// while 9-12 warps are capped at 168 registers by the sub-partitions'
-// register files and spill (pool: 256 x 480 B of shared memory).
-#ifndef LSM_IX_P1_BLOCK
-#define LSM_IX_P1_BLOCK 256
-#endif
-constexpr int kIxP1Block = LSM_IX_P1_BLOCK;
-
-size_t p1_smem_bytes() {
-  return (size_t)kIxP1Block * (3 * kIxPoints + IxP1Sink<int32_t, kIxP1Block>::kLaneDoubles) * sizeof(double);
-}
-
 // partials written by launch_p1_mass: one per 2D block, or the fixed-order
 // reduction's blocks in 3D
 int p1_grid_blocks(int dim) { return dim == 2 ? sm_count() * 4 : kReduceBlocks; }
@@ -4060,8 +4889,8 @@ cudaError_t launch_p1_mass(int dim, int64_t npairs, const int32_t* pair_a, const
                            int idx_bytes, const double* u_a, const double* v_b, double* blocks,
                            Partial* partials, cudaStream_t s, int32_t* survivors, unsigned long long* work,
                            const double* faces_a, const double* screen_b, double* pair_uv, const SegList* seg) {
-  const int g = dim == 2 ? p1_grid_blocks(2) : sm_count();
   if (dim == 2) {
+    const int g = p1_grid_blocks(2);
     count_launch();
     if (idx_bytes == 4)
       k_p1_mass<int32_t><<<g, 128, 0, s>>>(npairs, pair_a, pair_b, coords_a, tol_a, coords_b, setup_b, enlist_a, enlist_b, u_a, v_b, blocks, partials);
@@ -4070,7 +4899,7 @@ cudaError_t launch_p1_mass(int dim, int64_t npairs, const int32_t* pair_a, const
     return cudaGetLastError();
   }
   // the early-out pass lists the pairs with output tets (blocks and u^T M v
-  // of the others stay zero), then the index clipper integrates their tets;
+  // of the others stay zero), then the breadth-first clipper integrates their tets;
   // u^T M v per pair is summed in pair order (a fixed-order reduction into
   // reduce_pairs_blocks() partials), so the integral does not depend on the
   // order in which the lanes took the pairs
@@ -4079,22 +4908,17 @@ cudaError_t launch_p1_mass(int dim, int64_t npairs, const int32_t* pair_a, const
   if (blocks && npairs > 0) cudaMemsetAsync(blocks, 0, sizeof(double) * 16 * npairs, s);
   if (uv && npairs > 0) cudaMemsetAsync(pair_uv, 0, sizeof(double) * npairs, s);
   if (npairs > 0)
-    run_prefilter<false, 4>(npairs, nullptr, pair_a, pair_b, coords_a, tol_a, setup_b, nullptr, nullptr, survivors,
+    run_prefilter<false, 4, true>(npairs, nullptr, pair_a, pair_b, coords_a, tol_a, setup_b, nullptr, nullptr, survivors,
                             work, faces_a, screen_b, nullptr, seg, s);
   const bool sg = seg_on(seg) && npairs > 0;
   const int4* list = reinterpret_cast<const int4*>(survivors);
-  count_launch();
-  if (idx_bytes == 4) {
-    using Sk = IxP1Sink<int32_t, kIxP1Block>;
-    Sk sk{coords_a, coords_b, enlist_a, enlist_b, u_a, v_b, blocks, pair_uv};
-    k_clip_tets_ix<Sk, kIxP1Block, 1><<<g, kIxP1Block, p1_smem_bytes(), s>>>(
-        list, sg ? work + 2 : work, coords_a, tol_a, setup_b, sk, work + 1, sg ? seg->table : nullptr);
-  } else {
-    using Sk = IxP1Sink<int64_t, kIxP1Block>;
-    Sk sk{coords_a, coords_b, enlist_a, enlist_b, u_a, v_b, blocks, pair_uv};
-    k_clip_tets_ix<Sk, kIxP1Block, 1><<<g, kIxP1Block, p1_smem_bytes(), s>>>(
-        list, sg ? work + 2 : work, coords_a, tol_a, setup_b, sk, work + 1, sg ? seg->table : nullptr);
-  }
+  const int4* table = sg ? seg->table : nullptr;
+  if (idx_bytes == 4)
+    run_bf(list, sg ? work + 2 : work, coords_a, tol_a, setup_b,
+           BfP1Sink<int32_t>{coords_a, coords_b, enlist_a, enlist_b, u_a, v_b, blocks, pair_uv}, work + 1, table, s);
+  else
+    run_bf(list, sg ? work + 2 : work, coords_a, tol_a, setup_b,
+           BfP1Sink<int64_t>{coords_a, coords_b, enlist_a, enlist_b, u_a, v_b, blocks, pair_uv}, work + 1, table, s);
   if (uv) {
     count_launch();
     k_reduce_pairs<<<kReduceBlocks, 256, 0, s>>>(npairs, pair_uv, nullptr, partials, nullptr);
@@ -4105,12 +4929,8 @@ cudaError_t launch_p1_mass(int dim, int64_t npairs, const int32_t* pair_a, const
 }
 
 cudaError_t init_p1_attributes() {
-  const int smem = (int)p1_smem_bytes();
-  cudaError_t e = cudaFuncSetAttribute(k_clip_tets_ix<IxP1Sink<int32_t, kIxP1Block>, kIxP1Block, 1>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_clip_tets_ix<IxP1Sink<int64_t, kIxP1Block>, kIxP1Block, 1>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = bf_attributes<BfP1Sink<int32_t>>();
+  if (e == cudaSuccess) e = bf_attributes<BfP1Sink<int64_t>>();
   return e;
 }
 

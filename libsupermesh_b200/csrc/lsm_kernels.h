@@ -295,7 +295,7 @@ cudaError_t launch_p2_inner(int64_t npairs, const int32_t* pair_a, const int32_t
 cudaError_t launch_check_index(int64_t n, const void* en, int idx_bytes, int64_t limit, int* bad, cudaStream_t s);
 // P1-P1 mixed mass: 2D clips every pair; 3D runs the exact early-out pass
 // (survivors: 4 ints per pair, work: two counters (three with seg),
-// faces_a / screen_b / seg as for launch_clip) and the index clipper with the quadrature on the survivors,
+// faces_a / screen_b / seg as for launch_clip) and the breadth-first clipper with the quadrature on the survivors,
 // with blocks of the other pairs zero-filled; 3D with u_a and v_b also needs
 // pair_uv [npairs] (u^T M v per pair, summed in pair order).  partials:
 // p1_grid_blocks(dim) entries.

@@ -1,0 +1,82 @@
+"""The breadth-first tet clipper (k_clip_tets_bf) at the edges of its batches
+and on inputs outside the ordinary: against the one-launch clipper that
+batches below 2048 pairs take, and the P1 mass blocks against the oracle.
+Both sides run the same operations in the same order, so every comparison is
+exact."""
+import numpy as np
+import pytest
+
+from libsupermesh_b200 import meshes as M
+
+pytestmark = pytest.mark.gpu
+
+
+def _pairs(n, seed):
+    """n pairs of overlapping tets: runs of 1 to 40 pairs with the same A,
+    among them A inside B, A equal to B, shared faces and vertices, and
+    elements with a repeated vertex."""
+    rng = np.random.default_rng(seed)
+    a = np.empty((n, 4, 3))
+    b = rng.random((n, 4, 3))
+    i = 0
+    while i < n:
+        k = int(rng.integers(1, 41))
+        a[i:i + k] = rng.random((4, 3))
+        i += k
+    kind = rng.integers(0, 12, n)
+    a[kind == 0] = 0.4 + 0.01 * rng.random((int((kind == 0).sum()), 4, 3))
+    b[kind == 0] = np.array([[-2, -2, -2], [5, 0, 0], [0, 5, 0], [0, 0, 5]])
+    b[kind == 1] = a[kind == 1]
+    b[kind == 2, :3] = a[kind == 2, :3]
+    b[kind == 3, 2] = a[kind == 3, 1]
+    b[kind == 4, 3] = b[kind == 4, 0]
+    a[kind == 5, 3] = a[kind == 5, 1]
+    return a, b
+
+
+def _small(ctx, a, b):
+    """The same pairs through the one-launch clipper, 2000 at a time."""
+    r = [ctx.intersect_pairs(3, a[i:i + 2000], b[i:i + 2000], want_elems=True) for i in range(0, len(a), 2000)]
+    return [np.concatenate(x) for x in zip(*r)]
+
+
+def _same(got, ref):
+    assert np.array_equal(got[1], ref[1])
+    assert np.array_equal(got[0], ref[0])
+    if got[2] is not None:
+        used = np.arange(81)[None] < got[1][:, None]
+        assert np.array_equal(got[2][used], ref[2][used])
+
+
+@pytest.mark.parametrize("n", [2048, 2049, 2079, 2081, 2111, 2113, 5003])
+@pytest.mark.parametrize("elems", [False, True])
+def test_batches_match_one_launch_clipper(gpu_ctx, n, elems):
+    a, b = _pairs(n, n)
+    _same(gpu_ctx.intersect_pairs(3, a, b, want_elems=elems), _small(gpu_ctx, a, b))
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf, 1e200])
+def test_coordinates_that_are_not_finite(gpu_ctx, value):
+    """Some vertices of A with a coordinate that is not finite, or whose
+    products overflow."""
+    a, b = _pairs(2300, 5)
+    rng = np.random.default_rng(6)
+    rows = rng.choice(len(a), 700, replace=False)
+    a[rows, rng.integers(0, 4, 700), rng.integers(0, 3, 700)] = value
+    _same(gpu_ctx.intersect_pairs(3, a, b, want_elems=True), _small(gpu_ctx, a, b))
+
+
+@pytest.mark.parametrize("na,nb,ja,jb,scale", [
+    (4, 4, 0.0, 0.0, 1.0),       # identical regular meshes: vertices and edges coincide
+    (4, 6, 0.0, 0.25, 1.0),
+    (7, 5, 0.25, 0.25, 2.0 ** -250),  # far from 1 in both directions
+    (5, 6, 0.2, 0.0, 2.0 ** 100),
+])
+def test_p1_blocks_match_oracle(gpu_ctx, oracle_mod, na, nb, ja, jb, scale):
+    A, B = M.grid3d(na, 3, ja), M.grid3d(nb, 2, jb)
+    A, B = (A[0] * scale, A[1]), (B[0] * scale, B[1])
+    u, v = np.cos(np.arange(len(A[0]))), np.sin(np.arange(len(B[0])))
+    val, blocks = gpu_ctx.p1_mass(A, B, u, v, want_blocks=True)
+    ip, ind = gpu_ctx.get_candidates(len(A[1]), len(blocks))
+    _, _, ref = oracle_mod.p1_mass(3, A, B, ip, ind, u, v, want_blocks=True)
+    assert np.array_equal(blocks, ref.reshape(blocks.shape))
