@@ -3,8 +3,8 @@
 //
 // Pipeline per mesh pair (all on one stream):
 //   prep A, prep B            gather coords, boxes, tolerances, B clip setup
-//   root box, Morton, sort    LBVH leaves in Morton order
-//   LBVH build + refit
+//   root box, Morton, sort    leaves in Morton order
+//   box hierarchy over them
 //   query (count) -> scan -> [host reads n_candidates] -> query (fill)
 //   clip (+ overflow re-run) -> finalize (compensated totals, counts)
 // The only host synchronisation inside the pipeline is the read of the
@@ -70,7 +70,7 @@ struct Ctx {
   // mesh B (tree side)
   DevBuf b_pos, b_en, b_coords, b_box64, b_box32, b_setup, b_screen;
   // tree
-  DevBuf keys, vals, keys_tmp, vals_tmp, hist, root_partial, rootbox, bvh_lo, bvh_work, bvh_leaf;
+  DevBuf keys, vals, keys_tmp, vals_tmp, hist, root_partial, rootbox, tree_rec;
   // candidates
   DevBuf counts, offsets, scan_tmp, pair_a, pair_b, i64_tmp, q_cache, q_over, q_pool, q_next, q_first;
   // narrow phase
@@ -85,7 +85,7 @@ struct Ctx {
   DevBuf x_setup, x_tol, x_iota, x_faces, x_screen, x_list;  // explicit tet pairs through the early-out pass
   DevBuf x_sub;  // hexahedron pairs: A's five tets
   DevBuf elem_off, x_pa, x_pb;  // supermesh elements: per-pair offsets, parents
-  DevBuf bt_tabs, bt_pair_a, bt_pair_b, bt_mort, bt_codes, bt_roots, bt_stops, bt_tot, bt_ncand, bt_indptr;
+  DevBuf bt_tabs, bt_pair_a, bt_pair_b, bt_tot, bt_ncand, bt_indptr;
   // host meshes of a batch staged on the device, one set per dimension (the
   // 3D set is copied on the side stream while the 2D group computes)
   DevBuf bt_stage_pa[2], bt_stage_ea[2], bt_stage_pb[2], bt_stage_eb[2];
@@ -281,13 +281,13 @@ void fini_ctx(Ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   DevBuf* all[] = {&c->a_pos, &c->a_en, &c->a_coords, &c->a_box64, &c->a_tol, &c->b_pos, &c->b_en,
                    &c->b_coords, &c->b_box64, &c->b_box32, &c->b_setup, &c->keys, &c->vals,
-                   &c->keys_tmp, &c->vals_tmp, &c->hist, &c->root_partial, &c->rootbox, &c->bvh_lo,
-                   &c->bvh_work, &c->bvh_leaf, &c->counts, &c->offsets, &c->scan_tmp, &c->pair_a,
+                   &c->keys_tmp, &c->vals_tmp, &c->hist, &c->root_partial, &c->rootbox, &c->tree_rec,
+                   &c->counts, &c->offsets, &c->scan_tmp, &c->pair_a,
                    &c->pair_b, &c->i64_tmp, &c->pair_measure, &c->pair_nout, &c->partials,
                    &c->ovf_list, &c->p1_list, &c->misc, &c->elem_measure, &c->totals, &c->x_a, &c->x_b, &c->x_measure,
                    &c->x_nout, &c->x_elems, &c->x_setup, &c->x_tol, &c->x_iota, &c->x_faces, &c->x_screen,
                    &c->x_list, &c->elem_off, &c->x_pa, &c->x_pb, &c->u_a, &c->v_b, &c->blocks, &c->bt_tabs, &c->bt_pair_a,
-                   &c->bt_pair_b, &c->bt_mort, &c->bt_codes, &c->bt_roots, &c->bt_stops, &c->bt_tot,
+                   &c->bt_pair_b, &c->bt_tot,
                    &c->bt_ncand, &c->bt_stage_pa[0], &c->bt_stage_ea[0], &c->bt_stage_pb[0],
                    &c->bt_stage_eb[0], &c->bt_stage_pa[1], &c->bt_stage_ea[1], &c->bt_stage_pb[1],
                    &c->bt_stage_eb[1],
@@ -504,31 +504,25 @@ void prep_chunks(Ctx* c, const MeshDev& d, int chunks, const cudaEvent_t* ev, cu
   }
 }
 
-lsm::BVH build_tree(Ctx* c, const MeshDev& b, cudaStream_t s) {
+lsm::Tree build_tree(Ctx* c, const MeshDev& b, cudaStream_t s) {
   const int64_t n = b.nel;
-  lsm::BVH bvh;
-  bvh.n = (int)n;
-  if (n == 0) return bvh;
+  if (n == 0) return lsm::Tree{};
   const int dim = b.dim;
   uint32_t* keys = ensure<uint32_t>(c, c->keys, n);
-  int32_t* vals = ensure<int32_t>(c, c->vals, n);
+  int32_t* vals = ensure<int32_t>(c, c->vals, n + 3);
   uint32_t* kt = ensure<uint32_t>(c, c->keys_tmp, n);
   int32_t* vt = ensure<int32_t>(c, c->vals_tmp, n);
   uint32_t* hist = ensure<uint32_t>(c, c->hist, lsm::radix_hist_entries(n));
   const int pcap = 4096;
   double* part = ensure<double>(c, c->root_partial, (int64_t)pcap * 2 * dim);
-  double* root = ensure<double>(c, c->rootbox, 2 * dim);
-  CU(lsm::launch_root_box(dim, n, static_cast<double*>(c->b_box64.p), part, pcap, root, s));
+  double* root = ensure<double>(c, c->rootbox, 2 * dim + 1);
+  unsigned* ticket = reinterpret_cast<unsigned*>(root + 2 * dim);
+  CU(lsm::launch_root_box(dim, n, static_cast<double*>(c->b_box64.p), part, pcap, root, ticket, s));
   CU(lsm::launch_morton(dim, n, static_cast<double*>(c->b_box64.p), root, keys, vals, s));
   CU(lsm::radix_sort_pairs(n, dim == 2 ? 32 : 30, keys, vals, kt, vt, hist, s, bad_flag(c) + 3));
-  bvh.lo_left = ensure<float4>(c, c->bvh_lo, 2 * (2 * n - 1));
-  bvh.hi_esc = bvh.lo_left + 1;
-  bvh.leaf = ensure<double>(c, c->bvh_leaf, 8 * n);
-  int* work = ensure<int>(c, c->bvh_work, 8 * n);
-  bvh.bucket = lsm::tree_bucket((int)n, true);
-  CU(lsm::launch_bvh_build(dim, (int)n, keys, vals, static_cast<float*>(c->b_box32.p), bvh, work, s,
-                           static_cast<double*>(c->b_box64.p)));
-  return bvh;
+  const lsm::Tree tree = lsm::make_tree(dim, (int)n, vals, ensure<float>(c, c->tree_rec, lsm::tree_floats(dim, n)));
+  CU(lsm::launch_tree_build(dim, tree, static_cast<float*>(c->b_box32.p), ticket, s));
+  return tree;
 }
 
 // Gather, sort by left end (stable) and take sorted left/right ends of one
@@ -594,7 +588,7 @@ void find_candidates_1d(Ctx* c, const MeshDev& a, const MeshDev& b, cudaStream_t
 
 // Broad phase: candidates as CSR (offsets) + pair arrays.  1D meshes (and
 // intervals = true, the sort finder's entry) take the sort-and-sweep
-// search, 2D/3D the LBVH search.
+// search, 2D/3D the box hierarchy search.
 void find_candidates(Ctx* c, const lsm_gpu_mesh* ma, const lsm_gpu_mesh* mb, int on_device, bool simplex,
                      bool want_b_coords, cudaStream_t s, bool intervals = false) {
   intervals = intervals || (ma && ma->dim == 1);
@@ -652,7 +646,7 @@ void find_candidates(Ctx* c, const lsm_gpu_mesh* ma, const lsm_gpu_mesh* mb, int
   int64_t* offsets = ensure<int64_t>(c, c->offsets, nel_a + 1);
   int* counts = ensure<int>(c, c->counts, nel_a);
   int64_t* stmp = ensure<int64_t>(c, c->scan_tmp, lsm::scan_tmp_entries(nel_a) + 1);
-  lsm::BVH bvh{};
+  lsm::Tree tree;
   // candidate cache of the count pass: at most 256 per row
   const int cap = nel_a > 0 ? (int)std::min<int64_t>(256, cache_budget(c) / (4 * nel_a)) : 0;
   int32_t* cache = cap >= 8 ? ensure<int32_t>(c, c->q_cache, nel_a * cap) : nullptr;
@@ -661,10 +655,10 @@ void find_candidates(Ctx* c, const lsm_gpu_mesh* ma, const lsm_gpu_mesh* mb, int
   // chunks: its long rows are traversed again)
   const lsm::Spill spill{};
   if (b.nel > 0 && nel_a > 0) {
-    bvh = build_tree(c, b, s);
+    tree = build_tree(c, b, s);
     if (over) CU(cudaMemsetAsync(over, 0, sizeof(int), s));
     CU(cudaStreamWaitEvent(s, c->side_ev[1], 0));
-    CU(lsm::launch_query(a.dim, false, nel_a, static_cast<double*>(c->a_box64.p), bvh,
+    CU(lsm::launch_query(a.dim, false, nel_a, static_cast<double*>(c->a_box64.p), tree,
                          static_cast<double*>(c->b_box64.p), counts, nullptr, nullptr, nullptr, s, cache, cap,
                          over, spill));
   } else {
@@ -686,7 +680,7 @@ void find_candidates(Ctx* c, const lsm_gpu_mesh* ma, const lsm_gpu_mesh* mb, int
   int32_t* pa = ensure<int32_t>(c, c->pair_a, nnz);
   int32_t* pb = ensure<int32_t>(c, c->pair_b, nnz);
   if (nnz > 0)
-    CU(lsm::launch_query(a.dim, true, nel_a, static_cast<double*>(c->a_box64.p), bvh,
+    CU(lsm::launch_query(a.dim, true, nel_a, static_cast<double*>(c->a_box64.p), tree,
                          static_cast<double*>(c->b_box64.p), counts, offsets, pa, pb, s, cache, cap, over,
                          spill));
   c->dim = a.dim;
@@ -897,9 +891,10 @@ struct BatchOut {
 };
 
 // All mesh pairs of one dimension through each phase in one launch:
-// batched prep (pointer tables), one sort by (mesh, Morton), one LBVH with a
-// subtree per mesh, one traversal, the usual clipper over all candidates,
-// and a per-mesh-pair reduction.  One host synchronisation (candidate count).
+// batched prep (pointer tables), one sort by (mesh, Morton), one box
+// hierarchy over all meshes, one traversal (each row within its mesh's range
+// of leaves), the usual clipper over all candidates, and a per-mesh-pair
+// reduction.  One host synchronisation (candidate count).
 // staged: the device addresses from stage_batch_group (host meshes), or
 // null when the meshes are on the device.
 // Pinned area a launched group's results are copied to: totals[nm],
@@ -1039,38 +1034,26 @@ bool run_batch_group(Ctx* c, int dim, const std::vector<int>& idx, const lsm_gpu
   CU(lsm::launch_prep_batched(dim, nb, nm, d_eob, d_ptb, d_etb, d_nnb, ib, b_coords, b_box, b_box32, nullptr,
                               b_setup, pair_of_b, bad, s, nullptr, b_screen));
   // tree over all B meshes
-  lsm::BVH bvh;
-  bvh.n = (int)nb;
-  int* roots = ensure<int>(c, c->bt_roots, nm);
-  int* stops = ensure<int>(c, c->bt_stops, nm);
+  lsm::Tree tree;
   if (nb > 0) {
     uint32_t* keys = ensure<uint32_t>(c, c->keys, nb);
-    int32_t* vals = ensure<int32_t>(c, c->vals, nb);
+    int32_t* vals = ensure<int32_t>(c, c->vals, nb + 3);
     uint32_t* kt = ensure<uint32_t>(c, c->keys_tmp, nb);
     int32_t* vt = ensure<int32_t>(c, c->vals_tmp, nb);
     uint32_t* hist = ensure<uint32_t>(c, c->hist, lsm::radix_hist_entries(nb));
-    uint32_t* mort = ensure<uint32_t>(c, c->bt_mort, nb);
     const int pcap = 4096;
     double* part = ensure<double>(c, c->root_partial, (int64_t)pcap * 2 * dim);
-    double* root = ensure<double>(c, c->rootbox, 2 * dim);
-    CU(lsm::launch_root_box(dim, nb, b_box, part, pcap, root, s));
+    double* root = ensure<double>(c, c->rootbox, 2 * dim + 1);
+    unsigned* ticket = reinterpret_cast<unsigned*>(root + 2 * dim);
+    CU(lsm::launch_root_box(dim, nb, b_box, part, pcap, root, ticket, s));
     CU(lsm::launch_morton(dim, nb, b_box, root, keys, vals, s));
-    CU(cudaMemcpyAsync(mort, keys, sizeof(uint32_t) * nb, cudaMemcpyDeviceToDevice, s));
     CU(lsm::radix_sort_pairs(nb, dim == 2 ? 32 : 30, keys, vals, kt, vt, hist, s, bad + 3));
     int mbits = 1;
     while ((1 << mbits) < nm) ++mbits;
     CU(lsm::launch_pair_keys(nb, vals, pair_of_b, keys, s));
     CU(lsm::radix_sort_pairs(nb, mbits, keys, vals, kt, vt, hist, s, bad + 3));
-    bvh.lo_left = ensure<float4>(c, c->bvh_lo, 2 * (2 * nb - 1));
-    bvh.hi_esc = bvh.lo_left + 1;
-    bvh.leaf = ensure<double>(c, c->bvh_leaf, 8 * nb);
-    int* work = ensure<int>(c, c->bvh_work, 8 * nb);
-    unsigned long long* codes = ensure<unsigned long long>(c, c->bt_codes, nb);
-    CU(lsm::launch_batched_tree((int)nb, nm, vals, pair_of_b, mort, codes, b_box32, d_eob, bvh, work, roots,
-                                stops, s, dim, b_box, bad + 3));
-  } else {
-    CU(cudaMemsetAsync(roots, 0xff, sizeof(int) * nm, s));
-    CU(cudaMemsetAsync(stops, 0xff, sizeof(int) * nm, s));
+    tree = lsm::make_tree(dim, (int)nb, vals, ensure<float>(c, c->tree_rec, lsm::tree_floats(dim, nb)));
+    CU(lsm::launch_tree_build(dim, tree, b_box32, ticket, s));
   }
   int64_t* offsets = ensure<int64_t>(c, c->offsets, na + 1);
   int* counts = ensure<int>(c, c->counts, na);
@@ -1082,7 +1065,7 @@ bool run_batch_group(Ctx* c, int dim, const std::vector<int>& idx, const lsm_gpu
   const lsm::Spill spill = cache ? make_spill(c, na, cap) : lsm::Spill{};
   if (na > 0 && nb > 0) {
     if (over) CU(cudaMemsetAsync(over, 0, sizeof(int), s));
-    CU(lsm::launch_query_batched(dim, false, na, a_box, pair_of_a, roots, stops, bvh, b_box, counts, nullptr,
+    CU(lsm::launch_query_batched(dim, false, na, a_box, pair_of_a, d_eob, tree, b_box, counts, nullptr,
                                  nullptr, nullptr, s, cache, cap, over, spill));
   }
   else if (na > 0)
@@ -1105,7 +1088,7 @@ bool run_batch_group(Ctx* c, int dim, const std::vector<int>& idx, const lsm_gpu
   int32_t* pa = ensure<int32_t>(c, c->pair_a, nnz);
   int32_t* pb = ensure<int32_t>(c, c->pair_b, nnz);
   if (nnz > 0)
-    CU(lsm::launch_query_batched(dim, true, na, a_box, pair_of_a, roots, stops, bvh, b_box, counts, offsets,
+    CU(lsm::launch_query_batched(dim, true, na, a_box, pair_of_a, d_eob, tree, b_box, counts, offsets,
                                  pa, pb, s, cache, cap, over, spill, pair_cap > 0 ? pair_cap : INT64_MAX));
   c->dim = dim;
   c->loc_a = c->loc_b = loc;

@@ -6,12 +6,12 @@
 //   K2  radix sort      stable LSD, 8-bit digits, warp-match ranking;
 //                       one digit-count kernel, then one kernel per pass
 //                       with decoupled look-back (k_radix_onesweep)
-//   K3  k_bvh_internal  Karras LBVH hierarchy + rope table;
-//       k_bvh_refit     bottom-up FP32 box refit, escape links, leaf records
-//   K4  k_query         stackless LBVH traversal per A element (FP32,
-//                       outward-rounded boxes) + exact strict FP64 box test
-//                       at the leaf records; the count pass caches rows,
-//                       k_fill_from_cache copies
+//   K3  k_tree_build    four-wide hierarchy of outward-rounded FP32 boxes
+//                       over the sorted leaves
+//   K4  k_query         depth-first traversal per A element, four children a
+//                       visit (k_query_warp: a warp per element, 32), exact
+//                       strict box test at the leaves; the count pass caches
+//                       rows, k_fill_from_cache copies
 //   K5  k_clip_tris     one candidate pair per thread, polygon in shared
 //                       memory, FP64 Sutherland-Hodgman
 //   K6  k_prefilter_tets two exact early-outs and the no-op plane mask;
@@ -68,11 +68,6 @@ int query_block() { return g_query_block; }
 void set_query_block(int v) { g_query_block = v; }
 int leaf_bucket() { return g_leaf_bucket; }
 void set_leaf_bucket(int v) { g_leaf_bucket = v; }
-int tree_bucket(int n, bool leaf_records) {
-  // buckets need the leaf records and fit the node encoding (first leaf
-  // below 2^27, at most 8 leaves)
-  return leaf_records && g_leaf_bucket > 1 && n < (1 << 27) ? g_leaf_bucket : 1;
-}
 
 void count_launch(int n) { __atomic_fetch_add(&g_launches, (unsigned long long)n, __ATOMIC_RELAXED); }
 
@@ -415,7 +410,8 @@ __global__ void k_root_partial(int64_t nel, const double* __restrict__ box64, do
 }
 
 template <int DIM>
-__global__ void __launch_bounds__(256) k_root_final(int np, const double* partial, double* root) {
+__global__ void __launch_bounds__(256) k_root_final(int np, const double* partial, double* root,
+                                                    unsigned* ticket) {
   double lo[DIM], hi[DIM];
 #pragma unroll
   for (int c = 0; c < DIM; ++c) {
@@ -445,6 +441,7 @@ __global__ void __launch_bounds__(256) k_root_final(int np, const double* partia
     }
   __syncthreads();
   if (threadIdx.x == 0) {
+    *ticket = 0;
     for (int w = 1; w < 8; ++w)
 #pragma unroll
       for (int c = 0; c < DIM; ++c) {
@@ -460,17 +457,17 @@ __global__ void __launch_bounds__(256) k_root_final(int np, const double* partia
 }
 
 cudaError_t launch_root_box(int dim, int64_t nel, const double* box64, double* partial,
-                            int partial_cap, double* rootbox, cudaStream_t s) {
+                            int partial_cap, double* rootbox, unsigned* ticket, cudaStream_t s) {
   const int B = 256;
   int g = grid_for(nel, B, 2);
   if (g > partial_cap) g = partial_cap;
   count_launch(2);
   if (dim == 2) {
     k_root_partial<2><<<g, B, 0, s>>>(nel, box64, partial);
-    k_root_final<2><<<1, 256, 0, s>>>(g, partial, rootbox);
+    k_root_final<2><<<1, 256, 0, s>>>(g, partial, rootbox, ticket);
   } else {
     k_root_partial<3><<<g, B, 0, s>>>(nel, box64, partial);
-    k_root_final<3><<<1, 256, 0, s>>>(g, partial, rootbox);
+    k_root_final<3><<<1, 256, 0, s>>>(g, partial, rootbox, ticket);
   }
   return cudaGetLastError();
 }
@@ -750,190 +747,173 @@ cudaError_t radix_sort_pairs(int64_t n, int bits, uint32_t* keys, int32_t* vals,
 }
 
 // ======================================================================
-// K3: LBVH (Karras 2012) + ropes + refit
+// K3: four-wide box hierarchy over the sorted leaves
 // ======================================================================
-// Node ids: internal i in [0, n-2]; leaf k -> (n-1) + k.  Root = node 0.
-__device__ __forceinline__ int bvh_delta(const uint32_t* __restrict__ codes, int n, int i, int j) {
-  if (j < 0 || j >= n) return -1;
-  const uint32_t a = codes[i], b = codes[j];
-  if (a != b) return __clz(a ^ b);
-  return 32 + __clz((uint32_t)i ^ (uint32_t)j);
-}
-
-// work layout (ints): parent[2n-1] | rope[n] | visit[n] | last[n] | left[n] | right[n] | first[n]
-__global__ void k_bvh_internal(int n, const uint32_t* __restrict__ codes, int* parent, int* rope,
-                               int* last, int* left, int* right, int* first_leaf) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n - 1) return;
-  const int d = (bvh_delta(codes, n, i, i + 1) - bvh_delta(codes, n, i, i - 1)) >= 0 ? 1 : -1;
-  const int dmin = bvh_delta(codes, n, i, i - d);
-  int lmax = 2;
-  while (bvh_delta(codes, n, i, i + lmax * d) > dmin) lmax <<= 1;
-  int l = 0;
-  for (int t = lmax >> 1; t >= 1; t >>= 1)
-    if (bvh_delta(codes, n, i, i + (l + t) * d) > dmin) l += t;
-  const int j = i + l * d;
-  const int dnode = bvh_delta(codes, n, i, j);
-  int s = 0;
-  int t = l;
-  do {
-    t = (t + 1) >> 1;
-    if (bvh_delta(codes, n, i, i + (s + t) * d) > dnode) s += t;
-  } while (t > 1);
-  const int gamma = i + s * d + (d < 0 ? -1 : 0);
-  const int first = i < j ? i : j;
-  const int lst = i < j ? j : i;
-  const int lc = (first == gamma) ? (n - 1) + gamma : gamma;
-  const int rc = (lst == gamma + 1) ? (n - 1) + gamma + 1 : gamma + 1;
-  left[i] = lc;
-  right[i] = rc;
-  parent[lc] = i;
-  parent[rc] = i;
-  rope[gamma + 1] = rc;
-  last[i] = lst;
-  if (first_leaf) first_leaf[i] = first;
-}
-
-__device__ __forceinline__ int bvh_escape(int n, int node, const int* __restrict__ rope, const int* __restrict__ last) {
-  const int r = node >= n - 1 ? node - (n - 1) : last[node];
-  return r == n - 1 ? -1 : rope[r + 1];
-}
-
-constexpr int kRefitBlock = 256;
-
-template <bool BUCKET>
-__global__ void __launch_bounds__(kRefitBlock) k_bvh_refit(int n, const int32_t* __restrict__ sorted_vals, const float4* __restrict__ box32,
-                            const int* __restrict__ parent, const int* __restrict__ rope,
-                            const int* __restrict__ last, const int* __restrict__ left,
-                            const int* __restrict__ right, int* visit, float4* lo_left, float4* hi_esc,
-                            int dim, const double* __restrict__ box64, double* leaf,
-                            const int* __restrict__ first_leaf, int bucket) {
-  // Nodes whose leaf range lies within this block's 256 leaves are merged
-  // through shared memory (block-scope counters and boxes) when first_leaf
-  // is given; the climb above them uses the device-scope counters.  Node i
-  // is an end of its own range, so an in-block node i has i - L in [0, 256).
-  __shared__ float4 s_lo[2 * kRefitBlock], s_hi[2 * kRefitBlock];  // leaves, then internal nodes
-  __shared__ int s_vis[kRefitBlock];
-  const int L = blockIdx.x * kRefitBlock;
-  const int R = (L + kRefitBlock < n ? L + kRefitBlock : n) - 1;
-  s_vis[threadIdx.x] = 0;
-  __syncthreads();
-  const int k = L + threadIdx.x;
-  if (k >= n) return;
-  const int elem = sorted_vals[k];
-  int node = (n - 1) + k;
-  float4 lo = box32[2 * elem], hi = box32[2 * elem + 1];
-  lo.w = __int_as_float(elem);
-  hi.w = __int_as_float(bvh_escape(n, node, rope, last));
-  lo_left[2 * node] = lo;
-  hi_esc[2 * node] = hi;
-  s_lo[threadIdx.x] = lo;
-  s_hi[threadIdx.x] = hi;
-  if (leaf) {
-    // leaf record in sorted order: FP64 box (lo at 0.., hi at 3..), element, escape
-    double* o = leaf + (int64_t)k * 8;
-    for (int c = 0; c < 3; ++c) {
-      o[c] = c < dim ? box64[(int64_t)elem * 2 * dim + c] : 0.0;
-      o[3 + c] = c < dim ? box64[(int64_t)elem * 2 * dim + dim + c] : 0.0;
-    }
-    reinterpret_cast<int2*>(o + 6)[0] = make_int2(elem, __float_as_int(hi.w));
-    o[7] = 0.0;
+// Level 0 is the leaves in Morton order; node j of level l+1 holds nodes 4j ..
+// 4j+3 of level l, up to the first level of at most four nodes.  A group of
+// four siblings is one record of their outward-rounded FP32 boxes, component
+// by component (lo.x of the four, lo.y, .., hi.z: six float4 in 3D, four in
+// 2D), so that a visit is one round of independent 16-byte loads and decides
+// four children at once; nodes past the end have empty boxes.  The search
+// waits for its chain of dependent visits, and this takes about a third of
+// those of a binary hierarchy with escape links, one node at a time; the
+// hierarchy follows from the sorted order alone, where the binary one was
+// built by two searches per node and a bottom-up merge over one counter per
+// node.  Search of tet3d_graded_55x51 / tri2d_777x1024_rot7: 1.85 -> 1.76 / 1.20 -> 0.76 ms.
+template <int DIM>
+__device__ __forceinline__ void tree_put(float* __restrict__ rec, int64_t node, const float (&lo)[3],
+                                         const float (&hi)[3]) {
+  float* r = rec + (node >> 2) * (8 * DIM) + (node & 3);
+#pragma unroll
+  for (int c = 0; c < DIM; ++c) {
+    r[4 * c] = lo[c];
+    r[4 * (DIM + c)] = hi[c];
   }
-  if (n == 1) return;
-  int p = parent[node];
-  bool local = first_leaf != nullptr;
-  for (int guard = 0; guard < 128 && p >= 0; ++guard) {
-    if (local) {
-      if (first_leaf[p] >= L && last[p] <= R) {
-        // block scope: this thread's boxes out, the sibling's in
-        __threadfence_block();
-        if (atomicAdd_block(&s_vis[p - L], 1) == 0) return;  // sibling not done yet
-        __threadfence_block();
-        const int lc = left[p], rc = right[p];
-        const int ia = lc >= n - 1 ? lc - (n - 1) - L : kRefitBlock + lc - L;
-        const int ib = rc >= n - 1 ? rc - (n - 1) - L : kRefitBlock + rc - L;
-        const float4 a0 = s_lo[ia], a1 = s_hi[ia], b0 = s_lo[ib], b1 = s_hi[ib];
-        float4 l, h;
-        l.x = fminf(a0.x, b0.x);
-        l.y = fminf(a0.y, b0.y);
-        l.z = fminf(a0.z, b0.z);
-        l.w = __int_as_float(lc);
-        if (BUCKET) {
-          const int f = first_leaf[p], cnt = last[p] - f + 1;
-          if (cnt <= bucket) l.w = __int_as_float((int)(0x80000000u | ((unsigned)(cnt - 1) << 27) | (unsigned)f));
-        }
-        h.x = fmaxf(a1.x, b1.x);
-        h.y = fmaxf(a1.y, b1.y);
-        h.z = fmaxf(a1.z, b1.z);
-        h.w = __int_as_float(bvh_escape(n, p, rope, last));
-        lo_left[2 * p] = l;
-        hi_esc[2 * p] = h;
-        s_lo[kRefitBlock + p - L] = l;
-        s_hi[kRefitBlock + p - L] = h;
-        if (p == 0) return;
-        p = parent[p];
-        continue;
+}
+
+template <int DIM>
+__device__ __forceinline__ void tree_join(const float* __restrict__ rec, int64_t group, float (&lo)[3],
+                                          float (&hi)[3]) {
+  const float4* r = reinterpret_cast<const float4*>(rec + group * (8 * DIM));
+#pragma unroll
+  for (int c = 0; c < DIM; ++c) {
+    const float4 l = __ldcg(r + c), h = __ldcg(r + DIM + c);
+    lo[c] = fminf(fminf(l.x, l.y), fminf(l.z, l.w));
+    hi[c] = fmaxf(fmaxf(h.x, h.y), fmaxf(h.z, h.w));
+  }
+}
+
+constexpr int kTreeBlock = 256;  // threads, one group of leaves each
+
+// Levels 0 to 5 of the block's 1024 leaves; the block that finishes last
+// (*ticket, zero before the launch) builds the levels above.
+template <int DIM>
+__global__ void __launch_bounds__(kTreeBlock) k_tree_build(const __grid_constant__ Tree T, const int32_t* __restrict__ vals,
+                                                           const float4* __restrict__ box32, float* rec,
+                                                           unsigned* ticket) {
+  __shared__ float sl[kTreeBlock][DIM], sh[kTreeBlock][DIM];
+  __shared__ bool s_last;
+  const float inf = __int_as_float(0x7f800000);
+  const int t = threadIdx.x;
+  const int64_t g = (int64_t)blockIdx.x * kTreeBlock + t;
+  const int64_t groups0 = T.off[1];
+  float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
+  if (g < groups0) {
+    float4 L[4], H[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      L[k] = make_float4(inf, inf, inf, 0.0f);
+      H[k] = make_float4(-inf, -inf, -inf, 0.0f);
+      if (4 * g + k < T.n) {
+        const int64_t e = vals[4 * g + k];
+        L[k] = box32[2 * e];
+        H[k] = box32[2 * e + 1];
       }
-      local = false;  // above the block's subtrees: device scope from here on
     }
-    // release: this thread's node boxes; acquire: the sibling's
-    cuda::atomic_ref<int, cuda::thread_scope_device> vis(visit[p]);
-    if (vis.fetch_add(1, cuda::memory_order_acq_rel) == 0) return;  // sibling not done yet
-    const int lc = left[p], rc = right[p];
-    const float4 a0 = __ldcg(&lo_left[2 * lc]), a1 = __ldcg(&hi_esc[2 * lc]);
-    const float4 b0 = __ldcg(&lo_left[2 * rc]), b1 = __ldcg(&hi_esc[2 * rc]);
-    float4 l, h;
-    l.x = fminf(a0.x, b0.x);
-    l.y = fminf(a0.y, b0.y);
-    l.z = fminf(a0.z, b0.z);
-    l.w = __int_as_float(lc);
-    if (BUCKET) {
-      // a subtree of at most `bucket` leaves becomes a bucket: the node
-      // records its first sorted leaf and leaf count instead of its left
-      // child, and the search scans those leaf records in order
-      const int f = first_leaf[p], cnt = last[p] - f + 1;
-      if (cnt <= bucket) l.w = __int_as_float((int)(0x80000000u | ((unsigned)(cnt - 1) << 27) | (unsigned)f));
+    float4* r = reinterpret_cast<float4*>(rec + g * (8 * DIM));
+    r[0] = make_float4(L[0].x, L[1].x, L[2].x, L[3].x);
+    r[1] = make_float4(L[0].y, L[1].y, L[2].y, L[3].y);
+    if (DIM == 3) r[2] = make_float4(L[0].z, L[1].z, L[2].z, L[3].z);
+    r[DIM] = make_float4(H[0].x, H[1].x, H[2].x, H[3].x);
+    r[DIM + 1] = make_float4(H[0].y, H[1].y, H[2].y, H[3].y);
+    if (DIM == 3) r[DIM + 2] = make_float4(H[0].z, H[1].z, H[2].z, H[3].z);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      lo[0] = fminf(lo[0], L[k].x);
+      lo[1] = fminf(lo[1], L[k].y);
+      lo[2] = fminf(lo[2], L[k].z);
+      hi[0] = fmaxf(hi[0], H[k].x);
+      hi[1] = fmaxf(hi[1], H[k].y);
+      hi[2] = fmaxf(hi[2], H[k].z);
     }
-    h.x = fmaxf(a1.x, b1.x);
-    h.y = fmaxf(a1.y, b1.y);
-    h.z = fmaxf(a1.z, b1.z);
-    h.w = __int_as_float(bvh_escape(n, p, rope, last));
-    __stcg(&lo_left[2 * p], l);
-    __stcg(&hi_esc[2 * p], h);
-    if (p == 0) return;
-    p = parent[p];
+  }
+  // thread t < w of step l holds node blockIdx * w + t of level l
+  int w = kTreeBlock;
+  for (int l = 1; l <= T.top; ++l) {
+    const int64_t node = (int64_t)blockIdx.x * w + t;
+    if (t < w) {
+      if ((node >> 2) < T.off[l + 1] - T.off[l]) tree_put<DIM>(rec + (int64_t)T.off[l] * (8 * DIM), node, lo, hi);
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        sl[t][c] = lo[c];
+        sh[t][c] = hi[c];
+      }
+    }
+    if (w == 1) break;
+    w >>= 2;
+    __syncthreads();
+    if (t < w) {
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        lo[c] = fminf(fminf(sl[4 * t][c], sl[4 * t + 1][c]), fminf(sl[4 * t + 2][c], sl[4 * t + 3][c]));
+        hi[c] = fmaxf(fmaxf(sh[4 * t][c], sh[4 * t + 1][c]), fmaxf(sh[4 * t + 2][c], sh[4 * t + 3][c]));
+      }
+    }
+    __syncthreads();
+  }
+  if (T.top <= 4) return;  // one block
+  if (t == 0) {
+    // the block's level-5 node out, then the ticket; the last block's reads
+    // after it
+    __threadfence();
+    s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!s_last) return;
+  // empty nodes fill level 5's last group
+  for (int l = 5; l <= T.top; ++l) {
+    const int64_t groups = T.off[l + 1] - T.off[l];
+    float* r = rec + (int64_t)T.off[l] * (8 * DIM);
+    const int64_t nodes = l == 5 ? gridDim.x : (int64_t)T.off[l] - T.off[l - 1];
+    for (int64_t j = t; j < 4 * groups; j += kTreeBlock) {
+      if (j >= nodes) {
+        const float el[3] = {inf, inf, inf}, eh[3] = {-inf, -inf, -inf};
+        tree_put<DIM>(r, j, el, eh);
+      } else if (l > 5) {
+        tree_join<DIM>(rec + (int64_t)T.off[l - 1] * (8 * DIM), j, lo, hi);
+        tree_put<DIM>(r, j, lo, hi);
+      }
+    }
+    __threadfence();
+    __syncthreads();
   }
 }
 
-cudaError_t launch_bvh_build(int dim, int n, const uint32_t* sorted_keys, const int32_t* sorted_vals,
-                             const float* box32, BVH bvh, int* work, cudaStream_t s, const double* box64) {
-  if (n <= 0) return cudaSuccess;
-  int* parent = work;
-  int* rope = parent + (2 * n - 1);
-  int* visit = rope + n;
-  int* last = visit + n;
-  int* left = last + n;
-  int* right = left + n;
-  cudaMemsetAsync(visit, 0, sizeof(int) * n, s);
-  cudaMemsetAsync(rope, 0xff, sizeof(int) * n, s);  // unset ropes read as "end"
-  count_launch(n > 1 ? 2 : 1);
-  // leaf buckets need the leaf records (box64) and fit the node encoding
-  // (first leaf below 2^27, at most 8 leaves)
-  int* first_leaf = right + n;
-  const bool buckets = tree_bucket(n, box64 != nullptr) > 1;
-  if (n > 1) {
-    k_bvh_internal<<<(n - 1 + 255) / 256, 256, 0, s>>>(n, sorted_keys, parent, rope, last, left, right,
-                                                       first_leaf);
-  }
-  cudaMemsetAsync(parent, 0xff, sizeof(int), s);  // parent[root] = -1
-  if (buckets)
-    k_bvh_refit<true><<<(n + kRefitBlock - 1) / kRefitBlock, kRefitBlock, 0, s>>>(
-        n, sorted_vals, reinterpret_cast<const float4*>(box32), parent, rope, last, left, right, visit, bvh.lo_left,
-        bvh.hi_esc, dim, box64, bvh.leaf, n > 1 ? first_leaf : nullptr, g_leaf_bucket);
+int64_t tree_floats(int dim, int64_t n) {
+  int64_t g = 0, k = n;
+  do {
+    k = (k + 3) / 4;
+    g += k;
+  } while (k > 1);
+  return g * 8 * dim;
+}
+
+Tree make_tree(int dim, int n, const int32_t* sorted_vals, float* rec) {
+  Tree T;
+  T.n = n;
+  T.vals = sorted_vals;
+  T.rec = rec;
+  int64_t k = n;
+  int l = 0;
+  T.off[0] = 0;
+  do {
+    k = (k + 3) / 4;
+    T.off[l + 1] = T.off[l] + (int)k;
+    ++l;
+  } while (k > 1);
+  T.top = l - 1;
+  return T;
+}
+
+cudaError_t launch_tree_build(int dim, const Tree& T, const float* box32, unsigned* ticket, cudaStream_t s) {
+  if (T.n <= 0) return cudaSuccess;
+  const int g = (T.off[1] + kTreeBlock - 1) / kTreeBlock;
+  count_launch();
+  if (dim == 2)
+    k_tree_build<2><<<g, kTreeBlock, 0, s>>>(T, T.vals, reinterpret_cast<const float4*>(box32), T.rec, ticket);
   else
-    k_bvh_refit<false><<<(n + kRefitBlock - 1) / kRefitBlock, kRefitBlock, 0, s>>>(
-        n, sorted_vals, reinterpret_cast<const float4*>(box32), parent, rope, last, left, right, visit, bvh.lo_left,
-        bvh.hi_esc, dim, box64, box64 ? bvh.leaf : nullptr, n > 1 ? first_leaf : nullptr, 1);
+    k_tree_build<3><<<g, kTreeBlock, 0, s>>>(T, T.vals, reinterpret_cast<const float4*>(box32), T.rec, ticket);
   return cudaGetLastError();
 }
 
@@ -975,125 +955,233 @@ __device__ __forceinline__ void cache_put(int32_t* cache, int cap, const Spill& 
   sp.pool[(int64_t)ch * kSpillChunk + o] = w;
 }
 
+// One thread per row, depth first: the pending children of the levels above
+// are four bits each in one 64-bit word.  A leaf's box test is decided in FP32
+// where the outward-rounded boxes leave no doubt, and by the element's FP64
+// box otherwise: the strict test of the reference in either case.  No doubt:
+// a leaf's lower bound b has the FP32 bound L, b <= L + 2^-23 |L| (plus one
+// subnormal); if L < t - 2^-21 |t| - tiny for t = the query's upper bound
+// rounded down, then either |L| <= 2 |t| and b < t, or L < -2 |t| and b < -|t|;
+// likewise for the other sides.
 // The count pass (FILL = false) also keeps the first `cap` candidates of
 // every row in cache[a * cap ..] (when cache is given) and lists rows with
 // more than cap candidates in over_rows; the fill then copies cached rows
 // (k_fill_from_cache) and traverses again only for the listed rows
-// (FILL = true with `rows`).
-// With leaf records (`leaf`, in sorted order: FP64 box, element, escape) a
-// leaf visit is one load that gives the exact box test and the next node;
-// without them it reads the leaf's FP32 node and then the element's FP64
-// box, two dependent loads.  Both give the same candidates in the same order.
-template <int DIM, bool FILL, bool BUCKET>
-__global__ void __launch_bounds__(256) k_query(int64_t nel_a, const double* __restrict__ box64_a,
-                                               const float4* __restrict__ lo_left,
-                                               const float4* __restrict__ hi_esc, int n,
+// (FILL = true with `rows`).  MESH: rows of mesh pair_of_a[a] take only the
+// leaves of that B mesh, mesh_off[m] .. mesh_off[m+1]-1 in sorted order, and
+// may spill (cache_put).
+template <int DIM, bool FILL, bool MESH>
+__global__ void __launch_bounds__(256) k_query(int64_t nel_a, const double* __restrict__ box64_a, const __grid_constant__ Tree T,
                                                const double* __restrict__ box64_b, int* counts,
                                                const int64_t* __restrict__ offsets, int32_t* pair_a,
                                                int32_t* pair_b, int32_t* cache, int cap,
-                                               const int32_t* __restrict__ rows, int* over_rows,
-                                               const double* __restrict__ leaf, int64_t pair_cap) {
+                                               const int32_t* __restrict__ rows, int* over_rows, int64_t pair_cap,
+                                               const int32_t* __restrict__ pair_of_a,
+                                               const int64_t* __restrict__ mesh_off, Spill sp) {
   const int64_t nrows = rows ? (int64_t)*over_rows : nel_a;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows;
        r += (int64_t)gridDim.x * blockDim.x) {
     const int64_t a = rows ? rows[r] : r;
-    double lo[DIM], hi[DIM];
+    const double* qb = box64_a + a * 2 * DIM;
+    // the query box, rounded outwards, and inwards by the margin
+    float ql[DIM], qh[DIM], il[DIM], ih[DIM];
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
-      lo[c] = box64_a[a * 2 * DIM + c];
-      hi[c] = box64_a[a * 2 * DIM + DIM + c];
+      const double lo = qb[c], hi = qb[DIM + c];
+      const float l = __double2float_ru(lo), h = __double2float_rd(hi);
+      ql[c] = __double2float_rd(lo);
+      qh[c] = __double2float_ru(hi);
+      il[c] = fmaf(fabsf(l), 0x1p-21f, l) + 0x1p-140f;
+      ih[c] = fmaf(fabsf(h), -0x1p-21f, h) - 0x1p-140f;
     }
-    float ql[3], qh[3];
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      ql[c] = __double2float_rd(lo[c]);
-      qh[c] = __double2float_ru(hi[c]);
+    int first = 0, last = T.n - 1;
+    if (MESH) {
+      const int m = pair_of_a[a];
+      first = (int)mesh_off[m];
+      last = (int)mesh_off[m + 1] - 1;
     }
     int cnt = 0;
-    int64_t out = FILL ? offsets[a] : 0;
-    int node = 0;
-    // Each step moves forward in depth-first order; 2n-1 nodes bound it.
-    const int nodes = 2 * n - 1;
-    for (int guard = 0; node >= 0 && guard < 2 * n + 1; ++guard) {
-      if (node >= nodes) break;  // never taken for a well-formed hierarchy
-      if (leaf && node >= n - 1) {
-        const double2* q = reinterpret_cast<const double2*>(leaf + (int64_t)(node - (n - 1)) * 8);
-        const double2 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q3 = __ldg(q + 3);
-        const double blo[3] = {q0.x, q0.y, q1.x}, bhi[3] = {q1.y, q2.x, q2.y};
-        const int2 meta = make_int2(__double2loint(q3.x), __double2hiint(q3.x));
-        bool ex = true;
+    const int64_t out = FILL ? offsets[a] : 0;
+    int chunk = -1;     // MESH: current spill chunk of this row
+    bool lost = false;  // MESH: the row goes to the second traversal
+    int lvl = T.top, grp = 0;
+    unsigned long long pending = 0;  // levels lvl + 1 and up, lowest first
+    while (first <= last) {
+      const float4* g = reinterpret_cast<const float4*>(T.rec) + ((int64_t)T.off[lvl] + grp) * (2 * DIM);
+      float4 L[DIM], H[DIM];
 #pragma unroll
-        for (int c = 0; c < DIM; ++c) ex = ex && (hi[c] > blo[c]) && (lo[c] < bhi[c]);
-        if (ex) {
-          if (FILL) {
-            if (out + cnt < pair_cap) {
-              pair_a[out + cnt] = (int32_t)a;
-              pair_b[out + cnt] = meta.x;
-            }
-          } else if (cache) {
-            if (cnt < cap) cache[a * cap + cnt] = meta.x;
-          }
-          ++cnt;
-        }
-        node = meta.y;
+      for (int c = 0; c < DIM; ++c) {
+        L[c] = __ldg(g + c);
+        H[c] = __ldg(g + DIM + c);
+      }
+      bool o0 = true, o1 = true, o2 = true, o3 = true;
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        o0 = o0 && H[c].x > ql[c] && L[c].x < qh[c];
+        o1 = o1 && H[c].y > ql[c] && L[c].y < qh[c];
+        o2 = o2 && H[c].z > ql[c] && L[c].z < qh[c];
+        o3 = o3 && H[c].w > ql[c] && L[c].w < qh[c];
+      }
+      unsigned mask = (o0 ? 1u : 0u) | (o1 ? 2u : 0u) | (o2 ? 4u : 0u) | (o3 ? 8u : 0u);
+      if (MESH) {
+        const int j0 = (first >> (2 * lvl)) - 4 * grp, j1 = (last >> (2 * lvl)) - 4 * grp;
+        if (j0 > 0) mask &= 15u << min(j0, 4);
+        if (j1 < 3) mask &= j1 < 0 ? 0u : 15u >> (3 - j1);
+      }
+      if (lvl > 0 && mask) {
+        const int c = __ffs(mask) - 1;
+        pending = pending << 4 | (mask & (mask - 1u));
+        --lvl;
+        grp = 4 * grp + c;
         continue;
       }
-      const float4 L = __ldg(&lo_left[2 * node]);
-      const float4 H = __ldg(&hi_esc[2 * node]);
-      bool ov = H.x > ql[0] && L.x < qh[0] && H.y > ql[1] && L.y < qh[1];
-      if (DIM == 3) ov = ov && H.z > ql[2] && L.z < qh[2];
-      if (ov) {
-        const int w = __float_as_int(L.w);
-        if (BUCKET && node < n - 1 && w < 0) {
-          // leaf bucket: its sorted leaves in order, exact FP64 test each
-          // (independent loads), then on past the subtree
-          const int f = w & 0x07ffffff, nl = ((w >> 27) & 7) + 1;
-          for (int k = 0; k < nl; ++k) {
-            const double2* q = reinterpret_cast<const double2*>(leaf + (int64_t)(f + k) * 8);
-            const double2 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q3 = __ldg(q + 3);
-            const double blo[3] = {q0.x, q0.y, q1.x}, bhi[3] = {q1.y, q2.x, q2.y};
-            bool ex = true;
+      if (lvl == 0 && mask) {
+        // which of the hits the FP32 boxes prove
+        bool s0 = true, s1 = true, s2 = true, s3 = true;
 #pragma unroll
-            for (int c = 0; c < DIM; ++c) ex = ex && (hi[c] > blo[c]) && (lo[c] < bhi[c]);
-            if (ex) {
-              const int e = __double2loint(q3.x);
-              if (FILL) {
-                if (out + cnt < pair_cap) {
-                  pair_a[out + cnt] = (int32_t)a;
-                  pair_b[out + cnt] = e;
-                }
-              } else if (cache) {
-                if (cnt < cap) cache[a * cap + cnt] = e;
+        for (int c = 0; c < DIM; ++c) {
+          s0 = s0 && H[c].x > il[c] && L[c].x < ih[c];
+          s1 = s1 && H[c].y > il[c] && L[c].y < ih[c];
+          s2 = s2 && H[c].z > il[c] && L[c].z < ih[c];
+          s3 = s3 && H[c].w > il[c] && L[c].w < ih[c];
+        }
+        const unsigned sure = (s0 ? 1u : 0u) | (s1 ? 2u : 0u) | (s2 ? 4u : 0u) | (s3 ? 8u : 0u);
+        do {
+          const int c = __ffs(mask) - 1;
+          mask &= mask - 1u;
+          const int e = T.vals[4 * grp + c];
+          bool ex = (sure >> c) & 1u;
+          if (!ex) {
+            const double* bb = box64_b + (int64_t)e * 2 * DIM;
+            ex = true;
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) ex = ex && qb[DIM + d] > bb[d] && qb[d] < bb[DIM + d];
+          }
+          if (ex) {
+            if (FILL) {
+              if (out + cnt < pair_cap) {
+                pair_a[out + cnt] = (int32_t)a;
+                pair_b[out + cnt] = e;
               }
-              ++cnt;
+            } else if (cache) {
+              if (MESH)
+                cache_put(cache, cap, sp, a, cnt, e, chunk, lost);
+              else if (cnt < cap)
+                cache[a * cap + cnt] = e;
             }
+            ++cnt;
           }
-          node = __float_as_int(H.w);
-          continue;
-        }
-        if (node < n - 1) {
-          node = w;
-          continue;
-        }
-        const double* bb = box64_b + (int64_t)w * 2 * DIM;
-        bool ex = true;
-#pragma unroll
-        for (int c = 0; c < DIM; ++c) ex = ex && (hi[c] > bb[c]) && (lo[c] < bb[DIM + c]);
-        if (ex) {
-          if (FILL) {
-            if (out + cnt < pair_cap) {
-              pair_a[out + cnt] = (int32_t)a;
-              pair_b[out + cnt] = w;
-            }
-          } else if (cache) {
-            if (cnt < cap) cache[a * cap + cnt] = w;
-          }
-          ++cnt;
-        }
+        } while (mask);
       }
-      node = __float_as_int(H.w);
+      // the nearest pending child
+      if (!pending) break;
+      const int z = (__ffsll((long long)pending) - 1) >> 2;
+      const unsigned m = (unsigned)(pending >> (4 * z)) & 15u;
+      lvl += z;
+      grp = ((grp >> (2 * z + 2)) << 2) + __ffs(m) - 1;
+      pending = (pending >> (4 * z)) & ~15ull | (m & (m - 1u));
     }
     if (!FILL) {
+      counts[a] = cnt;
+      if (cache && (MESH ? lost : cnt > cap)) {
+        if (MESH && sp.row_chunk) sp.row_chunk[a] = -2;
+        over_rows[1 + atomicAdd(over_rows, 1)] = (int32_t)a;
+      }
+    }
+  }
+}
+
+// The count pass with a warp per row: for meshes too small for a thread per
+// row to fill the chip, where the longest row's serial walk is the time, and
+// (3D) up to medium ones, whose rows of 50 and more candidates keep 32 lanes
+// busy.  The warp takes two levels of the hierarchy at once: the 16 + 16
+// grandchildren of two nodes, one per lane; then the first two hits' in turn,
+// the others pending in lane l for level 2 l.  Hits are appended in leaf
+// order, as by k_query.
+template <int DIM>
+__global__ void __launch_bounds__(256) k_query_warp(int64_t nel_a, const double* __restrict__ box64_a,
+                                                    const __grid_constant__ Tree T,
+                                                    const double* __restrict__ box64_b, int* counts, int32_t* cache,
+                                                    int cap, int* over_rows) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const int warps = (int)(gridDim.x * (blockDim.x >> 5));
+  for (int64_t a = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); a < nel_a; a += warps) {
+    const double* qb = box64_a + a * 2 * DIM;
+    float ql[DIM], qh[DIM], il[DIM], ih[DIM];
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      const double lo = qb[c], hi = qb[DIM + c];
+      const float l = __double2float_ru(lo), h = __double2float_rd(hi);
+      ql[c] = __double2float_rd(lo);
+      qh[c] = __double2float_ru(hi);
+      il[c] = fmaf(fabsf(l), 0x1p-21f, l) + 0x1p-140f;
+      ih[c] = fmaf(fabsf(h), -0x1p-21f, h) - 0x1p-140f;
+    }
+    int cnt = 0;
+    int lvl = T.top & ~1;
+    // the two parents (the first level: nodes 0-15 and no second)
+    int p0 = 0, p1 = -1;
+    int s0 = 0, s1 = 0;  // lane l: parents of level 2 l's tested nodes,
+    unsigned sm = 0;     // and those of them still pending
+    for (;;) {
+      const int p = lane < 16 ? p0 : p1;
+      const int64_t node = 16 * (int64_t)p + (lane & 15);
+      bool hit = false, sure = false;
+      const int64_t groups = T.off[lvl + 1] - T.off[lvl];
+      if (p >= 0 && (node >> 2) < groups) {
+        const float* r = T.rec + ((int64_t)T.off[lvl] + (node >> 2)) * (8 * DIM) + (node & 3);
+        float L[DIM], H[DIM];
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) {
+          L[c] = __ldg(r + 4 * c);
+          H[c] = __ldg(r + 4 * (DIM + c));
+        }
+        hit = sure = true;
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) {
+          hit = hit && H[c] > ql[c] && L[c] < qh[c];
+          sure = sure && H[c] > il[c] && L[c] < ih[c];
+        }
+      }
+      if (lvl == 0) {
+        int e = 0;
+        if (hit) {
+          e = T.vals[node];
+          if (!sure) {
+            const double* bb = box64_b + (int64_t)e * 2 * DIM;
+#pragma unroll
+            for (int c = 0; c < DIM; ++c) hit = hit && qb[DIM + c] > bb[c] && qb[c] < bb[DIM + c];
+          }
+        }
+        const unsigned hm = __ballot_sync(full, hit);
+        const int at = cnt + __popc(hm & lt);
+        if (hit && cache && at < cap) cache[a * cap + at] = e;
+        cnt += __popc(hm);
+      } else {
+        const unsigned hm = __ballot_sync(full, hit);
+        if (lane == lvl >> 1) {
+          s0 = p0;
+          s1 = p1;
+          sm = hm;
+        }
+      }
+      // the lowest level with pending nodes: its first two are the next parents
+      const unsigned lv = __ballot_sync(full, sm != 0);
+      if (!lv) break;
+      const int k = __ffs(lv) - 1;
+      const unsigned m = __shfl_sync(full, sm, k);
+      const int q0 = __shfl_sync(full, s0, k), q1 = __shfl_sync(full, s1, k);
+      const int b0 = __ffs(m) - 1;
+      const unsigned m1 = m & (m - 1u);
+      const int b1 = __ffs(m1) - 1;
+      p0 = 16 * (b0 < 16 ? q0 : q1) + (b0 & 15);
+      p1 = m1 ? 16 * (b1 < 16 ? q0 : q1) + (b1 & 15) : -1;
+      if (lane == k) sm = m1 & (m1 - 1u);
+      lvl = 2 * k - 2;
+    }
+    if (lane == 0) {
       counts[a] = cnt;
       if (cache && cnt > cap) over_rows[1 + atomicAdd(over_rows, 1)] = (int32_t)a;
     }
@@ -1101,25 +1189,25 @@ __global__ void __launch_bounds__(256) k_query(int64_t nel_a, const double* __re
 }
 
 // Fill of the rows whose candidates the count pass cached: each warp copies
-// its 32 rows one after the other, lanes striding over the row (coalesced
+// rpw rows one after the other, lanes striding over the row (coalesced
 // reads of the cache and writes of the pair arrays).
 __global__ void __launch_bounds__(256) k_fill_from_cache(int64_t nel_a, const int* __restrict__ counts,
                                                          const int64_t* __restrict__ offsets,
                                                          const int32_t* __restrict__ cache, int cap,
                                                          int32_t* pair_a, int32_t* pair_b, Spill sp,
-                                                         int64_t pair_cap) {
+                                                         int64_t pair_cap, int rpw) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; base < nel_a;
-       base += warps * 32) {
+  for (int64_t base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * rpw; base < nel_a;
+       base += warps * rpw) {
     const int64_t a = base + lane;
     int cnt = 0;
     int64_t off = 0;
-    if (a < nel_a) {
+    if (lane < rpw && a < nel_a) {
       cnt = counts[a];
       off = offsets[a];
     }
-    for (int r = 0; r < 32; ++r) {
+    for (int r = 0; r < rpw; ++r) {
       const int c = __shfl_sync(0xffffffffu, cnt, r);
       const int64_t o = __shfl_sync(0xffffffffu, off, r);
       const int64_t row = base + r;
@@ -1155,41 +1243,66 @@ __global__ void __launch_bounds__(256) k_fill_from_cache(int64_t nel_a, const in
   }
 }
 
-cudaError_t launch_query(int dim, bool fill, int64_t nel_a, const double* box64_a, BVH bvh,
-                         const double* box64_b, int* counts, const int64_t* offsets, int32_t* pair_a,
-                         int32_t* pair_b, cudaStream_t s, int32_t* cache, int cap, int* over_rows, Spill sp,
-                         int64_t pair_cap) {
-  if (nel_a <= 0 || bvh.n <= 0) return cudaSuccess;
-  const int B = query_block();
+// The count pass takes a warp per row below this many rows.  Whole search
+// (prep to pair arrays), thread / warp per row: 2D 10,658 rows 165 / 146 us,
+// 45,000 rows 168 / 186 us; 3D 6,000 rows 288 / 162 us, 48,000 rows 369 / 338
+// us, 118,098 rows 401 / 465 us.
+constexpr int64_t kWarpRows2 = 24 << 10, kWarpRows3 = 64 << 10;
+
+// Threads per block of the search: the option's, or a warp where that leaves
+// SMs without a block (the row's serial walk is then the time).
+static int query_threads(int64_t nel_a) {
+  return nel_a < (int64_t)sm_count() * 4 * query_block() ? 32 : query_block();
+}
+
+template <bool MESH>
+static cudaError_t run_query(int dim, bool fill, int64_t nel_a, const double* box64_a, const Tree& T,
+                             const double* box64_b, int* counts, const int64_t* offsets, int32_t* pair_a,
+                             int32_t* pair_b, cudaStream_t s, int32_t* cache, int cap, int* over_rows,
+                             int64_t pair_cap, const int32_t* pair_of_a, const int64_t* mesh_off, const Spill& sp) {
+  if (nel_a <= 0 || T.n <= 0) return cudaSuccess;
+  const int B = query_threads(nel_a);
   const int g = grid_for(nel_a, B, 2048 / B);
   if (fill && cache) {
     count_launch(2);
-    k_fill_from_cache<<<grid_for(nel_a, 256, 8), 256, 0, s>>>(nel_a, counts, offsets, cache, cap, pair_a, pair_b,
-                                                              sp, pair_cap);
+    // 32 rows per warp, fewer while that leaves warps to spare
+    int rpw = 32;
+    while (rpw > 1 && nel_a < (int64_t)sm_count() * 32 * rpw) rpw >>= 1;
+    k_fill_from_cache<<<grid_for((nel_a + rpw - 1) / rpw * 32, 256, 8), 256, 0, s>>>(
+        nel_a, counts, offsets, cache, cap, pair_a, pair_b, sp, pair_cap, rpw);
   } else {
     count_launch();
   }
+  if (!MESH && !fill && cache && nel_a < (dim == 2 ? kWarpRows2 : kWarpRows3)) {
+    const int gw = grid_for(nel_a * 32, 256, 8);
+    (dim == 2 ? k_query_warp<2> : k_query_warp<3>)<<<gw, 256, 0, s>>>(nel_a, box64_a, T, box64_b, counts, cache, cap,
+                                                                      over_rows);
+    return cudaGetLastError();
+  }
   const int32_t* rows = (fill && cache) ? over_rows + 1 : nullptr;
   int32_t* cc = fill ? nullptr : cache;
-#define LSM_QUERY_ARGS                                                                                    \
-  nel_a, box64_a, bvh.lo_left, bvh.hi_esc, bvh.n, box64_b, counts, offsets, pair_a, pair_b, cc, cap, rows, \
-      over_rows, bvh.leaf, pair_cap
-  // the bucket scan is compiled in only where the hierarchy has buckets:
-  // without them its branch alone slows the walk (2D count pass +27%)
-  const bool bk = bvh.bucket > 1;
-  if (dim == 2) {
-    if (fill)
-      bk ? k_query<2, true, true><<<g, B, 0, s>>>(LSM_QUERY_ARGS) : k_query<2, true, false><<<g, B, 0, s>>>(LSM_QUERY_ARGS);
-    else
-      bk ? k_query<2, false, true><<<g, B, 0, s>>>(LSM_QUERY_ARGS) : k_query<2, false, false><<<g, B, 0, s>>>(LSM_QUERY_ARGS);
-  } else {
-    if (fill)
-      bk ? k_query<3, true, true><<<g, B, 0, s>>>(LSM_QUERY_ARGS) : k_query<3, true, false><<<g, B, 0, s>>>(LSM_QUERY_ARGS);
-    else
-      bk ? k_query<3, false, true><<<g, B, 0, s>>>(LSM_QUERY_ARGS) : k_query<3, false, false><<<g, B, 0, s>>>(LSM_QUERY_ARGS);
-  }
-#undef LSM_QUERY_ARGS
+  const auto k = dim == 2 ? (fill ? k_query<2, true, MESH> : k_query<2, false, MESH>)
+                          : (fill ? k_query<3, true, MESH> : k_query<3, false, MESH>);
+  k<<<g, B, 0, s>>>(nel_a, box64_a, T, box64_b, counts, offsets, pair_a, pair_b, cc, cap, rows, over_rows, pair_cap,
+                    pair_of_a, mesh_off, sp);
   return cudaGetLastError();
+}
+
+cudaError_t launch_query(int dim, bool fill, int64_t nel_a, const double* box64_a, const Tree& T,
+                         const double* box64_b, int* counts, const int64_t* offsets, int32_t* pair_a,
+                         int32_t* pair_b, cudaStream_t s, int32_t* cache, int cap, int* over_rows, Spill sp,
+                         int64_t pair_cap) {
+  return run_query<false>(dim, fill, nel_a, box64_a, T, box64_b, counts, offsets, pair_a, pair_b, s, cache, cap,
+                          over_rows, pair_cap, nullptr, nullptr, sp);
+}
+
+cudaError_t launch_query_batched(int dim, bool fill, int64_t nel_a, const double* box64_a,
+                                 const int32_t* pair_of_a, const int64_t* mesh_off_b, const Tree& T,
+                                 const double* box64_b, int* counts, const int64_t* offsets, int32_t* pair_a,
+                                 int32_t* pair_b, cudaStream_t s, int32_t* cache, int cap, int* over_rows,
+                                 Spill sp, int64_t pair_cap) {
+  return run_query<true>(dim, fill, nel_a, box64_a, T, box64_b, counts, offsets, pair_a, pair_b, s, cache, cap,
+                         over_rows, pair_cap, pair_of_a, mesh_off_b, sp);
 }
 
 // ======================================================================
@@ -3340,13 +3453,22 @@ cudaError_t launch_finalize(const Partial* partials, int npartials, Partial* out
   return cudaGetLastError();
 }
 
+// One thread per row, eight loads ahead of the adds (in row order).
 __global__ void k_row_sums(int64_t nel_a, const int64_t* __restrict__ off, const double* __restrict__ pm,
-                           double* em) {
+                           double* out) {
   for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < nel_a;
        a += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
-    for (int64_t p = off[a]; p < off[a + 1]; ++p) s = s + pm[p];
-    em[a] = s;
+    const int64_t end = off[a + 1];
+    for (int64_t p = off[a]; p < end; p += 8) {
+      double v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = p + k < end ? pm[p + k] : 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (p + k < end) s = s + v[k];
+    }
+    out[a] = s;
   }
 }
 
@@ -3354,7 +3476,8 @@ cudaError_t launch_row_sums(int64_t nel_a, const int64_t* offsets, const double*
                             double* elem_measure, cudaStream_t s) {
   if (nel_a <= 0) return cudaSuccess;
   count_launch();
-  k_row_sums<<<grid_for(nel_a, 256, 8), 256, 0, s>>>(nel_a, offsets, pair_measure, elem_measure);
+  const int B = nel_a < (int64_t)sm_count() * 512 ? 32 : 256;
+  k_row_sums<<<grid_for(nel_a, B, 2048 / B), B, 0, s>>>(nel_a, offsets, pair_measure, elem_measure);
   return cudaGetLastError();
 }
 
@@ -3371,115 +3494,15 @@ cudaError_t launch_i32_to_i64(int64_t n, const int32_t* in, int64_t* out, cudaSt
 }
 
 // ======================================================================
-// Batched search: one LBVH over many meshes, one subtree per mesh
+// Batched search: one hierarchy over many meshes
 // ======================================================================
-// After sorting the B elements of all meshes by (mesh, Morton) the combined
-// 64-bit keys (mesh << 32 | Morton) give a Karras hierarchy in which every
-// mesh's elements form one subtree (they share the mesh-id prefix, no other
-// key does).  A query of mesh p starts at p's subtree root and stops at the
-// root's escape node.
+// The B elements of all meshes are sorted by (mesh, Morton), so a mesh's
+// leaves are one range of the sorted order, its element range; a row visits
+// only nodes that reach into the range of its own B mesh.
 __global__ void k_pair_keys(int64_t n, const int32_t* __restrict__ vals, const int32_t* __restrict__ pair_of,
                             uint32_t* keys) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     keys[i] = (uint32_t)pair_of[vals[i]];
-}
-
-// After a sort whose look-back wait gave up (*err != 0, values repaired to
-// the identity) the Morton part is left out: equal codes within a mesh give
-// a well-formed hierarchy (ties break by position), so the kernels after it
-// stay in bounds while the host reports the failure.
-__global__ void k_combined_codes(int64_t n, const int32_t* __restrict__ vals, const int32_t* __restrict__ pair_of,
-                                 const uint32_t* __restrict__ mort, unsigned long long* codes,
-                                 const uint32_t* __restrict__ err) {
-  const bool failed = err && *err != 0u;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t v = vals[i];
-    codes[i] = ((unsigned long long)(uint32_t)pair_of[v] << 32) | (failed ? 0ull : (unsigned long long)mort[v]);
-  }
-}
-
-__device__ __forceinline__ int bvh_delta64(const unsigned long long* __restrict__ codes, int n, int i, int j) {
-  if (j < 0 || j >= n) return -1;
-  const unsigned long long a = codes[i], b = codes[j];
-  if (a != b) return __clzll((long long)(a ^ b));
-  return 64 + __clz((uint32_t)i ^ (uint32_t)j);
-}
-
-__global__ void k_bvh_internal64(int n, const unsigned long long* __restrict__ codes, int* parent, int* rope,
-                                 int* last, int* left, int* right, const int64_t* __restrict__ mesh_off,
-                                 int* roots) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n - 1) return;
-  const int d = (bvh_delta64(codes, n, i, i + 1) - bvh_delta64(codes, n, i, i - 1)) >= 0 ? 1 : -1;
-  const int dmin = bvh_delta64(codes, n, i, i - d);
-  int lmax = 2;
-  while (bvh_delta64(codes, n, i, i + lmax * d) > dmin) lmax <<= 1;
-  int l = 0;
-  for (int t = lmax >> 1; t >= 1; t >>= 1)
-    if (bvh_delta64(codes, n, i, i + (l + t) * d) > dmin) l += t;
-  const int j = i + l * d;
-  const int dnode = bvh_delta64(codes, n, i, j);
-  int s = 0;
-  int t = l;
-  do {
-    t = (t + 1) >> 1;
-    if (bvh_delta64(codes, n, i, i + (s + t) * d) > dnode) s += t;
-  } while (t > 1);
-  const int gamma = i + s * d + (d < 0 ? -1 : 0);
-  const int first = i < j ? i : j;
-  const int lst = i < j ? j : i;
-  const int lc = (first == gamma) ? (n - 1) + gamma : gamma;
-  const int rc = (lst == gamma + 1) ? (n - 1) + gamma + 1 : gamma + 1;
-  left[i] = lc;
-  right[i] = rc;
-  parent[lc] = i;
-  parent[rc] = i;
-  rope[gamma + 1] = rc;
-  last[i] = lst;
-  const int mesh = (int)(codes[first] >> 32);
-  if (mesh_off[mesh] == first && mesh_off[mesh + 1] - 1 == lst) roots[mesh] = i;
-}
-
-// Roots of single-element meshes, and the stop node (the root's escape) of
-// every mesh.  Meshes without elements get root -1.
-__global__ void k_mesh_roots(int nm, int n, const int64_t* __restrict__ mesh_off, const int* __restrict__ rope,
-                             const int* __restrict__ last, int* roots, int* stops) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= nm) return;
-  const int64_t cnt = mesh_off[p + 1] - mesh_off[p];
-  int r = -1;
-  if (cnt == 1)
-    r = (n - 1) + (int)mesh_off[p];
-  else if (cnt > 1)
-    r = roots[p];
-  roots[p] = r;
-  stops[p] = r >= 0 ? bvh_escape(n, r, rope, last) : -1;
-}
-
-cudaError_t launch_batched_tree(int n, int nm, const int32_t* sorted_vals, const int32_t* pair_of_b,
-                                const uint32_t* mort, unsigned long long* codes, const float* box32,
-                                const int64_t* mesh_off_b, BVH bvh, int* work, int* roots, int* stops,
-                                cudaStream_t s, int dim, const double* box64, const int* sort_err) {
-  if (n <= 0) return cudaSuccess;
-  int* parent = work;
-  int* rope = parent + (2 * n - 1);
-  int* visit = rope + n;
-  int* last = visit + n;
-  int* left = last + n;
-  int* right = left + n;
-  count_launch(4);
-  k_combined_codes<<<grid_for(n, 256, 8), 256, 0, s>>>(n, sorted_vals, pair_of_b, mort, codes,
-                                                       reinterpret_cast<const uint32_t*>(sort_err));
-  cudaMemsetAsync(visit, 0, sizeof(int) * n, s);
-  cudaMemsetAsync(rope, 0xff, sizeof(int) * n, s);
-  cudaMemsetAsync(roots, 0xff, sizeof(int) * nm, s);
-  if (n > 1) k_bvh_internal64<<<(n - 1 + 255) / 256, 256, 0, s>>>(n, codes, parent, rope, last, left, right, mesh_off_b, roots);
-  cudaMemsetAsync(parent, 0xff, sizeof(int), s);
-  k_mesh_roots<<<(nm + 255) / 256, 256, 0, s>>>(nm, n, mesh_off_b, rope, last, roots, stops);
-  k_bvh_refit<false><<<(n + kRefitBlock - 1) / kRefitBlock, kRefitBlock, 0, s>>>(n, sorted_vals, reinterpret_cast<const float4*>(box32), parent,
-                                                     rope, last, left, right, visit, bvh.lo_left, bvh.hi_esc, dim,
-                                                     box64, box64 ? bvh.leaf : nullptr, nullptr, 1);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_pair_keys(int64_t n, const int32_t* vals, const int32_t* pair_of, uint32_t* keys,
@@ -3487,141 +3510,6 @@ cudaError_t launch_pair_keys(int64_t n, const int32_t* vals, const int32_t* pair
   if (n <= 0) return cudaSuccess;
   count_launch();
   k_pair_keys<<<grid_for(n, 256, 8), 256, 0, s>>>(n, vals, pair_of, keys);
-  return cudaGetLastError();
-}
-
-template <int DIM, bool FILL>
-__global__ void __launch_bounds__(256) k_query_batched(int64_t nel_a, const double* __restrict__ box64_a,
-                                                       const int32_t* __restrict__ pair_of_a,
-                                                       const int* __restrict__ roots, const int* __restrict__ stops,
-                                                       const float4* __restrict__ lo_left,
-                                                       const float4* __restrict__ hi_esc, int n,
-                                                       const double* __restrict__ box64_b, int* counts,
-                                                       const int64_t* __restrict__ offsets, int32_t* pair_a,
-                                                       int32_t* pair_b, int32_t* cache, int cap,
-                                                       const int32_t* __restrict__ rows, int* over_rows,
-                                                       const double* __restrict__ leaf, Spill sp,
-                                                       int64_t pair_cap) {
-  // cache / rows / over_rows / leaf: as k_query
-  const int64_t nrows = rows ? (int64_t)*over_rows : nel_a;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t a = rows ? rows[r] : r;
-    double lo[DIM], hi[DIM];
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      lo[c] = box64_a[a * 2 * DIM + c];
-      hi[c] = box64_a[a * 2 * DIM + DIM + c];
-    }
-    float ql[3], qh[3];
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      ql[c] = __double2float_rd(lo[c]);
-      qh[c] = __double2float_ru(hi[c]);
-    }
-    const int mesh = pair_of_a[a];
-    int node = roots[mesh];
-    const int stop = stops[mesh];
-    int cnt = 0;
-    int64_t out = FILL ? offsets[a] : 0;
-    int chunk = -1;     // current spill chunk of this row
-    bool lost = false;  // the row goes to the second traversal
-    const int nodes = 2 * n - 1;
-    for (int guard = 0; node >= 0 && node != stop && guard < 2 * n + 1; ++guard) {
-      if (node >= nodes) break;  // never taken for a well-formed hierarchy
-      if (leaf && node >= n - 1) {
-        const double2* q = reinterpret_cast<const double2*>(leaf + (int64_t)(node - (n - 1)) * 8);
-        const double2 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q3 = __ldg(q + 3);
-        const double blo[3] = {q0.x, q0.y, q1.x}, bhi[3] = {q1.y, q2.x, q2.y};
-        const int2 meta = make_int2(__double2loint(q3.x), __double2hiint(q3.x));
-        bool ex = true;
-#pragma unroll
-        for (int c = 0; c < DIM; ++c) ex = ex && (hi[c] > blo[c]) && (lo[c] < bhi[c]);
-        if (ex) {
-          if (FILL) {
-            if (out + cnt < pair_cap) {
-              pair_a[out + cnt] = (int32_t)a;
-              pair_b[out + cnt] = meta.x;
-            }
-          } else if (cache) {
-            cache_put(cache, cap, sp, a, cnt, meta.x, chunk, lost);
-          }
-          ++cnt;
-        }
-        node = meta.y;
-        continue;
-      }
-      const float4 L = __ldg(&lo_left[2 * node]);
-      const float4 H = __ldg(&hi_esc[2 * node]);
-      bool ov = H.x > ql[0] && L.x < qh[0] && H.y > ql[1] && L.y < qh[1];
-      if (DIM == 3) ov = ov && H.z > ql[2] && L.z < qh[2];
-      if (ov) {
-        const int w = __float_as_int(L.w);
-        if (node < n - 1) {
-          node = w;
-          continue;
-        }
-        const double* bb = box64_b + (int64_t)w * 2 * DIM;
-        bool ex = true;
-#pragma unroll
-        for (int c = 0; c < DIM; ++c) ex = ex && (hi[c] > bb[c]) && (lo[c] < bb[DIM + c]);
-        if (ex) {
-          if (FILL) {
-            if (out + cnt < pair_cap) {
-              pair_a[out + cnt] = (int32_t)a;
-              pair_b[out + cnt] = w;
-            }
-          } else if (cache) {
-            cache_put(cache, cap, sp, a, cnt, w, chunk, lost);
-          }
-          ++cnt;
-        }
-      }
-      node = __float_as_int(H.w);
-    }
-    if (!FILL) {
-      counts[a] = cnt;
-      if (cache && lost) {
-        if (sp.row_chunk) sp.row_chunk[a] = -2;
-        over_rows[1 + atomicAdd(over_rows, 1)] = (int32_t)a;
-      }
-    }
-  }
-}
-
-
-cudaError_t launch_query_batched(int dim, bool fill, int64_t nel_a, const double* box64_a,
-                                 const int32_t* pair_of_a, const int* roots, const int* stops, BVH bvh,
-                                 const double* box64_b, int* counts, const int64_t* offsets, int32_t* pair_a,
-                                 int32_t* pair_b, cudaStream_t s, int32_t* cache, int cap, int* over_rows,
-                                 Spill sp, int64_t pair_cap) {
-  if (nel_a <= 0 || bvh.n <= 0) return cudaSuccess;
-  const int B = query_block();
-  const int g = grid_for(nel_a, B, 2048 / B);
-  if (fill && cache) {
-    count_launch(2);
-    k_fill_from_cache<<<grid_for(nel_a, 256, 8), 256, 0, s>>>(nel_a, counts, offsets, cache, cap, pair_a, pair_b,
-                                                              sp, pair_cap);
-  } else {
-    count_launch();
-  }
-  const int32_t* rows = (fill && cache) ? over_rows + 1 : nullptr;
-  int32_t* cc = fill ? nullptr : cache;
-#define LSM_QUERY_ARGS                                                                                         \
-  nel_a, box64_a, pair_of_a, roots, stops, bvh.lo_left, bvh.hi_esc, bvh.n, box64_b, counts, offsets, pair_a, \
-      pair_b, cc, cap, rows, over_rows, bvh.leaf, sp, pair_cap
-  if (dim == 2) {
-    if (fill)
-      k_query_batched<2, true><<<g, B, 0, s>>>(LSM_QUERY_ARGS);
-    else
-      k_query_batched<2, false><<<g, B, 0, s>>>(LSM_QUERY_ARGS);
-  } else {
-    if (fill)
-      k_query_batched<3, true><<<g, B, 0, s>>>(LSM_QUERY_ARGS);
-    else
-      k_query_batched<3, false><<<g, B, 0, s>>>(LSM_QUERY_ARGS);
-  }
-#undef LSM_QUERY_ARGS
   return cudaGetLastError();
 }
 

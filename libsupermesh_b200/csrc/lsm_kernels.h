@@ -46,28 +46,26 @@ int tri_blocks_per_sm();
 void set_tri_blocks_per_sm(int v);
 int query_block();
 void set_query_block(int v);
-// Leaves per bucket of the single-mesh hierarchy (1 = none; 2, 4 or 8):
-// subtrees of at most this many leaves are scanned as contiguous leaf
-// records instead of being walked.
+// Option leaf_bucket: kept and returned; the hierarchy scans four leaves at
+// a time whatever its value.
 int leaf_bucket();
 void set_leaf_bucket(int v);
-// The bucket size launch_bvh_build uses for n leaves (1 = none); BVH::bucket
-// must carry it to the search.
-int tree_bucket(int n, bool leaf_records);
 
-struct BVH {
-  int n = 0;                 // leaves
-  // Node k (2n-1 nodes) is the 32-byte pair lo_left[2k], hi_esc[2k] of one
-  // interleaved array (hi_esc = lo_left + 1), so a visit reads one sector.
-  float4* lo_left = nullptr;  // lo.xyz, .w = left child / element (int bits)
-  float4* hi_esc = nullptr;   // hi.xyz, .w = escape node (int bits), -1 = end
-  // optional [n][8] f64 leaf records in sorted order: lo (3), hi (3),
-  // {element, escape} as two ints, pad
-  double* leaf = nullptr;
-  // internal nodes of at most `bucket` leaves carry a leaf-bucket code in
-  // place of their left child (1: none)
-  int bucket = 1;
+// Four-wide box hierarchy over n leaves (elements vals[0..n) in sorted order,
+// 16-byte aligned, readable up to a multiple of four):
+// the groups of level l are records off[l] .. off[l+1]-1 of 8*dim floats,
+// levels 0 .. top (one group).
+struct Tree {
+  int n = 0;
+  int top = 0;
+  const int32_t* vals = nullptr;
+  float* rec = nullptr;
+  int off[18] = {};
 };
+int64_t tree_floats(int dim, int64_t n);  // size of rec
+Tree make_tree(int dim, int n, const int32_t* sorted_vals, float* rec);
+// ticket: a zero (launch_root_box leaves one)
+cudaError_t launch_tree_build(int dim, const Tree& T, const float* box32, unsigned* ticket, cudaStream_t s);
 
 // Mesh prep: gather coordinates, boxes, measures/tolerances, B clip setup.
 // idx_bytes selects the enlist element type (4 = int32, 8 = int64).
@@ -76,9 +74,9 @@ cudaError_t launch_prep(int dim, int loc, int64_t nel, const double* pos, const 
                         int* bad_index, int64_t nnodes, cudaStream_t s, double* faces = nullptr,
                         double* screen = nullptr);
 
-// Root box (float64) of a set of element boxes: rootbox[2*dim].
+// Root box (float64) of a set of element boxes: rootbox[2*dim]; *ticket = 0.
 cudaError_t launch_root_box(int dim, int64_t nel, const double* box64, double* partial,
-                            int partial_cap, double* rootbox, cudaStream_t s);
+                            int partial_cap, double* rootbox, unsigned* ticket, cudaStream_t s);
 
 cudaError_t launch_morton(int dim, int64_t nel, const double* box64, const double* rootbox,
                           uint32_t* keys, int32_t* vals, cudaStream_t s);
@@ -99,11 +97,6 @@ void set_sort_stall_block(int b);
 int sort_stall_block();
 cudaError_t radix_sort_pairs(int64_t n, int bits, uint32_t* keys, int32_t* vals, uint32_t* keys_tmp,
                              int32_t* vals_tmp, uint32_t* hist, cudaStream_t s, int* err = nullptr);
-
-// LBVH over sorted Morton codes.  work_int needs 8*n ints.
-cudaError_t launch_bvh_build(int dim, int n, const uint32_t* sorted_keys, const int32_t* sorted_vals,
-                             const float* box32, BVH bvh, int* work_int, cudaStream_t s,
-                             const double* box64 = nullptr);
 
 // Spill pool of the count pass's row cache: rows longer than the cache
 // continue in chunks of kSpillChunk candidates (pool[chunks][kSpillChunk]),
@@ -128,7 +121,7 @@ struct Spill {
 // the kept rows and traverses only the listed ones.
 // pair_cap: entries pair_a / pair_b hold; the fill writes no pair beyond it
 // (the caller compares the count with it afterwards).
-cudaError_t launch_query(int dim, bool fill, int64_t nel_a, const double* box64_a, BVH bvh,
+cudaError_t launch_query(int dim, bool fill, int64_t nel_a, const double* box64_a, const Tree& T,
                          const double* box64_b, int* counts, const int64_t* offsets, int32_t* pair_a,
                          int32_t* pair_b, cudaStream_t s, int32_t* cache = nullptr, int cap = 0,
                          int* over_rows = nullptr, Spill sp = Spill{}, int64_t pair_cap = INT64_MAX);
@@ -317,15 +310,10 @@ cudaError_t launch_prep_batched(int dim, int64_t nel, int nm, const int64_t* ele
 // keys[i] = pair_of[vals[i]] (second sort pass: by mesh)
 cudaError_t launch_pair_keys(int64_t n, const int32_t* vals, const int32_t* pair_of, uint32_t* keys,
                              cudaStream_t s);
-// One LBVH over all B meshes (sorted by mesh, then Morton); roots/stops per
-// mesh.  codes: n u64; work: 8n ints.
-cudaError_t launch_batched_tree(int n, int nm, const int32_t* sorted_vals, const int32_t* pair_of_b,
-                                const uint32_t* mort, unsigned long long* codes, const float* box32,
-                                const int64_t* mesh_off_b, BVH bvh, int* work, int* roots, int* stops,
-                                cudaStream_t s, int dim = 3,
-                                const double* box64 = nullptr, const int* sort_err = nullptr);
+// One hierarchy over all B meshes (sorted by mesh, then Morton); a row of
+// mesh m takes the leaves mesh_off_b[m] .. mesh_off_b[m+1]-1.
 cudaError_t launch_query_batched(int dim, bool fill, int64_t nel_a, const double* box64_a,
-                                 const int32_t* pair_of_a, const int* roots, const int* stops, BVH bvh,
+                                 const int32_t* pair_of_a, const int64_t* mesh_off_b, const Tree& T,
                                  const double* box64_b, int* counts, const int64_t* offsets, int32_t* pair_a,
                                  int32_t* pair_b, cudaStream_t s, int32_t* cache = nullptr, int cap = 0,
                                  int* over_rows = nullptr, Spill sp = Spill{}, int64_t pair_cap = INT64_MAX);

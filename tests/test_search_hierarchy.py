@@ -1,0 +1,72 @@
+"""The four-wide box hierarchy of the candidate search at the edges of its
+groups and levels, on boxes that FP32 cannot decide, and with both traversals
+(a warp per row below 24,576 rows in 2D and 65,536 in 3D, a thread per row
+from there on): candidate sets against brute force over the FP64 boxes with
+the reference's strict test, rows in the same order from both."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _elements(dim, n, rng, size):
+    """n small simplices as a mesh of its own nodes."""
+    c = rng.random((n, 1, dim))
+    pos = (c + size * (rng.random((n, dim + 1, dim)) - 0.5)).reshape(-1, dim)
+    return pos, np.arange(n * (dim + 1), dtype=np.int32).reshape(n, dim + 1)
+
+
+def _rows(ctx, A, B):
+    n = ctx.find_candidates(A, B)
+    ip, ind = ctx.get_candidates(len(A[1]), n)
+    return ip, ind
+
+
+def _brute(A, B):
+    va, vb = A[0][A[1]], B[0][B[1]]
+    la, ha, lb, hb = va.min(1), va.max(1), vb.min(1), vb.max(1)
+    for a in range(len(la)):
+        yield np.flatnonzero(((ha[a] > lb) & (la[a] < hb)).all(1))
+
+
+def _check(ctx, A, B):
+    ip, ind = _rows(ctx, A, B)
+    for a, ref in enumerate(_brute(A, B)):
+        got = ind[ip[a]:ip[a + 1]]
+        assert np.array_equal(np.sort(got), ref), a
+    return ip, ind
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("nb", [1, 2, 4, 5, 16, 17, 63, 65, 256, 257, 1023, 1025, 4097])
+def test_group_and_level_edges(gpu_ctx, dim, nb):
+    rng = np.random.default_rng(nb)
+    _check(gpu_ctx, _elements(dim, 300, rng, 0.3), _elements(dim, nb, rng, 0.1))
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("shift,scale,step", [
+    (0.0, 1.0, 8), (-0.5, 1.0, 8),       # many equal coordinates: boxes that touch
+    (1.0e6, 1.0, 8), (0.0, 1.0e6, 1000),  # boxes closer than FP32's spacing
+    (0.0, 2.0 ** -140, 1 << 20),          # FP32 subnormals
+    (3.0e38, 1.0e36, 64),                 # beyond FP32's range
+])
+def test_boxes_fp32_cannot_decide(gpu_ctx, dim, shift, scale, step):
+    rng = np.random.default_rng(dim)
+    A, B = _elements(dim, 400, rng, 0.2), _elements(dim, 700, rng, 0.2)
+    A, B = ((np.round(m[0] * step) / step * scale + shift, m[1]) for m in (A, B))
+    _check(gpu_ctx, A, B)
+
+
+@pytest.mark.parametrize("dim,na", [(2, 24575), (2, 24576), (3, 65535), (3, 65536)])
+def test_both_traversals_give_the_same_rows(gpu_ctx, dim, na):
+    """Rows of a large A (around the line between the traversals) and of its
+    first 3000 elements alone; long rows among them (more than 256)."""
+    rng = np.random.default_rng(na)
+    pos, en = _elements(dim, na, rng, 0.02)
+    pos[:(dim + 1) * 5] = rng.random(((dim + 1) * 5, dim)) * 1.2
+    B = _elements(dim, 5000, rng, 0.05)
+    ip, ind = _rows(gpu_ctx, (pos, en), B)
+    ips, inds = _check(gpu_ctx, (pos, en[:3000]), B)
+    assert np.array_equal(ip[:3001], ips)
+    assert np.array_equal(ind[:ips[-1]], inds)
