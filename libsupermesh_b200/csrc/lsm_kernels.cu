@@ -1956,15 +1956,21 @@ void run_prefilter(int64_t n, const int32_t* order, const int32_t* pa, const int
 // K6: depth-first tet clipper over point indices
 // ----------------------------------------------------------------------
 // One pair per lane, depth-first, lanes refilled from the survivor list; a
-// tet is four 5-bit indices into the lane's point pool in shared memory
+// tet is four byte indices into the lane's point pool in shared memory
 // instead of twelve doubles in registers.  Pool slots 0-3 hold A's vertices; the split at
 // plane L writes its (at most four) new points to slots 4+4L .. 7+4L.  In
 // depth-first order that is safe: a tet at plane L references only points of
 // planes < L, and when a sibling is taken from the stack every point written
-// by the previous sibling's subtree belongs to planes >= its own.  Child
-// assembly becomes integer work on index tuples, a pending tet is one word,
-// and vertices are fetched by index with shared-memory loads instead of
-// chains of selects.
+// by the previous sibling's subtree belongs to planes >= its own.
+// What a visit costs is mostly integer work around 24 FP64 operations: lists of
+// vertices by class, indices picked from them, children put together case by
+// case.  All of that comes from the split table (below) instead: a table word
+// for the classes gives the order in which to fetch the vertices, so that the
+// interpolated edges are the same registers in every case, and the children
+// as byte permutes of the old tet and the new points.  Early-out pass and
+// clipper, tet3d_graded_55x51 8.61 -> 7.66 ms, tet3d_27x32 1.83 -> 1.61 ms
+// (952 -> 709 million warp instructions in the clipper); 524,288 tet-hexahedron pairs, whole
+// call, 1.06 -> 0.92 ms.
 constexpr int kIxPoints = 20;  // 4 + 4 per plane
 #ifndef LSM_IX_BLOCK
 #define LSM_IX_BLOCK 480
@@ -2009,6 +2015,18 @@ __device__ __forceinline__ void ix_gather(const Pool& pool, unsigned tet, Tet& t
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
     const V3 q = pool.get(ix_vert(tet, v));
+    t.x[v] = q.x;
+    t.y[v] = q.y;
+    t.z[v] = q.z;
+  }
+}
+
+// Coordinates of a tet of four byte indices.
+template <class Pool>
+__device__ __forceinline__ void ix_bytes(const Pool& pool, unsigned tet, Tet& t) {
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    const V3 q = pool.get((tet >> (8 * v)) & 255u);
     t.x[v] = q.x;
     t.y[v] = q.y;
     t.z[v] = q.z;
@@ -2185,181 +2203,6 @@ struct IxCarrySinkT {
 };
 constexpr int kHexHexCap = 5 * 729;  // output tets per hexahedron pair
 
-// Points in a lane's pool for NP planes: A's 4 vertices + 4 per plane.
-__host__ __device__ constexpr int ix_points(int np) { return 4 + 4 * np; }
-
-template <class Sink, int BLOCK, int BPS, int NP = 4>
-__global__ void __launch_bounds__(BLOCK, BPS) k_clip_tets_ix(
-    const int4* __restrict__ list, const unsigned long long* __restrict__ nlist, const double* __restrict__ coords_a,
-    const double* __restrict__ tol_a, const double* __restrict__ setup_b, Sink sk, unsigned long long* work,
-    const int4* __restrict__ chunks = nullptr) {
-  // chunks (optional): the list is segmented; nlist then counts the table's
-  // chunks and work counts the chunks taken
-  static_assert(ix_points(NP) <= 32, "pool indices are 5 bits");
-  extern __shared__ double ix_mem[];
-  IxPool<BLOCK> pool{ix_mem + threadIdx.x};
-  // pending tets (at most 2 per plane but the last): a shift register of
-  // 20-bit index tuples over kW words (stk[kW-1]:...:stk[0], newest in the
-  // low bits) and their planes, kLB bits each (stk_lv)
-  constexpr int kW = NP <= 4 ? 2 : 4;
-  constexpr int kLB = NP <= 4 ? 2 : 3;
-  static_assert(2 * (NP - 1) * 20 <= 64 * kW && 2 * (NP - 1) * kLB <= 32, "pending-tet stack too small");
-  unsigned long long stk[kW];
-#pragma unroll
-  for (int w = 0; w < kW; ++w) stk[w] = 0;
-  unsigned stk_lv = 0;
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  const int64_t npairs = (int64_t)*nlist;
-  // warp cursor over the list (warp-uniform)
-  int64_t cbeg = 0, cend = 0;
-  bool exhausted = false;
-  // prefetch pipeline of the next pair: stage 0 idle, 1 record loading,
-  // 2 element data loading (ready for the next refill)
-  int nstage = 0;
-  int4 nrec = make_int4(0, 0, 0, 0);
-  Tet nt;
-  double ntol = 0.0;
-  // current pair
-  int64_t p = -1;
-  const double* planes = setup_b;
-  unsigned cur = 0;
-  double tol = 0.0;
-  int L = 0, sp = 0;
-  // planes this pair clips at (bit L; the prefilter's no-op planes are
-  // skipped) and the last of them
-  constexpr unsigned kAll = (1u << NP) - 1u;
-  unsigned act = kAll;
-  int lastL = NP - 1;
-  for (;;) {
-    // ---- prefetch pipeline
-    if (nstage == 1) {
-      load_tet(coords_a + (int64_t)nrec.y * 12, nt);
-      ntol = fmin(tol_a[nrec.y], setup_b[(int64_t)nrec.z * clip_row(NP) + 4 * NP]);
-      nstage = 2;
-    }
-    if (p < 0 && nstage == 2) {
-      p = nrec.x;
-#pragma unroll
-      for (int v = 0; v < 4; ++v) pool.put(v, V3{nt.x[v], nt.y[v], nt.z[v]});
-      planes = setup_b + (int64_t)nrec.z * clip_row(NP);
-      tol = ntol;
-      cur = ix_pack(0, 1, 2, 3);
-      sk.begin(nrec);
-      act = ~(unsigned)nrec.w & kAll;  // never 0 unless Sink::kInside
-      L = __ffs(act) - 1;
-      lastL = 31 - __clz(act);
-      sp = 0;
-      nstage = 0;
-#pragma unroll
-      for (int w = 0; w < kW; ++w) stk[w] = 0;
-      stk_lv = 0;
-      if (Sink::kInside && act == 0u) {
-        // A inside all four planes: the reference keeps A as its one tet
-        Tet o;
-        ix_gather(pool, cur, o);
-        double v1;
-        if (final_tet_keep(o, tol, v1)) sk.tet(o, v1);
-        sk.end(p);
-        p = -1;
-      }
-    }
-    {
-      const bool want = nstage == 0 && !exhausted;
-      unsigned wm = __ballot_sync(full, want);
-      while (wm) {
-        if (cbeg >= cend) {
-          unsigned long long base = 0;
-          if (lane == 0) base = atomicAdd(work, chunks ? 1ull : (unsigned long long)kIxChunk);
-          base = __shfl_sync(full, base, 0);
-          if ((int64_t)base >= npairs) {
-            exhausted = true;
-            break;
-          }
-          if (chunks) {
-            const int4 ch = chunks[base];
-            cbeg = ch.x;
-            cend = ch.y;
-          } else {
-            cbeg = (int64_t)base;
-            cend = cbeg + kIxChunk < npairs ? cbeg + kIxChunk : npairs;
-          }
-        }
-        const int navail = (int)(cend - cbeg);
-        const int rank = __popc(wm & lt);
-        const bool take = want && ((wm >> lane) & 1u) && rank < navail;
-        if (take) {
-          nrec = list[cbeg + rank];
-          nstage = 1;
-        }
-        const unsigned tm = __ballot_sync(full, take);
-        cbeg += __popc(tm);
-        wm &= ~tm;
-      }
-    }
-    if (__all_sync(full, p < 0 && nstage == 0 && exhausted)) break;
-    if (p < 0) continue;
-    Tet t;
-    ix_gather(pool, cur, t);
-    double nx, ny, nz, c;
-    load_plane(planes, L, nx, ny, nz, c);
-    TetClass cls;
-    classify_tet(t, nx, ny, nz, c, cls);
-    int k = 0;
-    unsigned c0 = cur, c1 = 0, c2 = 0;
-    if (cls.nn > 0) k = cls.np == 0 ? 1 : ix_split(cur, cls, pool, 4 + 4 * L, c0, c1, c2);
-    if (L == lastL) {
-      // final tets, in the reference's order
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        if (j < k) {
-          Tet o;
-          ix_gather(pool, j == 0 ? c0 : (j == 1 ? c1 : c2), o);
-          double v1;
-          if (final_tet_keep(o, tol, v1)) sk.tet(o, v1);
-        }
-      }
-      k = 0;
-    }
-    if (k > 0) {
-      const unsigned lv = (unsigned)(__ffs(act & (~0u << (L + 1))) - 1);  // next plane clipped at
-      if (k == 3) {
-#pragma unroll
-        for (int w = kW - 1; w > 0; --w) stk[w] = (stk[w] << 20) | (stk[w - 1] >> 44);
-        stk[0] = (stk[0] << 20) | c2;
-        stk_lv = (stk_lv << kLB) | lv;
-        ++sp;
-      }
-      if (k >= 2) {
-#pragma unroll
-        for (int w = kW - 1; w > 0; --w) stk[w] = (stk[w] << 20) | (stk[w - 1] >> 44);
-        stk[0] = (stk[0] << 20) | c1;
-        stk_lv = (stk_lv << kLB) | lv;
-        ++sp;
-      }
-      cur = c0;
-      L = (int)lv;
-      continue;
-    }
-    if (sp > 0) {
-      cur = (unsigned)(stk[0] & 0xfffffull);
-      L = (int)(stk_lv & ((1u << kLB) - 1u));
-#pragma unroll
-      for (int w = 0; w < kW - 1; ++w) stk[w] = (stk[w] >> 20) | (stk[w + 1] << 44);
-      stk[kW - 1] >>= 20;
-      stk_lv >>= kLB;
-      --sp;
-      continue;
-    }
-    sk.end(p);
-    p = -1;
-  }
-}
-
-// ----------------------------------------------------------------------
-// K6: breadth-first tet clipper, a warp per batch of pairs
-// ----------------------------------------------------------------------
 // Split table: for the 2-bit classes of a tet's vertices (0 zero, 1 negative,
 // 2 positive) the order in which to gather them (their roles), and each child
 // as a byte permute of (old tet, new points).  In role order the interpolated
@@ -2383,7 +2226,8 @@ struct ClipTable {
 // each four nibbles (vertex i of the child: 0-3 old vertex, 4-7 new point;
 // roles: old vertex).  Bit 2 of the roles' nibbles 0-3: ++--, two or more
 // children, three, a split (Tetrahedron_Intersection.F90:290-434: the same
-// cases, interpolation and child order as split_tet).
+// cases, interpolation and child order as split_tet).  Without a negative
+// vertex the roles are 0: no child.
 constexpr ClipTable make_clip_table() {
   ClipTable T{};
   for (unsigned c = 0; c < 256; ++c) {
@@ -2439,6 +2283,7 @@ constexpr ClipTable make_clip_table() {
       w[3] |= role[i] << (4 * i);
     }
     if (ok && nn > 0 && np > 0) w[3] |= 1u << 14;
+    if (!ok || nn == 0) w[3] = 0;
     if (two) w[3] |= 1u << 2;
     if (kids >= 2) w[3] |= 1u << 6;
     if (kids == 3) w[3] |= 1u << 10;
@@ -2472,6 +2317,217 @@ __device__ __forceinline__ unsigned class_bits(double d, unsigned neg_bit) {
   return w;
 }
 
+// Points in a lane's pool for NP planes: A's 4 vertices + 4 per plane.
+__host__ __device__ constexpr int ix_points(int np) { return 4 + 4 * np; }
+
+template <class Sink, int BLOCK, int BPS, int NP = 4>
+__global__ void __launch_bounds__(BLOCK, BPS) k_clip_tets_ix(
+    const int4* __restrict__ list, const unsigned long long* __restrict__ nlist, const double* __restrict__ coords_a,
+    const double* __restrict__ tol_a, const double* __restrict__ setup_b, Sink sk, unsigned long long* work,
+    const int4* __restrict__ chunks = nullptr) {
+  // chunks (optional): the list is segmented; nlist then counts the table's
+  // chunks and work counts the chunks taken
+  static_assert(ix_points(NP) <= 32, "pool indices are 5 bits");
+  extern __shared__ double ix_mem[];
+  uint2* table = reinterpret_cast<uint2*>(ix_mem);
+  for (int i = threadIdx.x; i < 256; i += BLOCK) table[i] = g_clip_table.e[i];
+  __syncthreads();
+  IxPool<BLOCK> pool{ix_mem + kClipTableBytes / 8 + threadIdx.x};
+  // pending tets (at most 2 per plane but the last), newest first: four point
+  // bytes each, the plane to clip at next in the top bits
+  constexpr int kW = 2 * (NP - 1);
+  unsigned stk[kW];
+#pragma unroll
+  for (int w = 0; w < kW; ++w) stk[w] = 0;
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const int64_t npairs = (int64_t)*nlist;
+  // warp cursor over the list (warp-uniform)
+  int64_t cbeg = 0, cend = 0;
+  bool exhausted = false;
+  // prefetch pipeline of the next pair: stage 0 idle, 1 record loading,
+  // 2 element data loading (ready for the next refill)
+  int nstage = 0;
+  int4 nrec = make_int4(0, 0, 0, 0);
+  Tet nt;
+  double ntol = 0.0;
+  // current pair
+  int64_t p = -1;
+  const double* planes = setup_b;
+  unsigned cur = 0;
+  double tol = 0.0;
+  int L = 0, sp = 0;
+  // planes this pair clips at (bit L; the prefilter's no-op planes are
+  // skipped) and the last of them
+  constexpr unsigned kAll = (1u << NP) - 1u;
+  unsigned act = kAll;
+  int lastL = NP - 1;
+  for (;;) {
+    // ---- prefetch pipeline
+    if (nstage == 1) {
+      load_tet(coords_a + (int64_t)nrec.y * 12, nt);
+      ntol = fmin(tol_a[nrec.y], setup_b[(int64_t)nrec.z * clip_row(NP) + 4 * NP]);
+      nstage = 2;
+    }
+    if (p < 0 && nstage == 2) {
+      p = nrec.x;
+#pragma unroll
+      for (int v = 0; v < 4; ++v) pool.put(v, V3{nt.x[v], nt.y[v], nt.z[v]});
+      planes = setup_b + (int64_t)nrec.z * clip_row(NP);
+      tol = ntol;
+      cur = 0x03020100u;
+      sk.begin(nrec);
+      act = ~(unsigned)nrec.w & kAll;  // never 0 unless Sink::kInside
+      L = __ffs(act) - 1;
+      lastL = 31 - __clz(act);
+      sp = 0;
+      nstage = 0;
+      if (Sink::kInside && act == 0u) {
+        // A inside all four planes: the reference keeps A as its one tet
+        Tet o;
+        ix_bytes(pool, cur, o);
+        double v1;
+        if (final_tet_keep(o, tol, v1)) sk.tet(o, v1);
+        sk.end(p);
+        p = -1;
+      }
+    }
+    {
+      const bool want = nstage == 0 && !exhausted;
+      unsigned wm = __ballot_sync(full, want);
+      while (wm) {
+        if (cbeg >= cend) {
+          unsigned long long base = 0;
+          if (lane == 0) base = atomicAdd(work, chunks ? 1ull : (unsigned long long)kIxChunk);
+          base = __shfl_sync(full, base, 0);
+          if ((int64_t)base >= npairs) {
+            exhausted = true;
+            break;
+          }
+          if (chunks) {
+            const int4 ch = chunks[base];
+            cbeg = ch.x;
+            cend = ch.y;
+          } else {
+            cbeg = (int64_t)base;
+            cend = cbeg + kIxChunk < npairs ? cbeg + kIxChunk : npairs;
+          }
+        }
+        const int navail = (int)(cend - cbeg);
+        const int rank = __popc(wm & lt);
+        const bool take = want && ((wm >> lane) & 1u) && rank < navail;
+        if (take) {
+          nrec = list[cbeg + rank];
+          nstage = 1;
+        }
+        const unsigned tm = __ballot_sync(full, take);
+        cbeg += __popc(tm);
+        wm &= ~tm;
+      }
+    }
+    if (__all_sync(full, p < 0 && nstage == 0 && exhausted)) break;
+    if (p < 0) continue;
+    double nx, ny, nz, c;
+    load_plane(planes, L, nx, ny, nz, c);
+    // classes from the signs, one bit each, unless a distance is neither
+    // clearly positive nor clearly negative (as in surv_code)
+    uint2 e;
+    {
+      unsigned neg = 0, irr = 0;
+      double d[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const V3 v = pool.get((cur >> (8 * i)) & 255u);
+        d[i] = ((nx * v.x + ny * v.y) + nz * v.z) - c;
+        const unsigned hi = (unsigned)__double2hiint(d[i]);
+        neg |= (hi >> 31) << (2 * i);
+        irr = max(irr, 2u * hi - 2u * kEpsHi);
+      }
+      unsigned code = neg | (neg ^ 0x55u) << 1;
+      if (irr >= 2u * (0x7ff00000u - kEpsHi)) {
+        code = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const unsigned b = class_bits(d[i], 1u);
+          code |= ((b & 1u) | (b >> 4) << 1) << (2 * i);
+        }
+      }
+      e = table[code];
+    }
+    int k = (int)(e.y >> 20 & 1u);
+    unsigned c0 = cur, c1 = 0, c2 = 0;
+    if (e.y >> 30 & 1u) {
+      const unsigned r = prmt(cur, cur, e.y >> 16);
+      V3 v[4];
+      double d[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v[i] = pool.get((r >> (8 * i)) & 255u);
+        d[i] = ((nx * v[i].x + ny * v[i].y) + nz * v[i].z) - c;
+      }
+      const bool two = (e.y >> 18) & 1u;
+      const unsigned base = 4u + 4u * (unsigned)L;
+      pool.put(base, interp_edge(v[0], v[3], d[0], d[3]));
+      pool.put(base + 1, interp_edge(v[1], v[3], d[1], d[3]));
+      pool.put(base + 2, interp_edge(v[2], two ? v[0] : v[3], d[2], two ? d[0] : d[3]));
+      if (two) pool.put(base + 3, interp_edge(v[1], v[2], d[1], d[2]));
+      const unsigned fresh = base * 0x01010101u + 0x03020100u;
+      c0 = prmt(cur, fresh, e.x);
+      c1 = prmt(cur, fresh, e.x >> 16);
+      c2 = prmt(cur, fresh, e.y);
+      k = 1 + (int)(e.y >> 22 & 1u) + (int)(e.y >> 26 & 1u);
+      // (the zero vertex of +--0 is the first of the reference's list, which a
+      // NaN distance does not enter: then vertex 0)
+      if (k == 2 && isnan(d[2])) c1 = prmt(c1, cur, 0x3240);
+    }
+    if (L == lastL) {
+      // final tets, in the reference's order
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        if (j < k) {
+          Tet o;
+          ix_bytes(pool, j == 0 ? c0 : (j == 1 ? c1 : c2), o);
+          double v1;
+          if (final_tet_keep(o, tol, v1)) sk.tet(o, v1);
+        }
+      }
+      k = 0;
+    }
+    if (k > 0) {
+      const unsigned lv = (unsigned)(__ffs(act & (~0u << (L + 1))) - 1);  // next plane clipped at
+      if (k == 3) {
+#pragma unroll
+        for (int w = kW - 1; w > 1; --w) stk[w] = stk[w - 2];
+        stk[0] = c1 | lv << 29;
+        stk[1] = c2 | lv << 29;
+        sp += 2;
+      } else if (k == 2) {
+#pragma unroll
+        for (int w = kW - 1; w > 0; --w) stk[w] = stk[w - 1];
+        stk[0] = c1 | lv << 29;
+        ++sp;
+      }
+      cur = c0;
+      L = (int)lv;
+      continue;
+    }
+    if (sp > 0) {
+      cur = stk[0] & 0x1fffffffu;
+      L = (int)(stk[0] >> 29);
+#pragma unroll
+      for (int w = 0; w < kW - 1; ++w) stk[w] = stk[w + 1];
+      --sp;
+      continue;
+    }
+    sk.end(p);
+    p = -1;
+  }
+}
+
+// ----------------------------------------------------------------------
+// K6: breadth-first tet clipper, a warp per batch of pairs
+// ----------------------------------------------------------------------
 // A pair whose distances are not all finite, by visits as in k_clip_tets_ix
 // (A's vertices in the pool): a vertex with a NaN distance belongs to none of
 // the reference's three lists, which class bits cannot say.
@@ -2546,9 +2602,8 @@ __device__ __forceinline__ void clip_nonfinite(const Pool& pool, const double* p
 // Measured (tet3d_27x32 unless said): P1 mass 12.8 -> 5.9 ms; supermesh elements 4.47 ->
 // 4.04 ms; measures of 330 thousand candidates (10^3 x 6 against 12^3 x 6
 // tets), early-out pass included, 0.212 -> 0.136 ms.  On the large measure
-// passes the two are level (1.38 against 1.34 ms; tet3d_graded_55x51 6.3
-// against 6.8 ms: as many instructions go into the lists and rounds as into
-// the idle lanes of the other), so those stay with k_clip_tets_ix.
+// passes k_clip_tets_ix is ahead (1.18 against 1.34 ms; as many instructions go
+// into the lists and rounds as into the idle lanes of the other).
 //
 // Shared memory of a warp: the point pool (groups of four points: point i of
 // group q at index 4 q + (i ^ (q >> 2 & 3)), so that the i-th points of
@@ -3028,10 +3083,11 @@ __global__ void __launch_bounds__(Sink::kWarps * 32, 1) k_clip_tets_bf(
 }
 
 // Measure passes of fewer candidate pairs than this go through
-// k_clip_tets_bf.  Early-out pass and clipper, k_clip_tets_ix against it:
-// 330 thousand candidates 0.212 / 0.136 ms, 1.05 million explicit pairs (whole call) 0.757 /
-// 0.699 ms, 10 million 1.83 / 1.80 ms, 56 million (graded) 8.67 / 9.14 ms.
-constexpr int64_t kBfMeasureMax = 4 << 20;
+// k_clip_tets_bf.  Narrow phase of two meshes, k_clip_tets_ix / k_clip_tets_bf:
+// 44 thousand candidates 148 / 93 us, 452 thousand 205 / 157, 1.37 million
+// 300 / 277, 1.81 million 388 / 385, 4.2 million 661 / 698, 10 million 1655 /
+// 1837 us.
+constexpr int64_t kBfMeasureMax = 3 << 19;
 
 template <class Sink>
 size_t bf_smem_bytes() {
@@ -3049,7 +3105,7 @@ void run_bf(const int4* list, const unsigned long long* nlist, const double* coo
                                                                                     setup_b, sk, work, chunks);
 }
 
-size_t ix_smem_bytes() { return (size_t)kIxBlock * 3 * kIxPoints * sizeof(double); }
+size_t ix_smem_bytes() { return (size_t)kIxBlock * 3 * kIxPoints * sizeof(double) + kClipTableBytes; }
 
 // Per-pair setup of explicit tetrahedron pairs (the prep kernel's work for
 // one-element meshes): B's planes and tolerance (setup row), A's tolerance,
@@ -3095,7 +3151,7 @@ cudaError_t launch_setup_pairs3(int64_t n, const double* tet_a, const double* te
 // per lane.
 constexpr int kIxHexBlock = 320;
 
-size_t ix_hex_smem_bytes() { return (size_t)kIxHexBlock * 3 * ix_points(6) * sizeof(double); }
+size_t ix_hex_smem_bytes() { return (size_t)kIxHexBlock * 3 * ix_points(6) * sizeof(double) + kClipTableBytes; }
 
 // kVec: hex_b is 16-byte aligned, each hexahedron is read in 12 16-byte loads
 template <bool kVec>

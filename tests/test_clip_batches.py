@@ -1,4 +1,4 @@
-"""The breadth-first tet clipper (k_clip_tets_bf) at the edges of its batches
+"""The tet clippers (k_clip_tets_bf and k_clip_tets_ix) at the edges of their batches
 and on inputs outside the ordinary: against the one-launch clipper that
 batches below 2048 pairs take, and the P1 mass blocks against the oracle.
 Both sides run the same operations in the same order, so every comparison is
@@ -6,6 +6,7 @@ exact."""
 import numpy as np
 import pytest
 
+import libsupermesh_b200 as lsm
 from libsupermesh_b200 import meshes as M
 
 pytestmark = pytest.mark.gpu
@@ -80,3 +81,24 @@ def test_p1_blocks_match_oracle(gpu_ctx, oracle_mod, na, nb, ja, jb, scale):
     ip, ind = gpu_ctx.get_candidates(len(A[1]), len(blocks))
     _, _, ref = oracle_mod.p1_mass(3, A, B, ip, ind, u, v, want_blocks=True)
     assert np.array_equal(blocks, ref.reshape(blocks.shape))
+
+
+@pytest.mark.parametrize("value", [None, np.nan, np.inf, 1e200])
+def test_tet_hexahedron_batches(gpu_ctx, value):
+    """The depth-first clipper's split table, six planes: batches of 2048 and
+    more against the one-launch clipper, special tets and (value) coordinates
+    that are not finite among them."""
+    a, b = _pairs(2307, 9)
+    corner = np.array([[0, 0, 0], [1, 0, 0], [1, 1, 0], [0, 1, 0], [0, 0, 1], [1, 0, 1], [1, 1, 1], [0, 1, 1]], float)
+    lo, hi = b.min(1), b.max(1)
+    h = lo[:, None] + corner[None] * (hi - lo)[:, None]
+    h[::5] = np.round(a[::5, :1] * 4) / 4 + corner[None] * 0.5  # faces through vertices' neighbourhoods
+    a[::5] = np.round(a[::5] * 8) / 8
+    if value is not None:
+        rng = np.random.default_rng(6)
+        rows = rng.choice(len(a), 700, replace=False)
+        a[rows, rng.integers(0, 4, 700), rng.integers(0, 3, 700)] = value
+    got = gpu_ctx.intersect_pairs_mixed(lsm.PAIR_TET_HEX, a, h)
+    ref = [gpu_ctx.intersect_pairs_mixed(lsm.PAIR_TET_HEX, a[i:i + 1000], h[i:i + 1000])[:2] for i in (0, 1000, 2000)]
+    assert np.array_equal(got[1], np.concatenate([r[1] for r in ref]))
+    assert np.array_equal(got[0], np.concatenate([r[0] for r in ref]))
