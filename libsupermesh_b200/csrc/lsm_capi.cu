@@ -82,7 +82,7 @@ struct Ctx {
   DevBuf p1_seg_cnt, p1_seg_tab, x_seg_cnt, x_seg_tab;  // the same for the P1 pass and explicit pairs
   // explicit pairs / p1 / batched
   DevBuf x_a, x_b, x_measure, x_nout, x_elems, u_a, v_b, blocks;
-  DevBuf x_setup, x_tol, x_iota, x_faces, x_screen, x_list;  // explicit tet pairs through the early-out pass
+  DevBuf x_setup, x_tol, x_iota, x_list;  // explicit tet pairs through the early-out pass
   DevBuf x_sub;  // hexahedron pairs: A's five tets
   DevBuf elem_off, x_pa, x_pb;  // supermesh elements: per-pair offsets, parents
   DevBuf bt_tabs, bt_pair_a, bt_pair_b, bt_tot, bt_ncand, bt_indptr;
@@ -285,7 +285,7 @@ void fini_ctx(Ctx* c) {
                    &c->counts, &c->offsets, &c->scan_tmp, &c->pair_a,
                    &c->pair_b, &c->i64_tmp, &c->pair_measure, &c->pair_nout, &c->partials,
                    &c->ovf_list, &c->p1_list, &c->misc, &c->elem_measure, &c->totals, &c->x_a, &c->x_b, &c->x_measure,
-                   &c->x_nout, &c->x_elems, &c->x_setup, &c->x_tol, &c->x_iota, &c->x_faces, &c->x_screen,
+                   &c->x_nout, &c->x_elems, &c->x_setup, &c->x_tol, &c->x_iota,
                    &c->x_list, &c->elem_off, &c->x_pa, &c->x_pb, &c->u_a, &c->v_b, &c->blocks, &c->bt_tabs, &c->bt_pair_a,
                    &c->bt_pair_b, &c->bt_tot,
                    &c->bt_ncand, &c->bt_stage_pa[0], &c->bt_stage_ea[0], &c->bt_stage_pb[0],
@@ -2049,25 +2049,16 @@ int libsupermesh_gpu_intersect_pairs(lsm_gpu_context* ctx, int dim, int64_t n, c
       de = elems ? ensure<double>(c, c->x_elems, n * cap * per) : nullptr;
     }
     if (dim == 3 && n >= kPairsPipelineMin && n <= INT32_MAX) {
-      // large batches: per-pair setup, the exact early-outs and the index
-      // clipper (one launch per stage); small ones stay on the one-launch
-      // register clipper below (identical results)
+      // large batches: setup and the exact early-outs in one pass, then the
+      // clipper; small ones stay on the one-launch register clipper below
+      // (identical results)
       double* setup = ensure<double>(c, c->x_setup, n * lsm::kSetup3);
       double* tol = ensure<double>(c, c->x_tol, n);
-      int32_t* iota = ensure<int32_t>(c, c->x_iota, n);
-      double* faces = g_tet_screen ? ensure<double>(c, c->x_faces, n * lsm::kScreen3) : nullptr;
-      double* screen = g_tet_screen ? ensure<double>(c, c->x_screen, n * lsm::kScreen3) : nullptr;
       int32_t* list = ensure<int32_t>(c, c->x_list, 4 * n);
       double* pm = dm ? dm : ensure<double>(c, c->x_measure, n);
       int32_t* pn = dn ? dn : ensure<int32_t>(c, c->x_nout, n);
-      unsigned long long* work = pairs_work(c);
-      const lsm::SegList sg = seg_list(c, c->x_seg_cnt, c->x_seg_tab, n);
-      CU(lsm::launch_setup_pairs3(n, da, db, setup, tol, iota, faces, screen, s));
-      if (de)
-        CU(lsm::launch_clip_elems(n, iota, iota, da, tol, setup, pm, pn, de, list, work, faces, screen, s, &sg));
-      else
-        CU(lsm::launch_clip(3, n, iota, iota, da, tol, setup, pm, pn, list, nullptr, work, s, nullptr, nullptr,
-                            nullptr, faces, screen, nullptr, nullptr, &sg));
+      CU(lsm::launch_tet_pairs(n, da, db, pm, pn, de, setup, tol, list, pairs_work(c), g_tet_screen != 0,
+                               seg_list(c, c->x_seg_cnt, c->x_seg_tab, n), s));
     } else {
       CU(lsm::launch_pairs_explicit(dim, n, da, db, dm, dn, de, s));
     }

@@ -32,26 +32,46 @@ __device__ __forceinline__ double spacing(double x) {
   return __longlong_as_double((long long)es << 52);
 }
 
-// gfortran's inline NORM2 of a 3-vector (scaled sum of squares).
+// gfortran's inline NORM2 of a 3-vector (scaled sum of squares): per nonzero
+// component with |v| above the scale so far, result = 1 + result (scale/|v|)^2
+// and the scale becomes |v|; otherwise result += (|v|/scale)^2.  The first
+// nonzero component leaves result 1 (its quotient is 0/|v|), so a division is
+// needed for the second and third only, smaller by larger in either case.
 __device__ __forceinline__ double norm2_3(double a, double b, double c) {
-  double scale = 0.0, result = 1.0;
-  const double v[3] = {a, b, c};
+  double scale = fabs(a), result = 1.0;
+  const double v[2] = {fabs(b), fabs(c)};
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
+  for (int i = 0; i < 2; ++i) {
+    const bool up = scale < v[i];
+    const double val = (up ? scale : v[i]) / (up ? v[i] : scale);
+    const double sq = val * val;
     if (v[i] != 0.0) {
-      const double ax = fabs(v[i]);
-      if (scale < ax) {
-        const double val = scale / ax;
-        result = 1.0 + result * (val * val);
-        scale = ax;
-      } else {
-        const double val = ax / scale;
-        result = result + val * val;
-      }
+      result = up ? 1.0 + result * sq : result + sq;
+      scale = up ? v[i] : scale;
     }
   }
   return sqrt(result) * scale;
 }
+
+// a / b, correctly rounded, for a divisor whose correctly rounded reciprocal
+// y is at hand.  Markstein (IBM J. Res. Dev. 34, 1990): if q is within one ulp
+// of a/b and y = RN(1/b), then r = a - b q is exact and RN(q + r y) = RN(a/b).
+// a y is within 1.5 ulp, so a first such step brings q within one ulp and the
+// second gives the quotient.  Holds while nothing underflows or overflows:
+// div_range keeps the largest 2 * (high word of |v|) - 2 * high(2^-400), modulo
+// 2^32, of the operands; div_ok(max) is false as soon as one lies outside
+// [2^-400, 2^400] (zero, infinity and NaN included), and the caller then
+// divides.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  double q = a * y;
+  q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+constexpr unsigned kDivLo = (1023u - 400u) << 20, kDivHi = (1023u + 400u) << 20;
+__device__ __forceinline__ unsigned div_range(unsigned range, double v) {
+  return max(range, 2u * (unsigned)__double2hiint(v) - 2u * kDivLo);
+}
+__device__ __forceinline__ bool div_ok(unsigned range) { return range <= 2u * (kDivHi - kDivLo); }
 
 // ---------------------------------------------------------------- measures
 // tri: vertices (x0,y0),(x1,y1),(x2,y2).  0.5*|u2 v1 - u1 v2| with u = v3-v1,
@@ -181,9 +201,21 @@ __device__ __forceinline__ void unit_cross(double ax, double ay, double az, doub
   oy = az * bx - ax * bz;
   oz = ax * by - ay * bx;
   const double n = norm2_3(ox, oy, oz);
-  ox = ox / n;
-  oy = oy / n;
-  oz = oz / n;
+  // three quotients by one divisor; a component that is zero stays as it is
+  unsigned range = div_range(0, n);
+  range = div_range(range, ox == 0.0 ? 1.0 : ox);
+  range = div_range(range, oy == 0.0 ? 1.0 : oy);
+  range = div_range(range, oz == 0.0 ? 1.0 : oz);
+  if (div_ok(range)) {
+    const double y = __drcp_rn(n);
+    ox = ox == 0.0 ? ox : div_by(ox, n, y);
+    oy = oy == 0.0 ? oy : div_by(oy, n, y);
+    oz = oz == 0.0 ? oz : div_by(oz, n, y);
+  } else {
+    ox = ox / n;
+    oy = oy / n;
+    oz = oz / n;
+  }
 }
 
 __device__ __forceinline__ void tet_planes(const Tet& t, Planes& P) {
@@ -283,8 +315,12 @@ __device__ __forceinline__ double det3(double ax, double ay, double az, double b
   return (ax * (by * cz - bz * cy) + ay * (bz * cx - bx * cz)) + az * (bx * cy - by * cx);
 }
 
-__device__ __forceinline__ void tet_screen_b(const Tet& t, const Planes& P, double* o) {
-  double M = max_abs_tet(t);
+// (a face's own normal may stand for any other direction in (4): with n not
+// normalised, every margin is multiplied by a bound of |n|.)
+//
+// B's factors: g, tau (with its rounding) and M.
+__device__ __forceinline__ void tet_screen_factors(const Tet& t, const Planes& P, double& g, double& tau_r, double& M) {
+  M = max_abs_tet(t);
 #pragma unroll
   for (int i = 0; i < 4; ++i) M = fmax(M, fabs(P.c[i]));
   // residuals of each plane at its three own vertices (plane f omits vertex 3-f)
@@ -310,14 +346,20 @@ __device__ __forceinline__ void tet_screen_b(const Tet& t, const Planes& P, doub
   const bool pos = D[0] > kDetErr && D[1] > kDetErr && D[2] > kDetErr && D[3] > kDetErr;
   const bool neg = D[0] < -kDetErr && D[1] < -kDetErr && D[2] < -kDetErr && D[3] < -kDetErr;
   const double dmin = fmin(fmin(fabs(D[0]), fabs(D[1])), fmin(fabs(D[2]), fabs(D[3])));
-  const double g = (pos || neg) ? 3.02 / (dmin - kDetErr) : pos_inf();
+  g = (pos || neg) ? 3.02 / (dmin - kDetErr) : pos_inf();
+  tau_r = tau + 16.0 * kEps * (1.0 + 2.0 * M);
+}
+
+__device__ __forceinline__ void tet_screen_b(const Tet& t, const Planes& P, double* o) {
+  double g, tau, M;
+  tet_screen_factors(t, P, g, tau, M);
   st2(o + 0, t.x[0], t.y[0]);
   st2(o + 2, t.z[0], t.x[1]);
   st2(o + 4, t.y[1], t.z[1]);
   st2(o + 6, t.x[2], t.y[2]);
   st2(o + 8, t.z[2], t.x[3]);
   st2(o + 10, t.y[3], t.z[3]);
-  st2(o + 12, g, tau + 16.0 * kEps * (1.0 + 2.0 * M));
+  st2(o + 12, g, tau);
   st2(o + 14, M, 0.0);
 }
 

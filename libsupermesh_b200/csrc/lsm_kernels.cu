@@ -3109,10 +3109,9 @@ size_t ix_smem_bytes() { return (size_t)kIxBlock * 3 * kIxPoints * sizeof(double
 
 // Per-pair setup of explicit tetrahedron pairs (the prep kernel's work for
 // one-element meshes): B's planes and tolerance (setup row), A's tolerance,
-// identity pair indices and, optionally, the rows of the second early-out
-// (A's face planes, B's screen row).
+// identity pair indices.
 __global__ void k_setup_pairs3(int64_t n, const double* __restrict__ tet_a, const double* __restrict__ tet_b,
-                               double* setup, double* tol_a, int32_t* iota, double* faces_a, double* screen_b) {
+                               double* setup, double* tol_a, int32_t* iota) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     // both pair arrays are 16-byte aligned (checked by the entry points)
     Tet a, b;
@@ -3130,16 +3129,126 @@ __global__ void k_setup_pairs3(int64_t n, const double* __restrict__ tet_a, cons
     st2(o + 18, 0.0, 0.0);
     tol_a[i] = 10.0 * spacing(tet_volume_v4(a));
     iota[i] = (int32_t)i;
-    if (screen_b) tet_screen_b(b, P, screen_b + i * kScreen3);
-    if (faces_a) tet_faces_screen(a, faces_a + i * kScreen3);
   }
 }
 
+// Setup and early-outs of explicit tetrahedron pairs in one pass, a thread per
+// pair: B's planes stay in registers for k_prefilter_tets' tests, and only the
+// pairs they leave write a setup row, A's tolerance and a survivor record (as
+// kSeg and kCode there; pairs inside all planes are listed).  The separate
+// passes wrote 428 bytes of setup per pair and read them back: 1,048,576
+// pairs, of which a third survive, 0.32 -> 0.15 ms.  A's faces enter the second
+// test as they come from the cross product: a direction need not be of unit
+// length there, only the margins scaled (kept clear of underflow).
+__global__ void __launch_bounds__(256, 2) k_pairs_early(int64_t n, const double* __restrict__ tet_a,
+                                                        const double* __restrict__ tet_b, double* setup,
+                                                        double* tol_a, double* measure, int32_t* nout, int4* survivors,
+                                                        int* seg_count, bool second) {
+  __shared__ unsigned s_cnt;
+  if (threadIdx.x == 0) s_cnt = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int64_t per = seg_per(n, gridDim.x);
+  const int64_t beg = (int64_t)blockIdx.x * per;
+  const int64_t end = beg + per < n ? beg + per : n;
+  for (int64_t base = beg; base < end; base += blockDim.x) {
+    const int64_t i = base + threadIdx.x;
+    bool live = false;
+    int code = 0;
+    if (i < end) {
+      Tet t, u;
+      load_tet(tet_a + 12 * i, t);
+      load_tet(tet_b + 12 * i, u);
+      Planes P;
+      tet_planes(u, P);
+      const double M = max_abs_tet(t);
+      bool reject = false;
+      unsigned neg = 0, irr = 0;
+      int noop = 0;
+#pragma unroll
+      for (int L = 0; L < 4; ++L) {
+        const double thr = kEps + 64.0 * kEps * (1.0 + 2.0 * fmax(M, fabs(P.c[L])));
+        double dmin = DBL_MAX, dmax = -DBL_MAX;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const double d = ((P.nx[L] * t.x[k] + P.ny[L] * t.y[k]) + P.nz[L] * t.z[k]) - P.c[L];
+          const unsigned hi = (unsigned)__double2hiint(d);
+          neg = __funnelshift_l(hi, neg, 1);
+          irr = max(irr, 2u * hi - 2u * kEpsHi);
+          dmin = fmin(dmin, d);
+          dmax = fmax(dmax, d);
+        }
+        reject = reject || dmin >= thr;
+        noop |= dmax <= -thr ? 1 << L : 0;
+      }
+      code = surv_code(noop, neg, irr);
+      if (!reject && second) {
+        double g, tau, MB;
+        tet_screen_factors(u, P, g, tau, MB);
+        if (g < DBL_MAX) {  // B's planes bound a proper tet
+          const double Mp = fmax(M, MB);
+          const double e = kEps + 128.0 * kEps * (1.0 + 2.0 * Mp);
+          const double margin =
+              1.01 * g * (tau + e) + 16.0 * kEps * (1.0 + Mp) + 128.0 * kEps * (1.0 + M);
+#pragma unroll
+          for (int f = 0; f < 4; ++f) {
+            // the face opposite vertex f, outwards
+            const int p = f == 0 ? 1 : 0, q = f <= 1 ? 2 : 1, r = f <= 2 ? 3 : 2;
+            const double ax = t.x[q] - t.x[p], ay = t.y[q] - t.y[p], az = t.z[q] - t.z[p];
+            const double bx = t.x[r] - t.x[p], by = t.y[r] - t.y[p], bz = t.z[r] - t.z[p];
+            double nx = ay * bz - az * by, ny = az * bx - ax * bz, nz = ax * by - ay * bx;
+            const double side = (nx * (t.x[f] - t.x[p]) + ny * (t.y[f] - t.y[p])) + nz * (t.z[f] - t.z[p]);
+            if (side > 0.0) {
+              nx = -nx;
+              ny = -ny;
+              nz = -nz;
+            }
+            const double size = (fabs(nx) + fabs(ny)) + fabs(nz);
+            double h = -DBL_MAX, m = DBL_MAX;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              h = fmax(h, (nx * t.x[k] + ny * t.y[k]) + nz * t.z[k]);
+              m = fmin(m, (nx * u.x[k] + ny * u.y[k]) + nz * u.z[k]);
+            }
+            // (a bound that is not finite, from coordinates that are not, proves nothing)
+            const double bound = size * margin;
+            reject = reject || (size > 0x1p-800 && bound < DBL_MAX && m - h >= bound);
+          }
+        }
+      }
+      live = !reject;
+      if (reject) {
+        measure[i] = 0.0;
+        nout[i] = 0;
+      } else {
+        double* o = setup + i * kSetup3;
+#pragma unroll
+        for (int L = 0; L < 4; ++L) {
+          st2(o + 4 * L, P.nx[L], P.ny[L]);
+          st2(o + 4 * L + 2, P.nz[L], P.c[L]);
+        }
+        st2(o + 16, 10.0 * spacing(tet_volume_v4(u)), 0.0);
+        tol_a[i] = 10.0 * spacing(tet_volume_v4(t));
+      }
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, live);
+    if (mask) {
+      const int leader = __ffs(mask) - 1;
+      unsigned off = 0;
+      if (lane == leader) off = atomicAdd(&s_cnt, (unsigned)__popc(mask));
+      off = __shfl_sync(0xffffffffu, off, leader);
+      if (live) survivors[beg + off + __popc(mask & ((1u << lane) - 1u))] = make_int4((int)i, (int)i, (int)i, code);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) seg_count[blockIdx.x] = (int)s_cnt;
+}
+
 cudaError_t launch_setup_pairs3(int64_t n, const double* tet_a, const double* tet_b, double* setup, double* tol_a,
-                                int32_t* iota, double* faces_a, double* screen_b, cudaStream_t s) {
+                                int32_t* iota, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   count_launch();
-  k_setup_pairs3<<<grid_for(n, 256, 8), 256, 0, s>>>(n, tet_a, tet_b, setup, tol_a, iota, faces_a, screen_b);
+  k_setup_pairs3<<<grid_for(n, 256, 8), 256, 0, s>>>(n, tet_a, tet_b, setup, tol_a, iota);
   return cudaGetLastError();
 }
 
@@ -3284,14 +3393,11 @@ cudaError_t launch_hex_hex_pairs(int64_t n, const double* hex_a, const double* h
   return cudaGetLastError();
 }
 
-cudaError_t launch_clip_elems(int64_t n, const int32_t* pair_a, const int32_t* pair_b, const double* tet_a,
-                              const double* tol_a, const double* setup, double* measure, int32_t* nout,
-                              double* elems, int32_t* survivors, unsigned long long* work, const double* faces_a,
-                              const double* screen_b, cudaStream_t s, const SegList* seg) {
-  cudaMemsetAsync(work, 0, 2 * sizeof(unsigned long long), s);
-  if (n <= 0) return cudaGetLastError();
-  run_prefilter<false, 4, true>(n, nullptr, pair_a, pair_b, tet_a, tol_a, setup, measure, nout, survivors, work, faces_a,
-                          screen_b, nullptr, seg, s);
+// The clipper over a survivor list that holds the pairs with every plane a
+// no-op, with kCode words: measures and counts, and the output tets (elems).
+static cudaError_t clip_listed(int64_t n, const double* tet_a, const double* tol_a, const double* setup,
+                               double* measure, int32_t* nout, double* elems, int32_t* survivors,
+                               unsigned long long* work, const SegList* seg, cudaStream_t s) {
   count_launch();
   const int4* list = reinterpret_cast<const int4*>(survivors);
   if (elems)
@@ -3305,6 +3411,30 @@ cudaError_t launch_clip_elems(int64_t n, const int32_t* pair_a, const int32_t* p
                                                                         IxInsideSink{{measure, nout, 0.0, 0}}, work + 1,
                                                                         seg_table(seg));
   return cudaGetLastError();
+}
+
+cudaError_t launch_clip_elems(int64_t n, const int32_t* pair_a, const int32_t* pair_b, const double* tet_a,
+                              const double* tol_a, const double* setup, double* measure, int32_t* nout,
+                              double* elems, int32_t* survivors, unsigned long long* work, const double* faces_a,
+                              const double* screen_b, cudaStream_t s, const SegList* seg) {
+  cudaMemsetAsync(work, 0, 2 * sizeof(unsigned long long), s);
+  if (n <= 0) return cudaGetLastError();
+  run_prefilter<false, 4, true>(n, nullptr, pair_a, pair_b, tet_a, tol_a, setup, measure, nout, survivors, work,
+                                faces_a, screen_b, nullptr, seg, s);
+  return clip_listed(n, tet_a, tol_a, setup, measure, nout, elems, survivors, work, seg, s);
+}
+
+cudaError_t launch_tet_pairs(int64_t n, const double* tet_a, const double* tet_b, double* measure, int32_t* nout,
+                             double* elems, double* setup, double* tol_a, int32_t* survivors,
+                             unsigned long long* work, bool second, const SegList& seg, cudaStream_t s) {
+  cudaMemsetAsync(work, 0, 2 * sizeof(unsigned long long), s);
+  if (n <= 0) return cudaGetLastError();
+  const int gp = seg_blocks(n);
+  count_launch(2);
+  k_pairs_early<<<gp, 256, 0, s>>>(n, tet_a, tet_b, setup, tol_a, measure, nout, reinterpret_cast<int4*>(survivors),
+                                   seg.count, second);
+  k_seg_chunks<<<gp, 256, 0, s>>>(n, nullptr, seg.count, seg.table, work);
+  return clip_listed(n, tet_a, tol_a, setup, measure, nout, elems, survivors, work, &seg, s);
 }
 
 
@@ -4346,26 +4476,6 @@ __device__ __forceinline__ int p1_factor_3d(const double* cc, double* F) {
     }
   return sw;
 }
-
-// a / b, correctly rounded, for a divisor whose correctly rounded reciprocal
-// y is at hand.  Markstein (IBM J. Res. Dev. 34, 1990): if q is within one ulp
-// of a/b and y = RN(1/b), then r = a - b q is exact and RN(q + r y) = RN(a/b).
-// a y is within 1.5 ulp, so a first such step brings q within one ulp and the
-// second gives the quotient.  Holds while nothing underflows or overflows:
-// div_range keeps the largest 2 * (high word of |v|) - 2 * high(2^-400), modulo
-// 2^32, of the operands; div_ok(max) is false as soon as one lies outside
-// [2^-400, 2^400] (zero, infinity and NaN included), and the caller then
-// divides.
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-  double q = a * y;
-  q = __fma_rn(__fma_rn(-b, q, a), y, q);
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
-constexpr unsigned kDivLo = (1023u - 400u) << 20, kDivHi = (1023u + 400u) << 20;
-__device__ __forceinline__ unsigned div_range(unsigned range, double v) {
-  return max(range, 2u * (unsigned)__double2hiint(v) - 2u * kDivLo);
-}
-__device__ __forceinline__ bool div_ok(unsigned range) { return range <= 2u * (kDivHi - kDivLo); }
 
 // FAST: the three divisions through the stored reciprocals; range gathers
 // their numerators.

@@ -197,15 +197,11 @@ cudaError_t launch_i32_to_i64(int64_t n, const int32_t* in, int64_t* out, cudaSt
 // Single-pair style batched intersections over explicit element arrays
 // (tri: [n][3][2]; tet: [n][4][3]).  out_elems optional ([n][22][3][2] or
 // [n][81][4][3]).
-// Explicit tetrahedron pairs through the early-out pass and the index
-// clipper: per-pair setup (setup [n][kSetup3], tol_a [n], iota [n]; faces_a /
-// screen_b [n][kScreen3] optional, for the second early-out), then, for
-// measures and counts, launch_clip(3, n, iota, iota, tet_a, ...), or, with
-// the output tets, launch_clip_elems (elems [n][81][4][3]; survivors: 4 ints
-// per pair; work: two counters, three with seg).  tet_a must be 16-byte
-// aligned.
+// Explicit tetrahedron pairs in separate passes (the allocation-free entry):
+// per-pair setup (setup [n][kSetup3], tol_a [n], iota [n]), then
+// launch_clip(3, n, iota, iota, tet_a, ...).  tet_a must be 16-byte aligned.
 cudaError_t launch_setup_pairs3(int64_t n, const double* tet_a, const double* tet_b, double* setup, double* tol_a,
-                                int32_t* iota, double* faces_a, double* screen_b, cudaStream_t s);
+                                int32_t* iota, cudaStream_t s);
 // launch_clip_elems: the 3D narrow phase whose survivor list also holds the
 // pairs with every plane a no-op (so that a second pass over the list sees
 // every pair with output tets); measure/nout for every pair, elems optional;
@@ -214,6 +210,13 @@ cudaError_t launch_clip_elems(int64_t n, const int32_t* pair_a, const int32_t* p
                               const double* tol_a, const double* setup, double* measure, int32_t* nout,
                               double* elems, int32_t* survivors, unsigned long long* work, const double* faces_a,
                               const double* screen_b, cudaStream_t s, const SegList* seg = nullptr);
+// Explicit tetrahedron pairs (16-byte aligned, n < 2^31) through one pass of
+// setup and early-outs (second: both of them) and the clipper: measure / nout
+// per pair and, optionally, elems [n][81][4][3]; setup [n][kSetup3], tol_a [n],
+// survivors 4 ints per pair, work three counters.
+cudaError_t launch_tet_pairs(int64_t n, const double* tet_a, const double* tet_b, double* measure, int32_t* nout,
+                             double* elems, double* setup, double* tol_a, int32_t* survivors,
+                             unsigned long long* work, bool second, const SegList& seg, cudaStream_t s);
 // The supermesh's simplices: pair p's output simplices (reference order) at
 // elems[pair_off[p] ..] ([3][2] or [4][3] doubles each), parents optional.
 // 3D takes the survivor list, work counters and seg of a launch_clip_elems

@@ -106,7 +106,7 @@ extern "C" int libsupermesh_gpu_intersect_tets_noalloc(int64_t n, const double* 
   lsm::Partial* tot = reinterpret_cast<lsm::Partial*>(b + kOffTotal);
   if (n > 0) {
     // B's planes and tolerance, A's tolerance and the identity pair indices
-    if (lsm::launch_setup_pairs3(n, tet_a, tet_b, setup, tol, iota, nullptr, nullptr, s) != cudaSuccess)
+    if (lsm::launch_setup_pairs3(n, tet_a, tet_b, setup, tol, iota, s) != cudaSuccess)
       return LSM_ERROR_CUDA;
     // launch_clip clears the two work counters (survivors, progress) first
     if (lsm::launch_clip(3, n, iota, iota, tet_a, tol, setup, measure, n_out, list, nullptr, work, s) !=

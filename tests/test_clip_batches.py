@@ -102,3 +102,22 @@ def test_tet_hexahedron_batches(gpu_ctx, value):
     ref = [gpu_ctx.intersect_pairs_mixed(lsm.PAIR_TET_HEX, a[i:i + 1000], h[i:i + 1000])[:2] for i in (0, 1000, 2000)]
     assert np.array_equal(got[1], np.concatenate([r[1] for r in ref]))
     assert np.array_equal(got[0], np.concatenate([r[0] for r in ref]))
+
+
+@pytest.mark.parametrize("shift", [0.0, 1.0e4])
+def test_pairs_near_touching_across_a_face_of_a(gpu_ctx, shift):
+    """B on the far side of a face of A at gaps through zero and the rounding
+    margins: the second early-out of the explicit pairs must never drop a
+    pair with output."""
+    rng = np.random.default_rng(11)
+    n = 4000
+    a = rng.random((n, 4, 3))
+    nrm = np.cross(a[:, 1] - a[:, 0], a[:, 2] - a[:, 0])
+    nrm /= np.linalg.norm(nrm, axis=1)[:, None]
+    nrm *= -np.sign(((a[:, 3] - a[:, 0]) * nrm).sum(1))[:, None]  # outwards
+    gap = np.concatenate([[0.0], 10.0 ** -np.arange(3, 17), -10.0 ** -np.arange(3, 17)])[rng.integers(0, 29, n)]
+    base = a[:, 0] + 0.3 * (a[:, 1] - a[:, 0]) + 0.3 * (a[:, 2] - a[:, 0]) + gap[:, None] * nrm
+    u = a[:, 1] - a[:, 0]
+    v = np.cross(nrm, u)
+    b = np.stack([base, base + 0.4 * u, base + 0.4 * v, base + 0.5 * nrm + 0.1 * u], axis=1)
+    _same(gpu_ctx.intersect_pairs(3, a + shift, b + shift, want_elems=True), _small(gpu_ctx, a + shift, b + shift))
