@@ -515,13 +515,13 @@ lsm::Tree build_tree(Ctx* c, const MeshDev& b, cudaStream_t s) {
   uint32_t* hist = ensure<uint32_t>(c, c->hist, lsm::radix_hist_entries(n));
   const int pcap = 4096;
   double* part = ensure<double>(c, c->root_partial, (int64_t)pcap * 2 * dim);
-  double* root = ensure<double>(c, c->rootbox, 2 * dim + 1);
-  unsigned* ticket = reinterpret_cast<unsigned*>(root + 2 * dim);
+  double* root = ensure<double>(c, c->rootbox, 2 * dim);
+  unsigned* ticket = reinterpret_cast<unsigned*>(bad_flag(c) + 40);  // two, zeroed with the flags
   CU(lsm::launch_root_box(dim, n, static_cast<double*>(c->b_box64.p), part, pcap, root, ticket, s));
-  CU(lsm::launch_morton(dim, n, static_cast<double*>(c->b_box64.p), root, keys, vals, s));
-  CU(lsm::radix_sort_pairs(n, dim == 2 ? 32 : 30, keys, vals, kt, vt, hist, s, bad_flag(c) + 3));
+  CU(lsm::launch_morton(dim, n, static_cast<double*>(c->b_box64.p), root, keys, vals, hist, s));
+  CU(lsm::radix_sort_pairs(n, dim == 2 ? 32 : 30, keys, vals, kt, vt, hist, s, bad_flag(c) + 3, true, false));
   const lsm::Tree tree = lsm::make_tree(dim, (int)n, vals, ensure<float>(c, c->tree_rec, lsm::tree_floats(dim, n)));
-  CU(lsm::launch_tree_build(dim, tree, static_cast<float*>(c->b_box32.p), ticket, s));
+  CU(lsm::launch_tree_build(dim, tree, static_cast<float*>(c->b_box32.p), ticket + 1, bad_flag(c) + 3, s));
   return tree;
 }
 
@@ -1043,17 +1043,17 @@ bool run_batch_group(Ctx* c, int dim, const std::vector<int>& idx, const lsm_gpu
     uint32_t* hist = ensure<uint32_t>(c, c->hist, lsm::radix_hist_entries(nb));
     const int pcap = 4096;
     double* part = ensure<double>(c, c->root_partial, (int64_t)pcap * 2 * dim);
-    double* root = ensure<double>(c, c->rootbox, 2 * dim + 1);
-    unsigned* ticket = reinterpret_cast<unsigned*>(root + 2 * dim);
+    double* root = ensure<double>(c, c->rootbox, 2 * dim);
+    unsigned* ticket = reinterpret_cast<unsigned*>(bad + 40);  // two, zeroed with the flags
     CU(lsm::launch_root_box(dim, nb, b_box, part, pcap, root, ticket, s));
-    CU(lsm::launch_morton(dim, nb, b_box, root, keys, vals, s));
-    CU(lsm::radix_sort_pairs(nb, dim == 2 ? 32 : 30, keys, vals, kt, vt, hist, s, bad + 3));
+    CU(lsm::launch_morton(dim, nb, b_box, root, keys, vals, hist, s));
+    CU(lsm::radix_sort_pairs(nb, dim == 2 ? 32 : 30, keys, vals, kt, vt, hist, s, bad + 3, true));
     int mbits = 1;
     while ((1 << mbits) < nm) ++mbits;
     CU(lsm::launch_pair_keys(nb, vals, pair_of_b, keys, s));
-    CU(lsm::radix_sort_pairs(nb, mbits, keys, vals, kt, vt, hist, s, bad + 3));
+    CU(lsm::radix_sort_pairs(nb, mbits, keys, vals, kt, vt, hist, s, bad + 3, false, false));
     tree = lsm::make_tree(dim, (int)nb, vals, ensure<float>(c, c->tree_rec, lsm::tree_floats(dim, nb)));
-    CU(lsm::launch_tree_build(dim, tree, b_box32, ticket, s));
+    CU(lsm::launch_tree_build(dim, tree, b_box32, ticket + 1, bad + 3, s));
   }
   int64_t* offsets = ensure<int64_t>(c, c->offsets, na + 1);
   int* counts = ensure<int>(c, c->counts, na);

@@ -363,7 +363,8 @@ cudaError_t launch_prep_batched(int dim, int64_t nel, int nm, const int64_t* ele
 // K1b: root box and Morton keys
 // ======================================================================
 template <int DIM>
-__global__ void k_root_partial(int64_t nel, const double* __restrict__ box64, double* partial) {
+__global__ void __launch_bounds__(256) k_root_box(int64_t nel, const double* __restrict__ box64, double* partial,
+                                                  double* root, unsigned* ticket) {
   double lo[DIM], hi[DIM];
 #pragma unroll
   for (int c = 0; c < DIM; ++c) {
@@ -378,81 +379,58 @@ __global__ void k_root_partial(int64_t nel, const double* __restrict__ box64, do
       hi[c] = fmax(hi[c], box64[e * 2 * DIM + DIM + c]);
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      lo[c] = fmin(lo[c], __shfl_down_sync(0xffffffffu, lo[c], o));
-      hi[c] = fmax(hi[c], __shfl_down_sync(0xffffffffu, hi[c], o));
-    }
-  __shared__ double sl[32][DIM], sh[32][DIM];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0)
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      sl[wid][c] = lo[c];
-      sh[wid][c] = hi[c];
-    }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-#pragma unroll
-      for (int c = 0; c < DIM; ++c) {
-        lo[c] = fmin(lo[c], sl[w][c]);
-        hi[c] = fmax(hi[c], sh[w][c]);
-      }
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      partial[blockIdx.x * 2 * DIM + c] = lo[c];
-      partial[blockIdx.x * 2 * DIM + DIM + c] = hi[c];
-    }
-  }
-}
-
-template <int DIM>
-__global__ void __launch_bounds__(256) k_root_final(int np, const double* partial, double* root,
-                                                    unsigned* ticket) {
-  double lo[DIM], hi[DIM];
-#pragma unroll
-  for (int c = 0; c < DIM; ++c) {
-    lo[c] = DBL_MAX;
-    hi[c] = -DBL_MAX;
-  }
-  for (int b = threadIdx.x; b < np; b += blockDim.x)
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      lo[c] = fmin(lo[c], partial[b * 2 * DIM + c]);
-      hi[c] = fmax(hi[c], partial[b * 2 * DIM + DIM + c]);
-    }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      lo[c] = fmin(lo[c], __shfl_down_sync(0xffffffffu, lo[c], o));
-      hi[c] = fmax(hi[c], __shfl_down_sync(0xffffffffu, hi[c], o));
-    }
   __shared__ double sl[8][DIM], sh[8][DIM];
+  __shared__ bool s_last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0)
+  // the block's box, then, in the block that finishes last (*ticket, zero
+  // before the launch), the box of all blocks' boxes
+  for (int pass = 0; pass < 2; ++pass) {
 #pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      sl[wid][c] = lo[c];
-      sh[wid][c] = hi[c];
-    }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    *ticket = 0;
-    for (int w = 1; w < 8; ++w)
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
       for (int c = 0; c < DIM; ++c) {
-        lo[c] = fmin(lo[c], sl[w][c]);
-        hi[c] = fmax(hi[c], sh[w][c]);
+        lo[c] = fmin(lo[c], __shfl_down_sync(0xffffffffu, lo[c], o));
+        hi[c] = fmax(hi[c], __shfl_down_sync(0xffffffffu, hi[c], o));
       }
+    if (lane == 0)
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        sl[wid][c] = lo[c];
+        sh[wid][c] = hi[c];
+      }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 8; ++w)
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) {
+          lo[c] = fmin(lo[c], sl[w][c]);
+          hi[c] = fmax(hi[c], sh[w][c]);
+        }
+      double* o = pass == 0 ? partial + (int64_t)blockIdx.x * 2 * DIM : root;
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        o[c] = lo[c];
+        o[DIM + c] = hi[c];
+      }
+      if (pass == 0) {
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        __threadfence();
+      }
+    }
+    __syncthreads();
+    if (pass == 1 || !s_last) return;
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
-      root[c] = lo[c];
-      root[DIM + c] = hi[c];
+      lo[c] = DBL_MAX;
+      hi[c] = -DBL_MAX;
     }
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        lo[c] = fmin(lo[c], __ldcg(partial + b * 2 * DIM + c));
+        hi[c] = fmax(hi[c], __ldcg(partial + b * 2 * DIM + DIM + c));
+      }
   }
 }
 
@@ -461,14 +439,11 @@ cudaError_t launch_root_box(int dim, int64_t nel, const double* box64, double* p
   const int B = 256;
   int g = grid_for(nel, B, 2);
   if (g > partial_cap) g = partial_cap;
-  count_launch(2);
-  if (dim == 2) {
-    k_root_partial<2><<<g, B, 0, s>>>(nel, box64, partial);
-    k_root_final<2><<<1, 256, 0, s>>>(g, partial, rootbox, ticket);
-  } else {
-    k_root_partial<3><<<g, B, 0, s>>>(nel, box64, partial);
-    k_root_final<3><<<1, 256, 0, s>>>(g, partial, rootbox, ticket);
-  }
+  count_launch();
+  if (dim == 2)
+    k_root_box<2><<<g, B, 0, s>>>(nel, box64, partial, rootbox, ticket);
+  else
+    k_root_box<3><<<g, B, 0, s>>>(nel, box64, partial, rootbox, ticket);
   return cudaGetLastError();
 }
 
@@ -490,9 +465,14 @@ __device__ __forceinline__ uint32_t spread3(uint32_t x) {  // 10 bits -> every 3
   return x;
 }
 
+// counts: the sort's digit counts of all four passes (k_radix_counts).
 template <int DIM>
-__global__ void k_morton(int64_t nel, const double* __restrict__ box64, const double* __restrict__ root,
-                         uint32_t* keys, int32_t* vals) {
+__global__ void __launch_bounds__(256) k_morton(int64_t nel, const double* __restrict__ box64,
+                                                const double* __restrict__ root, uint32_t* keys, int32_t* vals,
+                                                uint32_t* counts) {
+  __shared__ uint32_t h[4][256];
+  for (int i = threadIdx.x; i < 4 * 256; i += 256) (&h[0][0])[i] = 0;
+  __syncthreads();
   constexpr double kScale = DIM == 2 ? 65536.0 : 1024.0;
   constexpr uint32_t kMax = DIM == 2 ? 65535u : 1023u;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nel;
@@ -514,20 +494,14 @@ __global__ void k_morton(int64_t nel, const double* __restrict__ box64, const do
       key = (spread3(q[DIM - 1]) << 2) | (spread3(q[1]) << 1) | spread3(q[0]);
     keys[e] = key;
     vals[e] = (int32_t)e;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) atomicAdd(&h[p][(key >> (8 * p)) & 255u], 1u);
   }
-}
-
-cudaError_t launch_morton(int dim, int64_t nel, const double* box64, const double* rootbox,
-                          uint32_t* keys, int32_t* vals, cudaStream_t s) {
-  if (nel <= 0) return cudaSuccess;
-  const int B = 256;
-  const int g = grid_for(nel, B, 8);
-  count_launch();
-  if (dim == 2)
-    k_morton<2><<<g, B, 0, s>>>(nel, box64, rootbox, keys, vals);
-  else
-    k_morton<3><<<g, B, 0, s>>>(nel, box64, rootbox, keys, vals);
-  return cudaGetLastError();
+  __syncthreads();
+  for (int i = threadIdx.x; i < 4 * 256; i += 256) {
+    const uint32_t c = (&h[0][0])[i];
+    if (c) atomicAdd(&counts[i], c);
+  }
 }
 
 // ======================================================================
@@ -539,6 +513,7 @@ constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortItems = 8;                           // per thread
 constexpr int kSortTile = kSortThreads * kSortItems;  // 2048 keys per block
 constexpr int kWarpTile = 32 * kSortItems;             // contiguous per warp
+constexpr int kLookBack = 8;                            // blocks looked back over at once
 }  // namespace
 
 // Single-pass digit binning per pass ("onesweep"): one kernel counts every
@@ -555,12 +530,12 @@ constexpr int kWarpTile = 32 * kSortItems;             // contiguous per warp
 // count (n < 2^30).  Waits are bounded: a block that gives up sets err and
 // treats the missing prefix as 0 (wrong order, never a hang); forward
 // progress does not need the bound, since a block only waits for blocks
-// that took earlier tickets and are running or done.  A partial prefix only
-// lowers the scatter positions, so they stay inside [0, n); some keys then
-// overwrite others, and k_sort_repair turns the output back into a
-// permutation (identity values, equal keys) so that the kernels after the
-// sort never read an element number that does not exist.  The caller sees
-// err and reports the failure.
+// that took earlier tickets and are running or done.  After that some keys
+// overwrite others and a later pass reads what the gaps held, so positions
+// are checked, and k_sort_repair (or k_tree_build, which reads the same word)
+// turns the output back into a permutation (identity values, equal keys) so
+// that the kernels after the sort never read an element number that does not
+// exist.  The caller sees err and reports the failure.
 //
 // Test hooks (process-wide, off by default): the bound of each wait
 // (set_sort_spin_limit) and one block per pass that never publishes its
@@ -585,6 +560,24 @@ int sort_stall_block() { return g_sort_stall; }
 int64_t radix_hist_entries(int64_t n) {
   const int64_t nb = (n + kSortTile - 1) / kSortTile;
   return kSortHdr + (int64_t)kSortPassesMax * 256 * (nb > 0 ? nb : 1);
+}
+
+// Words of the scratch that a sort of n keys in `passes` passes needs zeroed.
+static int64_t radix_zeros(int64_t n, int passes) {
+  return kSortHdr + (int64_t)passes * 256 * ((n + kSortTile - 1) / kSortTile);
+}
+
+cudaError_t launch_morton(int dim, int64_t nel, const double* box64, const double* rootbox, uint32_t* keys,
+                          int32_t* vals, uint32_t* hist, cudaStream_t s) {
+  if (nel <= 0) return cudaSuccess;
+  cudaMemsetAsync(hist, 0, sizeof(uint32_t) * radix_zeros(nel, kSortPassesMax), s);
+  const int g = grid_for(nel, 256, 8);
+  count_launch();
+  if (dim == 2)
+    k_morton<2><<<g, 256, 0, s>>>(nel, box64, rootbox, keys, vals, hist);
+  else
+    k_morton<3><<<g, 256, 0, s>>>(nel, box64, rootbox, keys, vals, hist);
+  return cudaGetLastError();
 }
 
 __global__ void __launch_bounds__(kSortThreads) k_radix_counts(int64_t n, int passes,
@@ -621,15 +614,23 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_onesweep(int64_t n, int 
   __syncthreads();
   const int b = bid_s;
   const int64_t base = (int64_t)b * kSortTile + (int64_t)wid * kWarpTile;
-  uint32_t k[kSortItems];
-  int dg[kSortItems];
+  const uint32_t digit_count = counts[threadIdx.x];
+  uint32_t k[kSortItems], rank[kSortItems];
+  int32_t v[kSortItems];
 #pragma unroll
   for (int r = 0; r < kSortItems; ++r) {
     const int64_t i = base + r * 32 + lane;
     k[r] = i < n ? keys_in[i] : 0u;
-    dg[r] = i < n ? (int)((k[r] >> shift) & 255u) : 256;
-    const unsigned peers = __match_any_sync(0xffffffffu, dg[r]);
-    if (dg[r] < 256 && (peers & lt) == 0) wh[wid][dg[r]] += __popc(peers);
+    v[r] = i < n ? vals_in[i] : 0;
+  }
+#pragma unroll
+  for (int r = 0; r < kSortItems; ++r) {
+    // rank among the warp's keys of the same digit, in key order
+    const int dg = base + r * 32 + lane < n ? (int)((k[r] >> shift) & 255u) : 256;
+    const unsigned peers = __match_any_sync(0xffffffffu, dg);
+    if (dg < 256) rank[r] = wh[wid][dg] + __popc(peers & lt);
+    __syncwarp();
+    if (dg < 256 && (peers & lt) == 0) wh[wid][dg] += __popc(peers);
     __syncwarp();
   }
   __syncthreads();
@@ -641,27 +642,44 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_onesweep(int64_t n, int 
   cuda::atomic_ref<uint32_t, cuda::thread_scope_device> mine(status[(int64_t)b * 256 + d]);
   const bool publish = b != stall;
   if (publish) mine.store((b == 0 ? kFlagIncl : kFlagLocal) | local, cuda::memory_order_relaxed);
+  // (kLookBack blocks' words at once: with all blocks of a pass resident the
+  // chain of single look-backs was most of its time)
   uint32_t prefix = 0;
-  for (int j = b - 1; j >= 0;) {
-    cuda::atomic_ref<uint32_t, cuda::thread_scope_device> st(status[(int64_t)j * 256 + d]);
-    uint32_t v = st.load(cuda::memory_order_relaxed);
-    for (int spin = 0; (v & kFlagMask) == 0; ++spin) {
-      if (spin > spin_limit) {
-        atomicExch(err, 1u);
-        v = kFlagIncl;
-        break;
-      }
-      __nanosleep(64);
-      v = st.load(cuda::memory_order_relaxed);
+  bool more = true;
+  for (int j = b - 1; more && j >= 0; j -= kLookBack) {
+    uint32_t w[kLookBack];
+#pragma unroll
+    for (int q = 0; q < kLookBack; ++q) {
+      w[q] = kFlagIncl;
+      if (j - q >= 0)
+        w[q] = cuda::atomic_ref<uint32_t, cuda::thread_scope_device>(status[(int64_t)(j - q) * 256 + d])
+                   .load(cuda::memory_order_relaxed);
     }
-    prefix += v & ~kFlagMask;
-    if ((v & kFlagMask) == kFlagIncl) break;
-    --j;
+#pragma unroll
+    for (int q = 0; q < kLookBack; ++q) {
+      if (!more) continue;
+      uint32_t x = w[q];
+      if ((x & kFlagMask) == 0) {
+        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> st(status[(int64_t)(j - q) * 256 + d]);
+        x = st.load(cuda::memory_order_relaxed);
+        for (int spin = 0; (x & kFlagMask) == 0; ++spin) {
+          if (spin > spin_limit) {
+            atomicExch(err, 1u);
+            x = kFlagIncl;
+            break;
+          }
+          __nanosleep(64);
+          x = st.load(cuda::memory_order_relaxed);
+        }
+      }
+      prefix += x & ~kFlagMask;
+      more = (x & kFlagMask) != kFlagIncl;
+    }
   }
   if (b > 0 && publish) mine.store(kFlagIncl | (prefix + local), cuda::memory_order_relaxed);
   // global start of digit d: exclusive scan of the pass's digit counts
   {
-    const uint32_t c = counts[d];
+    const uint32_t c = digit_count;
     uint32_t inc = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -686,16 +704,13 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_onesweep(int64_t n, int 
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < kSortItems; ++r) {
-    const int64_t i = base + r * 32 + lane;
-    const unsigned peers = __match_any_sync(0xffffffffu, dg[r]);
-    if (dg[r] < 256) {
-      const uint32_t pos = wh[wid][dg[r]] + __popc(peers & lt);
-      keys_out[pos] = k[r];
-      vals_out[pos] = vals_in[i];
+    if (base + r * 32 + lane < n) {
+      const uint32_t pos = wh[wid][(k[r] >> shift) & 255u] + rank[r];
+      if (pos < n) {  // (always, unless a wait gave up)
+        keys_out[pos] = k[r];
+        vals_out[pos] = v[r];
+      }
     }
-    __syncwarp();
-    if (dg[r] < 256 && (peers & lt) == 0) wh[wid][dg[r]] += __popc(peers);
-    __syncwarp();
   }
 }
 
@@ -710,7 +725,8 @@ __global__ void k_sort_repair(int64_t n, const uint32_t* __restrict__ err, uint3
 }
 
 cudaError_t radix_sort_pairs(int64_t n, int bits, uint32_t* keys, int32_t* vals, uint32_t* keys_tmp,
-                             int32_t* vals_tmp, uint32_t* hist, cudaStream_t s, int* err) {
+                             int32_t* vals_tmp, uint32_t* hist, cudaStream_t s, int* err, bool counted,
+                             bool repair) {
   if (n <= 1) return cudaSuccess;
   if (n >= (int64_t)1 << 30 || bits > 32) return cudaErrorInvalidValue;
   const int nb = (int)((n + kSortTile - 1) / kSortTile);
@@ -719,11 +735,11 @@ cudaError_t radix_sort_pairs(int64_t n, int bits, uint32_t* keys, int32_t* vals,
   uint32_t* tickets = hist + kSortPassesMax * 256;
   uint32_t* errw = err ? reinterpret_cast<uint32_t*>(err) : tickets + kSortPassesMax;
   uint32_t* status = hist + kSortHdr;
-  cudaMemsetAsync(hist, 0, sizeof(uint32_t) * (kSortHdr - 4 + (int64_t)passes * 256 * nb + 4), s);
+  if (!counted) cudaMemsetAsync(hist, 0, sizeof(uint32_t) * radix_zeros(n, passes), s);
   uint32_t *ki = keys, *ko = keys_tmp;
   int32_t *vi = vals, *vo = vals_tmp;
-  count_launch(1 + passes);
-  k_radix_counts<<<grid_for(n, kSortThreads, 4), kSortThreads, 0, s>>>(n, passes, ki, counts);
+  count_launch(passes + !counted);
+  if (!counted) k_radix_counts<<<grid_for(n, kSortThreads, 4), kSortThreads, 0, s>>>(n, passes, ki, counts);
   for (int p = 0; p < passes; ++p) {
     k_radix_onesweep<<<nb, kSortThreads, 0, s>>>(n, 8 * p, ki, vi, ko, vo, counts + 256 * p,
                                                  status + (int64_t)p * 256 * nb, tickets + p, errw,
@@ -739,7 +755,7 @@ cudaError_t radix_sort_pairs(int64_t n, int bits, uint32_t* keys, int32_t* vals,
     cudaMemcpyAsync(keys, ki, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s);
     cudaMemcpyAsync(vals, vi, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s);
   }
-  if (err) {
+  if (err && repair) {
     count_launch();
     k_sort_repair<<<grid_for(n, 256, 4), 256, 0, s>>>(n, errw, keys, vals);
   }
@@ -786,11 +802,12 @@ __device__ __forceinline__ void tree_join(const float* __restrict__ rec, int64_t
 constexpr int kTreeBlock = 256;  // threads, one group of leaves each
 
 // Levels 0 to 5 of the block's 1024 leaves; the block that finishes last
-// (*ticket, zero before the launch) builds the levels above.
+// (*ticket, zero before the launch) builds the levels above.  *sort_err: the
+// sort gave up (see k_sort_repair, whose work on vals is done here).
 template <int DIM>
-__global__ void __launch_bounds__(kTreeBlock) k_tree_build(const __grid_constant__ Tree T, const int32_t* __restrict__ vals,
+__global__ void __launch_bounds__(kTreeBlock) k_tree_build(const __grid_constant__ Tree T, int32_t* vals,
                                                            const float4* __restrict__ box32, float* rec,
-                                                           unsigned* ticket) {
+                                                           unsigned* ticket, const int* __restrict__ sort_err) {
   __shared__ float sl[kTreeBlock][DIM], sh[kTreeBlock][DIM];
   __shared__ bool s_last;
   const float inf = __int_as_float(0x7f800000);
@@ -805,6 +822,9 @@ __global__ void __launch_bounds__(kTreeBlock) k_tree_build(const __grid_constant
       L[k] = make_float4(inf, inf, inf, 0.0f);
       H[k] = make_float4(-inf, -inf, -inf, 0.0f);
       if (4 * g + k < T.n) {
+        // (after a sort whose look-back gave up, any permutation will do: the
+        // call reports the failure)
+        if (*sort_err) vals[4 * g + k] = (int32_t)(4 * g + k);
         const int64_t e = vals[4 * g + k];
         L[k] = box32[2 * e];
         H[k] = box32[2 * e + 1];
@@ -889,7 +909,7 @@ int64_t tree_floats(int dim, int64_t n) {
   return g * 8 * dim;
 }
 
-Tree make_tree(int dim, int n, const int32_t* sorted_vals, float* rec) {
+Tree make_tree(int dim, int n, int32_t* sorted_vals, float* rec) {
   Tree T;
   T.n = n;
   T.vals = sorted_vals;
@@ -906,14 +926,17 @@ Tree make_tree(int dim, int n, const int32_t* sorted_vals, float* rec) {
   return T;
 }
 
-cudaError_t launch_tree_build(int dim, const Tree& T, const float* box32, unsigned* ticket, cudaStream_t s) {
+cudaError_t launch_tree_build(int dim, const Tree& T, const float* box32, unsigned* ticket, const int* sort_err,
+                              cudaStream_t s) {
   if (T.n <= 0) return cudaSuccess;
   const int g = (T.off[1] + kTreeBlock - 1) / kTreeBlock;
   count_launch();
   if (dim == 2)
-    k_tree_build<2><<<g, kTreeBlock, 0, s>>>(T, T.vals, reinterpret_cast<const float4*>(box32), T.rec, ticket);
+    k_tree_build<2><<<g, kTreeBlock, 0, s>>>(T, T.vals, reinterpret_cast<const float4*>(box32), T.rec, ticket,
+                                              sort_err);
   else
-    k_tree_build<3><<<g, kTreeBlock, 0, s>>>(T, T.vals, reinterpret_cast<const float4*>(box32), T.rec, ticket);
+    k_tree_build<3><<<g, kTreeBlock, 0, s>>>(T, T.vals, reinterpret_cast<const float4*>(box32), T.rec, ticket,
+                                              sort_err);
   return cudaGetLastError();
 }
 
@@ -1393,9 +1416,71 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(int64_t n, const int
   if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = tmp[nb];
 }
 
+// The whole scan in one block, for counts that three launches would only
+// spread thin (10,658 rows: 11 -> 10 us).  A warp takes 256 counts in
+// four rows of 64, two neighbours a lane, so that its loads and stores are
+// nearly whole lines: with eight neighbours a lane the stores alone, each to
+// 32 lines, took most of 11 us.
+__global__ void __launch_bounds__(1024) k_scan_one(int64_t n, const int* __restrict__ counts, int64_t* out) {
+  constexpr int kRows = 4;
+  __shared__ int64_t wsum[2][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int64_t carry = 0;
+  for (int64_t b0 = 0, it = 0; b0 < n; b0 += 1024 * 2 * kRows, ++it) {
+    const int64_t base = b0 + wid * 64 * kRows + 2 * lane;
+    int v[kRows][2];
+    int64_t ex[kRows];  // before the lane's pair, from the warp's first count
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const int64_t i = base + 64 * r;
+      v[r][0] = i < n ? counts[i] : 0;
+      v[r][1] = i + 1 < n ? counts[i + 1] : 0;
+    }
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) ex[r] = (int64_t)v[r][0] + v[r][1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) {
+        const int64_t t = __shfl_up_sync(0xffffffffu, ex[r], o);
+        if (lane >= o) ex[r] += t;
+      }
+    int64_t run = 0;
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const int64_t tot = __shfl_sync(0xffffffffu, ex[r], 31);
+      ex[r] += run - v[r][0] - v[r][1];
+      run += tot;
+    }
+    // (two rows of sums, so that one barrier a tile is enough)
+    if (lane == 0) wsum[it & 1][wid] = run;
+    __syncthreads();
+    int64_t w = wsum[it & 1][lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t t = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += t;
+    }
+    const int64_t first = carry + __shfl_sync(0xffffffffu, w, wid) - run;
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const int64_t i = base + 64 * r;
+      if (i < n) out[i] = first + ex[r];
+      if (i + 1 < n) out[i + 1] = first + ex[r] + v[r][0];
+    }
+    carry += __shfl_sync(0xffffffffu, w, 31);
+  }
+  if (threadIdx.x == 0) out[n] = carry;
+}
+
 cudaError_t launch_scan(int64_t n, const int* counts, int64_t* offsets, int64_t* tmp, cudaStream_t s) {
   if (n <= 0) {
     cudaMemsetAsync(offsets, 0, sizeof(int64_t), s);
+    return cudaGetLastError();
+  }
+  if (n <= 32 << 10) {
+    count_launch();
+    k_scan_one<<<1, 1024, 0, s>>>(n, counts, offsets);
     return cudaGetLastError();
   }
   const int nb = (int)((n + kScanTile - 1) / kScanTile);

@@ -58,14 +58,15 @@ void set_leaf_bucket(int v);
 struct Tree {
   int n = 0;
   int top = 0;
-  const int32_t* vals = nullptr;
+  int32_t* vals = nullptr;
   float* rec = nullptr;
   int off[18] = {};
 };
 int64_t tree_floats(int dim, int64_t n);  // size of rec
-Tree make_tree(int dim, int n, const int32_t* sorted_vals, float* rec);
-// ticket: a zero (launch_root_box leaves one)
-cudaError_t launch_tree_build(int dim, const Tree& T, const float* box32, unsigned* ticket, cudaStream_t s);
+Tree make_tree(int dim, int n, int32_t* sorted_vals, float* rec);
+// ticket: a zero; *sort_err: the sort's err word
+cudaError_t launch_tree_build(int dim, const Tree& T, const float* box32, unsigned* ticket, const int* sort_err,
+                              cudaStream_t s);
 
 // Mesh prep: gather coordinates, boxes, measures/tolerances, B clip setup.
 // idx_bytes selects the enlist element type (4 = int32, 8 = int64).
@@ -74,12 +75,14 @@ cudaError_t launch_prep(int dim, int loc, int64_t nel, const double* pos, const 
                         int* bad_index, int64_t nnodes, cudaStream_t s, double* faces = nullptr,
                         double* screen = nullptr);
 
-// Root box (float64) of a set of element boxes: rootbox[2*dim]; *ticket = 0.
+// Root box (float64) of a set of element boxes: rootbox[2*dim]; ticket: a zero.
 cudaError_t launch_root_box(int dim, int64_t nel, const double* box64, double* partial,
                             int partial_cap, double* rootbox, unsigned* ticket, cudaStream_t s);
 
-cudaError_t launch_morton(int dim, int64_t nel, const double* box64, const double* rootbox,
-                          uint32_t* keys, int32_t* vals, cudaStream_t s);
+// Morton keys of the box centres, and the digit counts of their sort in hist
+// (zeroed here): radix_sort_pairs then takes counted = true.
+cudaError_t launch_morton(int dim, int64_t nel, const double* box64, const double* rootbox, uint32_t* keys,
+                          int32_t* vals, uint32_t* hist, cudaStream_t s);
 
 // Stable LSD radix sort of (key, val) pairs, 8 bits per pass over the low
 // `bits` bits (at most 32), n < 2^30.  tmp buffers must hold n entries; hist
@@ -96,7 +99,8 @@ int sort_spin_limit();
 void set_sort_stall_block(int b);
 int sort_stall_block();
 cudaError_t radix_sort_pairs(int64_t n, int bits, uint32_t* keys, int32_t* vals, uint32_t* keys_tmp,
-                             int32_t* vals_tmp, uint32_t* hist, cudaStream_t s, int* err = nullptr);
+                             int32_t* vals_tmp, uint32_t* hist, cudaStream_t s, int* err = nullptr,
+                             bool counted = false, bool repair = true);
 
 // Spill pool of the count pass's row cache: rows longer than the cache
 // continue in chunks of kSpillChunk candidates (pool[chunks][kSpillChunk]),

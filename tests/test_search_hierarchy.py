@@ -70,3 +70,27 @@ def test_both_traversals_give_the_same_rows(gpu_ctx, dim, na):
     ips, inds = _check(gpu_ctx, (pos, en[:3000]), B)
     assert np.array_equal(ip[:3001], ips)
     assert np.array_equal(ind[:ips[-1]], inds)
+
+
+@pytest.mark.parametrize("na", [1, 63, 65, 255, 257, 8191, 8193, 16385, 32768, 32769])
+def test_row_offsets_at_the_scan_edges(gpu_ctx, na):
+    """Row counts around a warp's rows, a tile and the one-block scan's limit;
+    the offsets are whole numbers, compared exactly."""
+    rng = np.random.default_rng(na)
+    A, B = _elements(2, na, rng, 0.05), _elements(2, 40, rng, 0.2)
+    ip, ind = _rows(gpu_ctx, A, B)
+    va, vb = A[0][A[1]], B[0][B[1]]
+    hit = ((va.max(1)[:, None] > vb.min(1)[None]) & (va.min(1)[:, None] < vb.max(1)[None])).all(2)
+    assert np.array_equal(ip, np.concatenate([[0], np.cumsum(hit.sum(1))]))
+    assert np.array_equal(np.sort(ind + 40 * np.repeat(np.arange(na), hit.sum(1))), np.flatnonzero(hit))
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("nb", [2047, 2049, 2048 * 8 + 1, 2048 * 9, 2048 * 17 + 5])
+def test_sort_look_back_edges(gpu_ctx, dim, nb):
+    """Trees over one to 18 blocks of the sort, whose look-back takes eight
+    blocks at a time; a third of the keys equal."""
+    rng = np.random.default_rng(nb)
+    pos, en = _elements(dim, nb, rng, 0.05)
+    pos[: (dim + 1) * (nb // 3)] = np.tile(pos[: dim + 1], (nb // 3, 1))
+    _check(gpu_ctx, _elements(dim, 60, rng, 0.1), (pos, en))
