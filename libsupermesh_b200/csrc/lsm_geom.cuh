@@ -139,6 +139,11 @@ __device__ __forceinline__ void tri_lines(const double* v, Lines& L) {
   }
 }
 
+// Whether tri_lines turns the normals around.
+__device__ __forceinline__ bool tri_flipped(const double* v) {
+  return (v[2] - v[0]) * -(v[1] - v[5]) + (v[3] - v[1]) * (v[0] - v[4]) > 0.0;
+}
+
 // Edge lines of a convex polygon B with `loc` vertices
 // (Triangle_Intersection.F90:422-451): normal (y_{i+1}-y_i, -(x_{i+1}-x_i)),
 // point v_i, all flipped when (v_1 - p_2) . n_2 > 0.
@@ -479,6 +484,95 @@ __device__ __forceinline__ int clip_tri(double ax0, double ay0, double ax1, doub
     yi = yj;
   }
   return kept;
+}
+
+// The same clip for lanes that stay together, on a polygon in place (vertex i
+// at p[i * B]).  A stage takes all distances of its at most N vertices first,
+// as bit masks, then both crossed edges at once: a walk along the vertices
+// that divides wherever a lane meets a crossed edge ran with 12 of 32 lanes.
+// Only vertices whose place changes are written.  n becomes 0 when less than
+// a triangle is left.  More than two crossed edges (not a convex polygon any
+// more, by rounding) set wide: clip_tri then has to do the pair.
+template <int N, int B>
+__device__ __forceinline__ void clip_stage_c(double2* p, const double2 (&v)[N], int& n, bool& wide, double nx,
+                                             double ny, double px, double py) {
+  unsigned neg = 0, keep = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const double d = nx * (v[i].x - px) + ny * (v[i].y - py);
+    neg |= d < 0.0 ? 1u << i : 0u;
+    keep |= d <= 0.0 ? 1u << i : 0u;
+  }
+  const unsigned all = (1u << n) - 1u;  // (vertices from n on are leftovers)
+  neg &= all;
+  keep &= all;
+  if (keep == all) return;
+  const unsigned pos = all & ~keep;
+  // bit i: vertex i + 1 (the first after the last)
+  const unsigned npos = pos >> 1 | (pos & 1u) << (n - 1), nneg = neg >> 1 | (neg & 1u) << (n - 1);
+  const unsigned cut = (neg & npos) | (pos & nneg);
+  const unsigned rest = cut & (cut - 1u);
+  const int m = __popc(keep) + __popc(cut);
+  if (m < 3) {
+    n = 0;
+    return;
+  }
+  if (rest & (rest - 1u)) {
+    wide = true;
+    n = 0;
+    return;
+  }
+  double2 c1 = {0.0, 0.0}, c2 = {0.0, 0.0};
+  int at1 = 0, at2 = 0;
+  if (cut) {
+    const int e1 = __ffs(cut) - 1, e2 = rest ? __ffs(rest) - 1 : e1;
+    const double2 s1 = p[e1 * B], t1 = p[(e1 + 1 == n ? 0 : e1 + 1) * B];
+    const double2 s2 = p[e2 * B], t2 = p[(e2 + 1 == n ? 0 : e2 + 1) * B];
+    const double ds1 = fabs(nx * (s1.x - px) + ny * (s1.y - py)), dt1 = fabs(nx * (t1.x - px) + ny * (t1.y - py));
+    const double ds2 = fabs(nx * (s2.x - px) + ny * (s2.y - py)), dt2 = fabs(nx * (t2.x - px) + ny * (t2.y - py));
+    double f1 = ds1 / (ds1 + dt1), f2 = ds2 / (ds2 + dt2);
+    f1 = f1 <= 1.0 ? f1 : 1.0;  // (never negative; NaN becomes 1)
+    f2 = f2 <= 1.0 ? f2 : 1.0;
+    c1 = make_double2(s1.x + f1 * (t1.x - s1.x), s1.y + f1 * (t1.y - s1.y));
+    c2 = make_double2(s2.x + f2 * (t2.x - s2.x), s2.y + f2 * (t2.y - s2.y));
+    at1 = __popc(keep & ((2u << e1) - 1u));
+    at2 = __popc(keep & ((2u << e2) - 1u)) + (rest ? 1 : 0);
+  }
+  int o = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    if ((keep >> i & 1u) && o != i) p[o * B] = v[i];
+    o += (int)(keep >> i & 1u) + (int)(cut >> i & 1u);
+  }
+  if (cut) {
+    p[at1 * B] = c1;
+    p[at2 * B] = c2;
+  }
+  n = m;
+}
+
+// The polygon of A clipped to B's lines: its vertex count (0: none), -1 for
+// a pair that needs clip_tri.  p: six vertices.
+template <int B>
+__device__ __forceinline__ int clip_tri_c(const double2 (&a)[3], const Lines& L, double2* p, bool on) {
+  int n = on ? 3 : 0;
+  bool wide = false;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) p[i * B] = a[i];
+  clip_stage_c<3, B>(p, a, n, wide, L.nx[0], L.ny[0], L.px[0], L.py[0]);
+  if (n) {
+    double2 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = p[i * B];
+    clip_stage_c<4, B>(p, v, n, wide, L.nx[1], L.ny[1], L.px[1], L.py[1]);
+  }
+  if (n) {
+    double2 v[5];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) v[i] = p[i * B];
+    clip_stage_c<5, B>(p, v, n, wide, L.nx[2], L.ny[2], L.px[2], L.py[2]);
+  }
+  return wide ? -1 : n;
 }
 
 // ------------------------------------------------------------ tet clipping

@@ -225,15 +225,10 @@ __device__ __forceinline__ void prep_element(int64_t e, const double* __restrict
   if (tolv) tolv[e] = tol;
   if (setup) {
     if (DIM == 2) {
-      Lines L;
-      tri_lines(v, L);
       double* o = setup + e * kSetup2;
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        st2(o + 4 * i, L.nx[i], L.ny[i]);
-        st2(o + 4 * i + 2, L.px[i], L.py[i]);
-      }
-      st2(o + 12, tol, 0.0);
+      for (int i = 0; i < 3; ++i) st2(o + 2 * i, v[2 * i], v[2 * i + 1]);
+      st2(o + 6, tol, tri_flipped(v) ? 1.0 : -1.0);
     } else {
       Planes P;
       tet_planes(t, P);
@@ -1496,22 +1491,10 @@ cudaError_t launch_scan(int64_t n, const int* counts, int64_t* offsets, int64_t*
 // ======================================================================
 namespace {
 constexpr int kTriBlock = 128;
-constexpr int kTriCap = 8;  // fast-path polygon slots (geometric max is 6)
+constexpr int kTriCap = 6;  // fast-path polygon slots (the geometric maximum)
 constexpr int kTriWideCap = 24;
 constexpr int kTetStack = 6;      // max pending tets: 2 per level for planes 0-2
 }  // namespace
-
-// Polygon in shared memory: slot i, coord c at base[(2*i + c) * BLOCK].
-template <int BLOCK>
-struct SmemPoly {
-  double* base;
-  __device__ __forceinline__ double x(int i) const { return base[(2 * i) * BLOCK]; }
-  __device__ __forceinline__ double y(int i) const { return base[(2 * i + 1) * BLOCK]; }
-  __device__ __forceinline__ void set(int i, double px, double py) {
-    base[(2 * i) * BLOCK] = px;
-    base[(2 * i + 1) * BLOCK] = py;
-  }
-};
 
 template <int CAP>
 struct LocalPoly {
@@ -1528,18 +1511,21 @@ struct NoEmit {
   __device__ __forceinline__ void operator()(int, double, double, double, double, double, double) const {}
 };
 
-// A setup row of kSetup2 doubles (16-byte aligned) in seven 16-byte loads.
+// A 2D setup row in four 16-byte loads: the vertices, the tolerance and, as
+// a sign, the orientation.  The lines' normals are differences of the vertices
+// (tri_lines); rows with the lines written out were 112 bytes of gathered
+// loads a pair.
 __device__ __forceinline__ void load_lines(const double* __restrict__ o, Lines& L, double& tol) {
   const double2* q = reinterpret_cast<const double2*>(o);
+  const double2 v[3] = {__ldg(q), __ldg(q + 1), __ldg(q + 2)}, t = __ldg(q + 3);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const double2 n = __ldg(q + 2 * i), pt = __ldg(q + 2 * i + 1);
-    L.nx[i] = n.x;
-    L.ny[i] = n.y;
-    L.px[i] = pt.x;
-    L.py[i] = pt.y;
+    L.nx[i] = (v[(i + 1) % 3].y - v[i].y) * t.y;
+    L.ny[i] = (v[i].x - v[(i + 1) % 3].x) * t.y;
+    L.px[i] = v[i].x;
+    L.py[i] = v[i].y;
   }
-  tol = __ldg(q + 6).x;
+  tol = t.x;
 }
 
 __global__ void __launch_bounds__(kTriBlock) k_clip_tris(int64_t npairs, const int32_t* __restrict__ pa,
@@ -1553,41 +1539,58 @@ __global__ void __launch_bounds__(kTriBlock) k_clip_tris(int64_t npairs, const i
                                                          const int64_t* __restrict__ n_dev) {
   // n_dev (optional): the pair count on the device, npairs its upper bound
   if (n_dev && *n_dev < npairs) npairs = *n_dev;
-  __shared__ double poly[2 * 2 * kTriCap * kTriBlock];
-  SmemPoly<kTriBlock> p{poly + threadIdx.x}, q{poly + 2 * kTriCap * kTriBlock + threadIdx.x};
+  __shared__ double2 poly[kTriCap * kTriBlock];
+  double2* p = poly + threadIdx.x;
   // each iteration loads the next one's pair indices (which stream from
-  // DRAM) before it clips its own pair
+  // DRAM) before it clips its own pair; a warp's lanes go on together
   const int64_t stride = (int64_t)gridDim.x * kTriBlock;
-  int64_t ni = (int64_t)blockIdx.x * kTriBlock + threadIdx.x;
+  int64_t j = (int64_t)blockIdx.x * kTriBlock + threadIdx.x;
+  int64_t ni = j;
   int na = 0, nb = 0;
-  if (ni < npairs) {
+  if (j < npairs) {
     if (order) ni = order[ni];
     na = pa[ni];
     nb = pb[ni];
   }
-  for (int64_t j = (int64_t)blockIdx.x * kTriBlock + threadIdx.x; j < npairs; j += stride) {
+  for (; j - (threadIdx.x & 31) < npairs; j += stride) {
     const int64_t i = ni;
     const int a = na, b = nb;
+    const bool on = j < npairs;
     if (j + stride < npairs) {
       ni = order ? (int64_t)order[j + stride] : j + stride;
       na = pa[ni];
       nb = pb[ni];
     }
     const double2* va = reinterpret_cast<const double2*>(coords_a + (int64_t)a * 6);
-    const double2 v0 = __ldg(va), v1 = __ldg(va + 1), v2 = __ldg(va + 2);
+    const double2 v[3] = {__ldg(va), __ldg(va + 1), __ldg(va + 2)};
     Lines L;
     double tolb;
     load_lines(setup_b + (int64_t)b * kSetup2, L, tolb);
     const double tol = fmin(tol_a[a], tolb);
-    double m;
-    const int n = clip_tri(v0.x, v0.y, v1.x, v1.y, v2.x, v2.y, L, tol, p, q, kTriCap, m, NoEmit{});
-    if (n < 0) {
-      const int k = atomicAdd(ovf_count, 1);
-      ovf_list[k] = (int32_t)i;
-      continue;
+    const int n = clip_tri_c<kTriBlock>(v, L, p, on);
+    double m = 0.0;
+    int kept = 0;
+    if (n > 0) {
+      const double2 o = p[0];
+      double2 s = p[kTriBlock];
+#pragma unroll
+      for (int k = 2; k < kTriCap; ++k) {
+        if (k < n) {
+          const double2 t = p[k * kTriBlock];
+          const double ar = tri_area(o.x, o.y, s.x, s.y, t.x, t.y);
+          const bool in = !(ar < tol);
+          m = in ? m + ar : m;
+          kept += in;
+          s = t;
+        }
+      }
     }
-    pair_measure[i] = m;
-    pair_nout[i] = n;
+    if (n < 0) {
+      ovf_list[atomicAdd(ovf_count, 1)] = (int32_t)i;
+    } else if (on) {
+      pair_measure[i] = m;
+      pair_nout[i] = kept;
+    }
   }
 }
 

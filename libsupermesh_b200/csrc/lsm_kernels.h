@@ -12,10 +12,11 @@ namespace lsm {
 //   coords  [nel][loc*dim]  float64 vertex coordinates (gathered)
 //   box64   [nel][2*dim]    float64 AABB (lo..., hi...)
 //   box32   [nel][8]        float32 AABB rounded outwards (lo.xyz, pad, hi.xyz, pad)
-//   setup   [nel][kSetup]   clip setup of a B element: 2D lines (12) or 3D
-//                           planes (16), then tol = 10*spacing(measure)
+//   setup   [nel][kSetup]   clip setup of a B element: 2D vertices (6), then
+//                           tol = 10*spacing(measure) and the lines'
+//                           orientation; 3D planes (16), then tol
 //   tolv    [nel]           10*spacing(measure) (A elements)
-constexpr int kSetup2 = 14;  // 3 lines x (nx, ny, px, py), tol, pad
+constexpr int kSetup2 = 8;   // 3 x (x, y), tol, 1 (normals (y2 - y1, x1 - x2)) or -1
 constexpr int kSetup3 = 20;  // 4 planes x (nx, ny, nz, c), tol, pad (16-byte aligned rows)
 // Separation screen of the tet clipper (3D simplices, optional):
 //   faces   [nel][kScreen3]  A: 4 outward face planes (nx, ny, nz, h), h
