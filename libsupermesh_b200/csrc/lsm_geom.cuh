@@ -531,8 +531,8 @@ __device__ __forceinline__ void clip_stage_c(double2* p, const double2 (&v)[N], 
     const double ds1 = fabs(nx * (s1.x - px) + ny * (s1.y - py)), dt1 = fabs(nx * (t1.x - px) + ny * (t1.y - py));
     const double ds2 = fabs(nx * (s2.x - px) + ny * (s2.y - py)), dt2 = fabs(nx * (t2.x - px) + ny * (t2.y - py));
     double f1 = ds1 / (ds1 + dt1), f2 = ds2 / (ds2 + dt2);
-    f1 = f1 <= 1.0 ? f1 : 1.0;  // (never negative; NaN becomes 1)
-    f2 = f2 <= 1.0 ? f2 : 1.0;
+    f1 = fmax(fmin(f1, 1.0), 0.0);
+    f2 = fmax(fmin(f2, 1.0), 0.0);
     c1 = make_double2(s1.x + f1 * (t1.x - s1.x), s1.y + f1 * (t1.y - s1.y));
     c2 = make_double2(s2.x + f2 * (t2.x - s2.x), s2.y + f2 * (t2.y - s2.y));
     at1 = __popc(keep & ((2u << e1) - 1u));

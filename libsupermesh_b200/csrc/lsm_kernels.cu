@@ -1490,7 +1490,7 @@ cudaError_t launch_scan(int64_t n, const int* counts, int64_t* offsets, int64_t*
 // K5: triangle clipping
 // ======================================================================
 namespace {
-constexpr int kTriBlock = 128;
+constexpr int kTriBlock = 96;
 constexpr int kTriCap = 6;  // fast-path polygon slots (the geometric maximum)
 constexpr int kTriWideCap = 24;
 constexpr int kTetStack = 6;      // max pending tets: 2 per level for planes 0-2
@@ -1528,7 +1528,13 @@ __device__ __forceinline__ void load_lines(const double* __restrict__ o, Lines& 
   tol = t.x;
 }
 
-__global__ void __launch_bounds__(kTriBlock) k_clip_tris(int64_t npairs, const int32_t* __restrict__ pa,
+// One pair a lane.  Bound by instructions and, next, by shared and L1
+// wavefronts (57 %), both of which divergence multiplies: with the walking
+// clip on 112-byte rows of lines 12 of 32 lanes were active on average and
+// 13.8 M pairs took 1190 us; clip_tri_c alone would have given 1108 (in two
+// buffers), in place and with 64-byte rows 630.  Eight blocks an SM, all
+// resident: 96 threads at 80 registers 629 us, 128 at 64 646, 64 at 104 642.
+__global__ void __launch_bounds__(kTriBlock, 8) k_clip_tris(int64_t npairs, const int32_t* __restrict__ pa,
                                                          const int32_t* __restrict__ pb,
                                                          const double* __restrict__ coords_a,
                                                          const double* __restrict__ tol_a,
