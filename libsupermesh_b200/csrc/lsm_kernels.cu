@@ -1528,6 +1528,26 @@ __device__ __forceinline__ void load_lines(const double* __restrict__ o, Lines& 
   tol = t.x;
 }
 
+// The supermesh triangles of one pair, as clip_tri gives them, by way of
+// clip_tri_c (whole calls: triangles of 180,000 x 320,000 elements 722 -> 596
+// us; blocks of 80,000 x 135,000, k_p1_mass 132 -> 99 us).  p: the thread's column of kTriCap vertices in shared memory.
+template <int B, class Emit>
+__device__ __forceinline__ void clip_tri_fan(const double2 (&a)[3], const Lines& L, double tol, double2* p, bool on,
+                                             const Emit& emit) {
+  const int n = clip_tri_c<B>(a, L, p, on);
+  int kept = 0;
+#pragma unroll 1
+  for (int k = 2; k < n; ++k) {
+    const double2 o = p[0], s = p[(k - 1) * B], t = p[k * B];
+    if (!(tri_area(o.x, o.y, s.x, s.y, t.x, t.y) < tol)) emit(kept++, o.x, o.y, s.x, s.y, t.x, t.y);
+  }
+  if (n < 0) {
+    LocalPoly<kTriWideCap> f, g;
+    double m;
+    clip_tri(a[0].x, a[0].y, a[1].x, a[1].y, a[2].x, a[2].y, L, tol, f, g, kTriWideCap, m, emit);
+  }
+}
+
 // One pair a lane.  Bound by instructions and, next, by shared and L1
 // wavefronts (57 %), both of which divergence multiplies: with the walking
 // clip on 112-byte rows of lines 12 of 32 lanes were active on average and
@@ -3623,19 +3643,19 @@ __global__ void __launch_bounds__(128) k_tris_emit(int64_t npairs, const int32_t
                                                    const double* __restrict__ tol_a, const double* __restrict__ setup_b,
                                                    const int64_t* __restrict__ pair_off, double* elems,
                                                    int64_t* parent_a, int64_t* parent_b) {
+  __shared__ double2 poly[kTriCap * 128];
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < npairs;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t at = pair_off[i];
     if (pair_off[i + 1] == at) continue;
     const int a = pa[i], b = pb[i];
-    const double* ca = coords_a + (int64_t)a * 6;
+    const double2* va = reinterpret_cast<const double2*>(coords_a + (int64_t)a * 6);
+    const double2 v[3] = {__ldg(va), __ldg(va + 1), __ldg(va + 2)};
     Lines L;
     double tolb;
     load_lines(setup_b + (int64_t)b * kSetup2, L, tolb);
     const double tol = fmin(tol_a[a], tolb);
-    LocalPoly<kTriWideCap> p, q;
-    double m;
-    clip_tri(ca[0], ca[1], ca[2], ca[3], ca[4], ca[5], L, tol, p, q, kTriWideCap, m,
+    clip_tri_fan<128>(v, L, tol, poly + threadIdx.x, true,
              [&](int k, double x0, double y0, double x1, double y1, double x2, double y2) {
                double2* e = reinterpret_cast<double2*>(elems + (at + k) * 6);
                e[0] = make_double2(x0, y0);
@@ -4815,7 +4835,7 @@ struct BfP1Sink {
 // 2D: one pair per thread, clipped with the triangle clipper; per supermesh
 // triangle the degree-2 rule (three points), P1 bases of A and B, 3x3 block.
 template <typename IDX>
-__global__ void __launch_bounds__(128) k_p1_mass(int64_t npairs, const int32_t* __restrict__ pa,
+__global__ void __launch_bounds__(128, 4) k_p1_mass(int64_t npairs, const int32_t* __restrict__ pa,
                                                  const int32_t* __restrict__ pb,
                                                  const double* __restrict__ coords_a,
                                                  const double* __restrict__ tol_a,
@@ -4824,6 +4844,7 @@ __global__ void __launch_bounds__(128) k_p1_mass(int64_t npairs, const int32_t* 
                                                  const void* en_b, const double* __restrict__ u_a,
                                                  const double* __restrict__ v_b, double* blocks,
                                                  Partial* partials) {
+  __shared__ double2 poly[kTriCap * 128];
   double sum = 0.0, err = 0.0;
   unsigned long long ni = 0;
   // each iteration loads the next one's pair indices (which stream from
@@ -4852,10 +4873,9 @@ __global__ void __launch_bounds__(128) k_p1_mass(int64_t npairs, const int32_t* 
     load_lines(setup_b + (int64_t)b * kSetup2, L, tolb);
     const double tol = fmin(tol_a[a], tolb);
     const P1Fac2 fa_ = p1_factor_2d(ca), fb_ = p1_factor_2d(coords_b + (int64_t)b * 6);
-    LocalPoly<kTriWideCap> p, q;
-    double m;
+    const double2 v[3] = {{ca[0], ca[1]}, {ca[2], ca[3]}, {ca[4], ca[5]}};
     const double qp0 = 4.0 / 6.0, qp1 = 1.0 / 6.0;
-    clip_tri(ca[0], ca[1], ca[2], ca[3], ca[4], ca[5], L, tol, p, q, kTriWideCap, m,
+    clip_tri_fan<128>(v, L, tol, poly + threadIdx.x, true,
              [&](int, double x0, double y0, double x1, double y1, double x2, double y2) {
                const double meas = tri_area(x0, y0, x1, y1, x2, y2);
                const double w = (1.0 / 3.0) * meas;
@@ -4892,6 +4912,150 @@ __global__ void __launch_bounds__(128) k_p1_mass(int64_t npairs, const int32_t* 
     ++ni;
   }
   block_reduce_partial<128>(sum, err, ni, 0ull, &partials[blockIdx.x]);
+}
+
+// 2D, u^T M v alone: the same sum by triangles, w (u_h v_h) at each point, with
+// full warps.  A pair of candidates has one supermesh triangle on average, 41 %
+// have none and some four, so a lane that integrates its own pair's triangles
+// waits three quarters of the time; here a warp clips 32 pairs (clip_tri_c),
+// queues their triangles and takes 32 at a time from the queue's end.  8.2 M
+// candidate pairs: 1206 us by k_p1_mass with the walking clip, 610 here (160
+// threads at 96 registers; 638 with 192 at 80, 640 with 128 at 120), bound by
+// L1 and shared wavefronts (78 %) and instructions.  Error of the integral
+// against 80-bit arithmetic as before or smaller (at most 2e-16 of the sum of
+// the terms' sizes).
+constexpr int kUvThreads = 160;
+constexpr int kUvQueue = 64;  // fewer than 32 left over, 32 more
+template <typename IDX>
+__device__ __forceinline__ double p1_uv_2d(const double2 (&t)[3], double w, int a, int b,
+                                           const double* __restrict__ coords_a, const double* __restrict__ coords_b,
+                                           const void* en_a, const void* en_b, const double* __restrict__ u_a,
+                                           const double* __restrict__ v_b) {
+  double ca[6], cb[6], u[3], v[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    u[k] = u_a[node_of<IDX>(en_a, a, 3, k)];
+    v[k] = v_b[node_of<IDX>(en_b, b, 3, k)];
+    const double2 x = __ldg(reinterpret_cast<const double2*>(coords_a + (int64_t)a * 6) + k);
+    const double2 y = __ldg(reinterpret_cast<const double2*>(coords_b + (int64_t)b * 6) + k);
+    ca[2 * k] = x.x;
+    ca[2 * k + 1] = x.y;
+    cb[2 * k] = y.x;
+    cb[2 * k + 1] = y.y;
+  }
+  const P1Fac2 fa = p1_factor_2d(ca), fb = p1_factor_2d(cb);
+  const double qp0 = 4.0 / 6.0, qp1 = 1.0 / 6.0;
+  double sv = 0.0;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const double w0 = q == 0 ? qp0 : qp1, w1 = q == 1 ? qp0 : qp1, w2 = q == 2 ? qp0 : qp1;
+    const double x = (w0 * t[0].x + w1 * t[1].x) + w2 * t[2].x;
+    const double y = (w0 * t[0].y + w1 * t[1].y) + w2 * t[2].y;
+    double ga[3], gb[3];
+    p1_apply_2d(fa, x, y, ga);
+    p1_apply_2d(fb, x, y, gb);
+    sv += w * ((u[0] * ga[0] + u[1] * ga[1]) + u[2] * ga[2]) * ((v[0] * gb[0] + v[1] * gb[1]) + v[2] * gb[2]);
+  }
+  return sv;
+}
+
+template <typename IDX>
+__global__ void __launch_bounds__(kUvThreads, 4)
+    k_p1_uv(int64_t npairs, const int32_t* __restrict__ pa, const int32_t* __restrict__ pb,
+            const double* __restrict__ coords_a, const double* __restrict__ tol_a,
+            const double* __restrict__ coords_b, const double* __restrict__ setup_b, const void* en_a,
+            const void* en_b, const double* __restrict__ u_a, const double* __restrict__ v_b, Partial* partials) {
+  __shared__ double2 poly[kTriCap * kUvThreads];
+  __shared__ double2 queue[kUvThreads / 32][4][kUvQueue];  // the vertices; the weight and the pair
+  double2* p = poly + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  auto& qu = queue[threadIdx.x >> 5];
+  int qn = 0;  // the warp's
+  double sum = 0.0, err = 0.0;
+  unsigned long long ni = 0;
+  bool any_wide = false;
+  const auto take = [&](int c) {
+    if (lane < c) {
+      const int e = qn - c + lane;
+      const double2 t[3] = {qu[0][e], qu[1][e], qu[2][e]}, w = qu[3][e];
+      cs_add(sum, err,
+             p1_uv_2d<IDX>(t, w.x, __double2hiint(w.y), __double2loint(w.y), coords_a, coords_b, en_a, en_b, u_a, v_b));
+    }
+    qn -= c;
+    __syncwarp();
+  };
+  // each iteration loads the next one's pair indices (which stream from
+  // DRAM) before it works on its own pair
+  const int64_t stride = (int64_t)gridDim.x * kUvThreads;
+  int64_t i = (int64_t)blockIdx.x * kUvThreads + threadIdx.x;
+  int na = 0, nb = 0;
+  if (i < npairs) {
+    na = pa[i];
+    nb = pb[i];
+  }
+  for (; i - lane < npairs; i += stride) {
+    const int a = na, b = nb;
+    const bool on = i < npairs;
+    if (i + stride < npairs) {
+      na = pa[i + stride];
+      nb = pb[i + stride];
+    }
+    const double2* va = reinterpret_cast<const double2*>(coords_a + (int64_t)a * 6);
+    const double2 v[3] = {__ldg(va), __ldg(va + 1), __ldg(va + 2)};
+    Lines L;
+    double tolb;
+    load_lines(setup_b + (int64_t)b * kSetup2, L, tolb);
+    const double tol = fmin(tol_a[a], tolb);
+    const int n = clip_tri_c<kUvThreads>(v, L, p, on);
+    any_wide |= n < 0;
+    ni += on;
+    __syncwarp();
+#pragma unroll 1
+    for (int k = 2; __any_sync(0xffffffffu, k < n); ++k) {
+      double2 t[3] = {};
+      double ar = 0.0;
+      bool in = k < n;
+      if (in) {
+        t[0] = p[0];
+        t[1] = p[(k - 1) * kUvThreads];
+        t[2] = p[k * kUvThreads];
+        ar = tri_area(t[0].x, t[0].y, t[1].x, t[1].y, t[2].x, t[2].y);
+        in = !(ar < tol);
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      if (in) {
+        const int e = qn + __popc(m & ((1u << lane) - 1u));
+#pragma unroll
+        for (int r = 0; r < 3; ++r) qu[r][e] = t[r];
+        qu[3][e] = make_double2((1.0 / 3.0) * ar, __hiloint2double(a, b));
+      }
+      qn += __popc(m);
+      __syncwarp();
+      if (qn >= 32) take(32);
+    }
+  }
+  take(qn);
+  // pairs that clip_tri_c leaves to clip_tri
+  if (any_wide) {
+    for (i = (int64_t)blockIdx.x * kUvThreads + threadIdx.x; i < npairs; i += stride) {
+      const int a = pa[i], b = pb[i];
+      const double2* va = reinterpret_cast<const double2*>(coords_a + (int64_t)a * 6);
+      const double2 v[3] = {__ldg(va), __ldg(va + 1), __ldg(va + 2)};
+      Lines L;
+      double tolb, m;
+      load_lines(setup_b + (int64_t)b * kSetup2, L, tolb);
+      const double tol = fmin(tol_a[a], tolb);
+      if (clip_tri_c<kUvThreads>(v, L, p, true) >= 0) continue;
+      LocalPoly<kTriWideCap> f, g;
+      clip_tri(v[0].x, v[0].y, v[1].x, v[1].y, v[2].x, v[2].y, L, tol, f, g, kTriWideCap, m,
+               [&](int, double x0, double y0, double x1, double y1, double x2, double y2) {
+                 const double2 t[3] = {{x0, y0}, {x1, y1}, {x2, y2}};
+                 cs_add(sum, err, p1_uv_2d<IDX>(t, (1.0 / 3.0) * tri_area(x0, y0, x1, y1, x2, y2), a, b, coords_a,
+                                                coords_b, en_a, en_b, u_a, v_b));
+               });
+    }
+  }
+  block_reduce_partial<kUvThreads>(sum, err, ni, 0ull, &partials[blockIdx.x]);
 }
 
 // ----------------------------------------------------------------------
@@ -5040,7 +5204,14 @@ cudaError_t launch_p1_mass(int dim, int64_t npairs, const int32_t* pair_a, const
   if (dim == 2) {
     const int g = p1_grid_blocks(2);
     count_launch();
-    if (idx_bytes == 4)
+    if (!blocks && u_a && v_b) {
+      if (idx_bytes == 4)
+        k_p1_uv<int32_t><<<g, kUvThreads, 0, s>>>(npairs, pair_a, pair_b, coords_a, tol_a, coords_b, setup_b, enlist_a,
+                                                  enlist_b, u_a, v_b, partials);
+      else
+        k_p1_uv<int64_t><<<g, kUvThreads, 0, s>>>(npairs, pair_a, pair_b, coords_a, tol_a, coords_b, setup_b, enlist_a,
+                                                  enlist_b, u_a, v_b, partials);
+    } else if (idx_bytes == 4)
       k_p1_mass<int32_t><<<g, 128, 0, s>>>(npairs, pair_a, pair_b, coords_a, tol_a, coords_b, setup_b, enlist_a, enlist_b, u_a, v_b, blocks, partials);
     else
       k_p1_mass<int64_t><<<g, 128, 0, s>>>(npairs, pair_a, pair_b, coords_a, tol_a, coords_b, setup_b, enlist_a, enlist_b, u_a, v_b, blocks, partials);
