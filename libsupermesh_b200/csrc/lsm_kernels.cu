@@ -1825,6 +1825,9 @@ __device__ __forceinline__ int surv_code(int noop, unsigned neg, unsigned irr) {
   return noop | (int)(neg << 4) | (irr >= 2u * (0x7ff00000u - kEpsHi) ? 1 << 30 : 0);
 }
 
+// max(m, |x|) for m >= 0; a NaN x leaves m.
+__device__ __forceinline__ double max_abs(double m, double x) { return fabs(x) > m ? fabs(x) : m; }
+
 template <bool kSettle, int NP, bool kSeg, bool kCode>
 __global__ void __launch_bounds__(256, LSM_PREFILTER_BPS) k_prefilter_tets(int64_t npairs, const int32_t* __restrict__ order,
                                                         const int32_t* __restrict__ pa,
@@ -1880,15 +1883,20 @@ __global__ void __launch_bounds__(256, LSM_PREFILTER_BPS) k_prefilter_tets(int64
       const double* pl = setup_b + (int64_t)b * clip_row(NP);
       double M = 0.0;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) M = fmax(M, fmax(fabs(t.x[k]), fmax(fabs(t.y[k]), fabs(t.z[k]))));
+      for (int k = 0; k < 4; ++k) M = max_abs(max_abs(max_abs(M, t.x[k]), t.y[k]), t.z[k]);
       bool reject = false;
       unsigned neg = 0, irr = 0;  // sign bits of the distances, and the clipper's class test (surv_code)
 #pragma unroll
       for (int L = 0; L < NP; ++L) {
         double nx, ny, nz, c;
         load_plane(pl, L, nx, ny, nz, c);
-        const double thr = kEps + 64.0 * kEps * (1.0 + 2.0 * fmax(M, fabs(c)));
-        double dmin = DBL_MAX, dmax = -DBL_MAX;
+        const double thr = kEps + 64.0 * kEps * (1.0 + 2.0 * max_abs(M, c));
+        // One predicate per distance: the smallest and largest of them, as
+        // doubles, were a third of the pass's instructions.  Without
+        // short-circuits, whose branches cost more (1,000,000 x 800,000 graded tets, 2444 -> 2264 us;
+        // with them 2830).  With an infinite bound nothing is proven; a
+        // distance that is NaN does not count against the others.
+        bool out = thr <= DBL_MAX, in = out;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const double d = ((nx * t.x[k] + ny * t.y[k]) + nz * t.z[k]) - c;
@@ -1897,11 +1905,11 @@ __global__ void __launch_bounds__(256, LSM_PREFILTER_BPS) k_prefilter_tets(int64
             neg = __funnelshift_l(hi, neg, 1);
             irr = max(irr, 2u * hi - 2u * kEpsHi);
           }
-          dmin = fmin(dmin, d);
-          dmax = fmax(dmax, d);
+          out = out & !(d < thr);
+          in = in & !(d > -thr);
         }
-        reject = reject || dmin >= thr;
-        noop |= dmax <= -thr ? 1 << L : 0;
+        reject = reject || out;
+        noop |= in ? 1 << L : 0;
       }
       code = kCode ? surv_code(noop, neg, irr) : noop;
       if (NP == 4 && !reject && faces_a) {
@@ -1917,10 +1925,11 @@ __global__ void __launch_bounds__(256, LSM_PREFILTER_BPS) k_prefilter_tets(int64
 #pragma unroll
           for (int P = 0; P < 4; ++P) {
             const double2 n01 = __ldg(fa + 2 * P), n2h = __ldg(fa + 2 * P + 1);
-            double m = DBL_MAX;
+            const double h = n2h.y + slack;
+            bool out = h <= DBL_MAX;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) m = fmin(m, (n01.x * u.x[k] + n01.y * u.y[k]) + n2h.x * u.z[k]);
-            reject = reject || m >= n2h.y + slack;
+            for (int k = 0; k < 4; ++k) out = out & !((n01.x * u.x[k] + n01.y * u.y[k]) + n2h.x * u.z[k] < h);
+            reject = reject || out;
           }
         }
       }

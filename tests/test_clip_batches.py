@@ -121,3 +121,39 @@ def test_pairs_near_touching_across_a_face_of_a(gpu_ctx, shift):
     v = np.cross(nrm, u)
     b = np.stack([base, base + 0.4 * u, base + 0.4 * v, base + 0.5 * nrm + 0.1 * u], axis=1)
     _same(gpu_ctx.intersect_pairs(3, a + shift, b + shift, want_elems=True), _small(gpu_ctx, a + shift, b + shift))
+
+
+def _soup(kind, n):
+    """Two meshes of n tets of their own nodes."""
+    rng = np.random.default_rng(n)
+    a, b = (rng.random((n, 1, 3)) + 0.35 * rng.random((n, 4, 3)) for _ in range(2))
+    if kind == "lattice":  # vertices on planes, shared and parallel faces
+        a, b = np.round(a * 16) / 16, np.round(b * 16) / 16
+    elif kind == "inside":
+        a[::2] = b[::2].mean(1, keepdims=True) + 1e-3 * (a[::2] - a[::2, :1])
+    elif kind == "degenerate":
+        a[::3, 2], b[::5, 1] = a[::3, 1], b[::5, 0]
+    elif kind == "large":  # bounds that overflow
+        a[::3] *= 1e200
+        b[::4] *= 1e200
+    elif kind == "infinite":
+        a[::4, 1, 0] = np.inf
+        a[1::4, 1:, 2] = -np.inf
+        b[1::3, :, 0] = [np.inf, 0, 1, -np.inf]
+    en = np.arange(4 * n, dtype=np.int32).reshape(n, 4)
+    return (a.reshape(-1, 3), en), (b.reshape(-1, 3), en)
+
+
+@pytest.mark.parametrize("kind", ["plain", "lattice", "inside", "degenerate", "large", "infinite"])
+@pytest.mark.parametrize("n", [33, 400])
+def test_mesh_early_outs_match_one_launch_clipper(gpu_ctx, kind, n):
+    """What the early-out pass rejects or settles, against clipping every
+    candidate."""
+    A, B = _soup(kind, n)
+    cand = gpu_ctx.find_candidates(A, B)
+    gpu_ctx.clip_candidates()
+    ip, ind = gpu_ctx.get_candidates(n, cand)
+    m, k = gpu_ctx.pair_results(cand)
+    rm, rk, _ = _small(gpu_ctx, A[0][A[1]][np.repeat(np.arange(n), np.diff(ip))], B[0][B[1]][ind])
+    assert np.array_equal(k, rk)
+    assert np.array_equal(m, rm, equal_nan=True)
