@@ -1,7 +1,7 @@
 """Benchmark of the supermesh hot path: clipped element pairs per second.
 
 One step = one pass of the hot path over one pair of meshes: candidate
-search (LBVH build + traversal), intersection of every candidate pair, and
+search (box hierarchy build + traversal), intersection of every candidate pair, and
 the compensated measure reduction, through libsupermesh_gpu_supermesh.
 
 Workload (default): 3D graded supermesh, target 55^3 x 6 = 998,250 Kuhn tets

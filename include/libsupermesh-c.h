@@ -57,7 +57,7 @@ void libsupermesh_sort_intersection_finder_query_output(long *nindices);
 void libsupermesh_sort_intersection_finder_get_output(long *nelements, long *nindices, long *indices, long *ind_ptr);
 
 /* Tree finder (C_bindings.F90:346-391): 2D quadtree / 3D octree candidate
- * set, computed on the GPU by an LBVH with the same strict box test. */
+ * set, computed on the GPU by a box hierarchy with the same strict box test. */
 void libsupermesh_tree_intersection_finder_set_input(long *nnodes_a, int *dim_a, long *nelements_a, int *loc_a,
                                                      long *nnodes_b, int *dim_b, long *nelements_b, int *loc_b,
                                                      c_kind *positions_a, long *enlist_a, c_kind *positions_b,

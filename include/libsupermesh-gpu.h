@@ -142,7 +142,7 @@ int libsupermesh_gpu_find_candidates(lsm_gpu_context *ctx, const lsm_gpu_mesh *a
 
 /* Copy the last candidate CSR out: ind_ptr[nelements_a + 1] (0-based, starts
  * at 0) and indices[n_candidates] (0-based B elements; within a row in
- * LBVH traversal order).  on_device selects the destination memory. */
+ * Morton order of their boxes).  on_device selects the destination memory. */
 int libsupermesh_gpu_get_candidates(lsm_gpu_context *ctx, int64_t *ind_ptr,
                                     int64_t *indices, int on_device, void *stream);
 
@@ -236,9 +236,9 @@ int libsupermesh_gpu_get_pair_results(lsm_gpu_context *ctx, double *measure,
  * [n][4][3].  measure[n] = sum of output simplex measures, n_out[n] = number
  * of output simplices; elems (optional) [n][22][3][2] or [n][81][4][3] in
  * the reference's output order (slots past a pair's n_out are left
- * unspecified).  Tet batches of 2048 pairs or more run through per-pair
- * setup, the exact early-out pass and the index clipper; smaller ones through
- * a one-launch clipper (same results).  With on_device = 1 and dim = 3, a, b
+ * unspecified).  Tet batches of 2048 pairs or more run through a pass of
+ * per-pair setup and exact early-outs and a batched clipper; smaller ones
+ * through a one-launch clipper (same results).  With on_device = 1 and dim = 3, a, b
  * and elems must be 16-byte aligned (tetrahedra are read and written with
  * 16-byte accesses); other pointers return LSM_ERROR_INVALID_ARGUMENT before
  * any launch. */

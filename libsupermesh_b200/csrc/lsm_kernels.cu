@@ -2,18 +2,19 @@
 //
 //   K1  k_prep          element gather, FP64/FP32 boxes, measures, tolerances,
 //                       B-element clip setup (lines / unit-normal planes)
-//   K1b k_root_*        root box reduction;  k_morton  Morton keys
-//   K2  radix sort      stable LSD, 8-bit digits, warp-match ranking;
-//                       one digit-count kernel, then one kernel per pass
-//                       with decoupled look-back (k_radix_onesweep)
+//   K1b k_root_box      root box;  k_morton  Morton keys and the sort's
+//                       digit counts
+//   K2  radix sort      stable LSD, 8-bit digits, warp-match ranking; one
+//                       kernel per pass with decoupled look-back
+//                       (k_radix_onesweep)
 //   K3  k_tree_build    four-wide hierarchy of outward-rounded FP32 boxes
 //                       over the sorted leaves
 //   K4  k_query         depth-first traversal per A element, four children a
 //                       visit (k_query_warp: a warp per element, 32), exact
 //                       strict box test at the leaves; the count pass caches
 //                       rows, k_fill_from_cache copies
-//   K5  k_clip_tris     one candidate pair per thread, polygon in shared
-//                       memory, FP64 Sutherland-Hodgman
+//   K5  k_clip_tris     one candidate pair per thread, polygon clipped in
+//                       place in shared memory, FP64 Sutherland-Hodgman
 //   K6  k_prefilter_tets two exact early-outs and the no-op plane mask;
 //                       k_clip_tets_bf breadth-first clipping, a warp per
 //                       batch of pairs, templated on what it does with the
@@ -25,15 +26,16 @@
 //                       of large passes; six planes: hexahedra)
 //   K7  compensated reductions (per-block (sum, err), then final; per mesh
 //                       pair for the batched path)
-//   K8  P1-P1 mixed mass blocks + u^T M v: 2D k_p1_mass; 3D the early-out
-//                       pass and k_clip_tets_bf with the quadrature sink;
+//   K8  P1-P1 mixed mass blocks + u^T M v: 2D k_p1_mass (blocks), k_p1_uv
+//                       (u^T M v alone); 3D the early-out pass and
+//                       k_clip_tets_bf with the quadrature sink;
 //                       k_p2_inner  P2 inner product
 //   K9  1D sort finder  k_prep_1d, 64-bit stable sort, max segment tree,
 //                       k_rows_1d, k_sweep_1d, k_emit_1d;  k_clip_intervals
 //   K10 explicit pairs  k_pairs_tris / _tets and the mixed element pairs
 //                       (intervals, tri-quad, quad-quad, tet-hex, hex-hex);
-//                       large tet-tet / tet-hex batches: k_setup_pairs3 /
-//                       k_setup_hex_pairs, then K6
+//                       large tet-tet batches: k_pairs_early (setup and
+//                       early-outs), tet-hex: k_setup_hex_pairs, then K6
 //   K13 supermesh elements  K6's emit pass (3D), k_tris_emit (2D)
 //
 // Everything FP64 is compiled with -fmad=false so that each +,-,*,/ is a
@@ -1548,10 +1550,10 @@ __device__ __forceinline__ void clip_tri_fan(const double2 (&a)[3], const Lines&
   }
 }
 
-// One pair a lane.  Bound by instructions and, next, by shared and L1
-// wavefronts (57 %), both of which divergence multiplies: with the walking
+// One pair a lane.  Bound by instructions (issue 64 %) and L1 and shared
+// wavefronts (69 %), both of which divergence multiplies: with the walking
 // clip on 112-byte rows of lines 12 of 32 lanes were active on average and
-// 13.8 M pairs took 1190 us; clip_tri_c alone would have given 1108 (in two
+// 14.9 M pairs took 1190 us; clip_tri_c alone would have given 1108 (in two
 // buffers), in place and with 64-byte rows 630.  Eight blocks an SM, all
 // resident: 96 threads at 80 registers 629 us, 128 at 64 646, 64 at 104 642.
 __global__ void __launch_bounds__(kTriBlock, 8) k_clip_tris(int64_t npairs, const int32_t* __restrict__ pa,
@@ -2722,8 +2724,8 @@ __device__ __forceinline__ void clip_nonfinite(const Pool& pool, const double* p
 // when the point is created; a list entry carries its four vertices' bytes,
 // and the same byte permute that makes a child's vertex indices out of the old
 // tet's and the new points' makes its classes.
-// Measured (tet3d_27x32 unless said): P1 mass 12.8 -> 5.9 ms; supermesh elements 4.47 ->
-// 4.04 ms; measures of 330 thousand candidates (10^3 x 6 against 12^3 x 6
+// Measured (tet3d_27x32 unless said): P1 mass 12.8 -> 5.9 ms; the emitting pass of the
+// supermesh's elements 1.86 -> 1.53 ms; measures of 330 thousand candidates (10^3 x 6 against 12^3 x 6
 // tets), early-out pass included, 0.212 -> 0.136 ms.  On the large measure
 // passes k_clip_tets_ix is ahead (1.18 against 1.34 ms; as many instructions go
 // into the lists and rounds as into the idle lanes of the other).
@@ -4927,10 +4929,10 @@ __global__ void __launch_bounds__(128, 4) k_p1_mass(int64_t npairs, const int32_
 // full warps.  A pair of candidates has one supermesh triangle on average, 41 %
 // have none and some four, so a lane that integrates its own pair's triangles
 // waits three quarters of the time; here a warp clips 32 pairs (clip_tri_c),
-// queues their triangles and takes 32 at a time from the queue's end.  8.2 M
+// queues their triangles and takes 32 at a time from the queue's end.  9.5 M
 // candidate pairs: 1206 us by k_p1_mass with the walking clip, 610 here (160
 // threads at 96 registers; 638 with 192 at 80, 640 with 128 at 120), bound by
-// L1 and shared wavefronts (78 %) and instructions.  Error of the integral
+// L1 and shared wavefronts (72 %) and instructions.  Error of the integral
 // against 80-bit arithmetic as before or smaller (at most 2e-16 of the sum of
 // the terms' sizes).
 constexpr int kUvThreads = 160;
