@@ -1209,14 +1209,16 @@ __global__ void __launch_bounds__(256) k_query_warp(int64_t nel_a, const double*
 }
 
 // Fill of the rows whose candidates the count pass cached: each warp copies
-// rpw rows one after the other, lanes striding over the row (coalesced
-// reads of the cache and writes of the pair arrays).
+// rpw rows, 32 / G at a time, G lanes striding over a row (coalesced reads of
+// the cache and writes of the pair arrays).  2D rows hold a dozen candidates,
+// which left most of 32 lanes idle and one row's reads in flight.
+template <int G>
 __global__ void __launch_bounds__(256) k_fill_from_cache(int64_t nel_a, const int* __restrict__ counts,
                                                          const int64_t* __restrict__ offsets,
                                                          const int32_t* __restrict__ cache, int cap,
                                                          int32_t* pair_a, int32_t* pair_b, Spill sp,
                                                          int64_t pair_cap, int rpw) {
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, sub = lane / G, l = lane % G;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * rpw; base < nel_a;
        base += warps * rpw) {
@@ -1227,7 +1229,9 @@ __global__ void __launch_bounds__(256) k_fill_from_cache(int64_t nel_a, const in
       cnt = counts[a];
       off = offsets[a];
     }
-    for (int r = 0; r < rpw; ++r) {
+    for (int r0 = 0; r0 < rpw; r0 += 32 / G) {
+      const int r = (r0 + sub) & 31;
+      // (lanes from rpw on hold empty rows)
       const int c = __shfl_sync(0xffffffffu, cnt, r);
       const int64_t o = __shfl_sync(0xffffffffu, off, r);
       const int64_t row = base + r;
@@ -1241,13 +1245,13 @@ __global__ void __launch_bounds__(256) k_fill_from_cache(int64_t nel_a, const in
         const int first = sp.row_chunk ? sp.row_chunk[row] : -2;
         if (first < 0) continue;
         const int head = lim < cap ? lim : cap;
-        for (int k = lane; k < head; k += 32) {
+        for (int k = l; k < head; k += G) {
           pair_a[o + k] = (int32_t)row;
           pair_b[o + k] = cache[row * cap + k];
         }
         int ch = first;
         for (int k0 = cap; k0 < c; k0 += kSpillChunk) {
-          for (int k = lane; k < kSpillChunk && k0 + k < lim; k += 32) {
+          for (int k = l; k < kSpillChunk && k0 + k < lim; k += G) {
             pair_a[o + k0 + k] = (int32_t)row;
             pair_b[o + k0 + k] = sp.pool[(int64_t)ch * kSpillChunk + k];
           }
@@ -1255,7 +1259,7 @@ __global__ void __launch_bounds__(256) k_fill_from_cache(int64_t nel_a, const in
         }
         continue;
       }
-      for (int k = lane; k < lim; k += 32) {
+      for (int k = l; k < lim; k += G) {
         pair_a[o + k] = (int32_t)row;
         pair_b[o + k] = cache[row * cap + k];
       }
@@ -1268,6 +1272,9 @@ __global__ void __launch_bounds__(256) k_fill_from_cache(int64_t nel_a, const in
 // 45,000 rows 168 / 186 us; 3D 6,000 rows 288 / 162 us, 48,000 rows 369 / 338
 // us, 118,098 rows 401 / 465 us.
 constexpr int64_t kWarpRows2 = 24 << 10, kWarpRows3 = 64 << 10;
+// Lanes per row of the fill (2D 4 / 8 / 16 / 32: whole call 1513 / 1494 / 1503 /
+// 1543 us, 14.9 M candidates; 3D 8 / 16 / 32: 9819 / 9740 / 9723 us, 56 M).
+constexpr int kFill2 = 8, kFill3 = 32;
 
 // Threads per block of the search: the option's, or a warp where that leaves
 // SMs without a block (the row's serial walk is then the time).
@@ -1288,8 +1295,9 @@ static cudaError_t run_query(int dim, bool fill, int64_t nel_a, const double* bo
     // 32 rows per warp, fewer while that leaves warps to spare
     int rpw = 32;
     while (rpw > 1 && nel_a < (int64_t)sm_count() * 32 * rpw) rpw >>= 1;
-    k_fill_from_cache<<<grid_for((nel_a + rpw - 1) / rpw * 32, 256, 8), 256, 0, s>>>(
-        nel_a, counts, offsets, cache, cap, pair_a, pair_b, sp, pair_cap, rpw);
+    (dim == 2 ? k_fill_from_cache<kFill2> : k_fill_from_cache<kFill3>)
+        <<<grid_for((nel_a + rpw - 1) / rpw * 32, 256, 8), 256, 0, s>>>(nel_a, counts, offsets, cache, cap, pair_a,
+                                                                       pair_b, sp, pair_cap, rpw);
   } else {
     count_launch();
   }

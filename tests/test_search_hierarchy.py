@@ -94,3 +94,22 @@ def test_sort_look_back_edges(gpu_ctx, dim, nb):
     pos, en = _elements(dim, nb, rng, 0.05)
     pos[: (dim + 1) * (nb // 3)] = np.tile(pos[: dim + 1], (nb // 3, 1))
     _check(gpu_ctx, _elements(dim, 60, rng, 0.1), (pos, en))
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_fill_row_lengths(gpu_ctx, dim):
+    """Rows of 0 to 300 candidates side by side, in the order of the target's
+    elements along a line: edges of the lanes that copy a row and of the row
+    cache."""
+    nb = 300
+    lens = np.array([0, 1, 7, 8, 9, 15, 16, 17, 31, 32, 33, 64, 65, 255, 256, 257, 300, 3, 0, 12] * 4 + [5])
+    e = np.vstack([np.zeros((1, dim)), np.eye(dim)])
+    b = e[None] * 0.5
+    b = np.repeat(b, nb, 0)
+    b[:, :, 0] += np.arange(nb)[:, None]
+    a = np.repeat(e[None], len(lens), 0)
+    a[:, :, 0] = a[:, :, 0] * np.maximum(lens - 0.25, 0.25)[:, None] - np.where(lens > 0, 0.0, 1.0)[:, None]
+    A = (a.reshape(-1, dim), np.arange(len(lens) * (dim + 1), dtype=np.int32).reshape(-1, dim + 1))
+    B = (b.reshape(-1, dim), np.arange(nb * (dim + 1), dtype=np.int32).reshape(-1, dim + 1))
+    ip, _ = _check(gpu_ctx, A, B)
+    assert np.array_equal(np.diff(ip), lens)
