@@ -3036,6 +3036,7 @@ __global__ void __launch_bounds__(Sink::kWarps * 32, 1) k_clip_tets_bf(
             if (on && (lane == 31 || f + 1 == nf || after != slot)) s_run[slot] = k + keep;
             __syncwarp();
           }
+          // (-1: dropped; a kept tet's volume may be NaN, where its products overflow)
           if (on && (Sink::kSum || Sink::kP1)) vol[f] = keep ? v1 : -1.0;
         }
         __syncwarp();
@@ -3049,7 +3050,7 @@ __global__ void __launch_bounds__(Sink::kWarps * 32, 1) k_clip_tets_bf(
             for (int i = 0; i < 4; ++i) v1[i] = f + i < fe ? vol[f + i] : -1.0;
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-              if (__double2hiint(v1[i]) >= 0) {
+              if (!(v1[i] < 0.0)) {
                 m = m + v1[i];
                 ++kept;
               }
@@ -4736,7 +4737,7 @@ struct BfP1Sink {
         v1 = vol[f0 + t];
       }
       const unsigned slot = id.y >> 27;
-      if (v1 >= 0.0) {
+      if (!(v1 < 0.0)) {
         Tet o;
         bf_tet(pool, id.x, id.y & 0x03030303u, o);
         const double* fac = reinterpret_cast<const double*>(mem + kFac) + slot;

@@ -5,6 +5,7 @@ Both sides run the same operations in the same order, so every comparison is
 exact."""
 import numpy as np
 import pytest
+import torch
 
 import libsupermesh_b200 as lsm
 from libsupermesh_b200 import meshes as M
@@ -81,6 +82,42 @@ def test_p1_blocks_match_oracle(gpu_ctx, oracle_mod, na, nb, ja, jb, scale):
     ip, ind = gpu_ctx.get_candidates(len(A[1]), len(blocks))
     _, _, ref = oracle_mod.p1_mass(3, A, B, ip, ind, u, v, want_blocks=True)
     assert np.array_equal(blocks, ref.reshape(blocks.shape))
+
+
+@pytest.mark.parametrize("exponent", [343, 344, 345, 348, 400, 500])
+def test_volumes_that_overflow(gpu_ctx, exponent):
+    """Coordinates whose volumes' products overflow: a kept tet of NaN volume
+    counts (in either clipper; the binned order takes the depth-first one) and
+    makes its pair's measure and every entry of its mass block NaN; the
+    elements' two passes agree on the count."""
+    A, B = M.grid3d(4, 3, 0.2), M.grid3d(5, 2, 0.2)
+    A, B = (A[0] * 2.0 ** exponent, A[1]), (B[0] * 2.0 ** exponent, B[1])
+    cand = gpu_ctx.find_candidates(A, B)
+    gpu_ctx.clip_candidates()
+    m, k = gpu_ctx.pair_results(cand)
+    lsm.set_option("tet_schedule", 2)
+    try:
+        gpu_ctx.clip_candidates()
+        rm, rk = gpu_ctx.pair_results(cand)
+    finally:
+        lsm.set_option("tet_schedule", 0)
+    assert np.array_equal(k, rk)
+    assert np.array_equal(m, rm, equal_nan=True)
+    _, blocks = gpu_ctx.p1_mass(A, B, want_blocks=True)
+    assert np.isnan(m).any() == (exponent > 343)
+    assert np.isnan(blocks[np.isnan(m)]).all()
+    # the emitting pass, into arrays of one element more than the count
+    _, off, _, pa, _ = gpu_ctx.supermesh_elements(A, B)
+    assert np.array_equal(np.diff(off), k)
+    n, dev = int(off[-1]), {"device": "cuda"}
+    out = {"cand_capacity": cand, "elem_capacity": n + 1, "elem_offset": torch.zeros(cand + 1, dtype=torch.int64, **dev),
+           "elems": torch.full((n + 1, 4, 3), 7.0, dtype=torch.float64, **dev),
+           "parent_a": torch.full((n + 1,), -7, dtype=torch.int64, **dev),
+           "parent_b": torch.full((n + 1,), -7, dtype=torch.int64, **dev)}
+    gpu_ctx.supermesh_elements_device(*(tuple(torch.from_numpy(x).cuda() for x in m_) for m_ in (A, B)), out)
+    torch.cuda.synchronize()
+    assert np.array_equal(out["parent_a"][:n].cpu().numpy(), pa)
+    assert (out["elems"][n] == 7.0).all() and out["parent_a"][n] == -7 and out["parent_b"][n] == -7
 
 
 @pytest.mark.parametrize("value", [None, np.nan, np.inf, 1e200])
