@@ -76,10 +76,14 @@ int64_t libsupermesh_gpu_kernel_launches(void);
 /* Process-wide tuning options.  They change launch shapes and work order,
  * never results (the autotuner in libsupermesh_b200/autotune.py picks the
  * launch shapes per GPU and workload):
- *   "tri_blocks_per_sm"  4, 8 (default) or 16 blocks of 128 threads per SM (2D clipper)
- *   "query_block"        64, 128 (default) or 256 threads per block (candidate search)
- *   "leaf_bucket"        1 (default), 2, 4 or 8: accepted and returned; the search hierarchy scans
- *                        four leaves at a time whatever its value
+ *   "tri_blocks_per_sm"  4, 8 (default) or 16 blocks of 96 threads per SM (2D clipper); 8 are
+ *                        resident at once
+ *   "query_block"        64, 128 (default) or 256 threads per block (candidate search with a
+ *                        thread per row, where that gives every SM four blocks and more).  The
+ *                        count pass of a single mesh pair takes a warp per row below 24,576 (2D)
+ *                        or 65,536 (3D) rows, in blocks of 256 threads whatever the option says
+ *   "leaf_bucket"        1 (default), 2, 4 or 8: accepted and returned, without effect (the search
+ *                        hierarchy scans four leaves at a time)
  *   "time_kernels"       1: record CUDA events around the clip kernel of every
  *                        narrow phase (read with libsupermesh_gpu_clip_kernel_ms); 0 (default)
  *   "spill_chunks"       -1 (default, automatic), 0 or n > 0: chunks of 64 candidates that the

@@ -56,3 +56,33 @@ def test_store_round_trip(tuner):
     autotune._store(db)
     assert autotune._load() == db
     assert not autotune.cache_path().with_suffix(".tmp").exists()
+
+
+@pytest.mark.parametrize("dim,runs", [(2, 9), (3, 3)])
+def test_settings_that_run_the_same_are_timed_once(tuner, dim, runs):
+    """An option that no kernel reads is neither swept nor chosen by noise."""
+    autotune, _ = tuner
+    seen = []
+
+    def measure(setting):
+        seen.append(tuple(v for n, v in setting.items() if n != "leaf_bucket"))
+        return 10.0 - len(seen), "same"  # the last timed is the fastest
+
+    res = autotune._search(dim, measure)
+    assert len(seen) == len(set(seen)) == runs
+    assert len(res) == 3 * runs
+    assert res[0][1]["leaf_bucket"] == 1
+    assert tuple(v for n, v in res[0][1].items() if n != "leaf_bucket") == seen[-1]
+
+
+@pytest.mark.parametrize("gain,chosen", [(0.03, 128), (0.1, 256)])
+def test_the_default_stays_within_the_noise(tuner, gain, chosen):
+    autotune, _ = tuner
+    res = autotune._search(3, lambda s: (1.0 - gain if s["query_block"] == 256 else 1.0, 0))
+    assert res[0][1] == {"query_block": chosen, "leaf_bucket": 1}
+
+
+def test_a_setting_that_changes_results_is_an_error(tuner):
+    autotune, _ = tuner
+    with pytest.raises(RuntimeError):
+        autotune._search(3, lambda s: (1.0, s["query_block"]))
