@@ -57,14 +57,16 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
 
 def build_probe(force: bool = False) -> Path:
-    """Measurement probe used by bench.py (FP64 issue-rate ceiling, L2 flush)."""
+    """Measurement probe used by bench.py (FP64 issue-rate ceiling, L2 flush)
+    and by the tests (quotients and normals on given operands)."""
     src = SRC / "lsm_probe.cu"
-    if not force and PROBE.exists() and PROBE.stat().st_mtime >= src.stat().st_mtime:
+    if not force and PROBE.exists() and all(
+            PROBE.stat().st_mtime >= f.stat().st_mtime for f in (src, SRC / "lsm_geom.cuh", Path(__file__))):
         return PROBE
     PROBE.parent.mkdir(parents=True, exist_ok=True)
     tmp = PROBE.with_suffix(".so.tmp")
-    subprocess.run([nvcc(), *ARCH, "-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "--cudart", "static",
-                    str(src), "-o", str(tmp)], check=True)
+    subprocess.run([nvcc(), *ARCH, "-O3", "-std=c++17", "-fmad=false", "-shared", "-Xcompiler", "-fPIC", "--cudart",
+                    "static", str(src), "-o", str(tmp)], check=True)
     os.replace(tmp, PROBE)
     return PROBE
 

@@ -60,8 +60,8 @@ __device__ __forceinline__ double norm2_3(double a, double b, double c) {
 // second gives the quotient.  Holds while nothing underflows or overflows:
 // div_range keeps the largest 2 * (high word of |v|) - 2 * high(2^-400), modulo
 // 2^32, of the operands; div_ok(max) is false as soon as one lies outside
-// [2^-400, 2^400] (zero, infinity and NaN included), and the caller then
-// divides.
+// [2^-400, 2^400 (1 + 2^-20)) (zero, infinity and NaN included), and the caller
+// then divides.
 __device__ __forceinline__ double div_by(double a, double b, double y) {
   double q = a * y;
   q = __fma_rn(__fma_rn(-b, q, a), y, q);

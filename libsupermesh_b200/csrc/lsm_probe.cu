@@ -2,10 +2,15 @@
 // ceiling that the clipping kernels run against.  The clipper is compiled
 // without FMA contraction, so its ceiling is the issue rate of separate
 // DADD/DMUL instructions; the probe measures that rate (and, for context,
-// the DFMA rate) with long chains of independent operations.
+// the DFMA rate) with long chains of independent operations.  And the
+// clippers' quotients and normals on given operands, for comparison with
+// divisions (built, like the library, without FMA contraction).
 #include <cuda_runtime.h>
 
+#include <cfloat>
 #include <cstdint>
+
+#include "lsm_geom.cuh"
 
 namespace {
 
@@ -45,9 +50,41 @@ __global__ void __launch_bounds__(256) k_dfma(double seed, double* sink) {
   if (s == 12345.678) sink[0] = s;
 }
 
+__global__ void __launch_bounds__(256) k_quotients(int64_t n, const double* __restrict__ a,
+                                                   const double* __restrict__ b, double* divided, double* by, int* ok) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const unsigned range = lsm::div_range(lsm::div_range(0, a[i]), b[i]);
+  divided[i] = a[i] / b[i];
+  by[i] = lsm::div_by(a[i], b[i], __drcp_rn(b[i]));
+  ok[i] = lsm::div_ok(range);
+}
+
+__global__ void __launch_bounds__(256) k_normals(int64_t n, const double* __restrict__ uv, double* out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double* v = uv + 6 * i;
+  double* o = out + 4 * i;
+  lsm::unit_cross(v[0], v[1], v[2], v[3], v[4], v[5], o[0], o[1], o[2]);
+  o[3] = lsm::norm2_3(v[0], v[1], v[2]);
+}
+
 }  // namespace
 
 extern "C" {
+
+// a[n] / b[n] by division and by the reciprocal of b (div_by), and whether
+// the range check lets the second stand for the first; device arrays.
+int lsm_probe_quotients(int64_t n, const double* a, const double* b, double* divided, double* by, int* ok) {
+  if (n > 0) k_quotients<<<(unsigned)((n + 255) / 256), 256>>>(n, a, b, divided, by, ok);
+  return (int)cudaDeviceSynchronize();
+}
+
+// uv[n][6] -> out[n][4]: the unit normal of u x v and the length of u.
+int lsm_probe_normals(int64_t n, const double* uv, double* out) {
+  if (n > 0) k_normals<<<(unsigned)((n + 255) / 256), 256>>>(n, uv, out);
+  return (int)cudaDeviceSynchronize();
+}
 
 // Returns FP64 operations per second: mode 0 = separate DADD+DMUL (1 op
 // each), mode 1 = DFMA (2 ops each).  Timed with CUDA events, best of
