@@ -285,7 +285,9 @@ int libsupermesh_gpu_intersect_pairs_mixed(lsm_gpu_context *ctx, int kind, int64
  * the local block M[i][j] = sum_c |c| sum_q w_q phi_i^A(x_q) phi_j^B(x_q)
  * (blocks, optional, [n_candidates][loc][loc], device memory only when
  * on_device), and integral = u_a^T M v_b (u_a [nnodes_a], v_b [nnodes_b],
- * optional).  Quadrature as test_parallel_p1_inner_product_{2d,3d}.F90. */
+ * optional).  Quadrature as test_parallel_p1_inner_product_{2d,3d}.F90.  In 2D
+ * the integral without blocks is summed by supermesh triangles, with blocks by
+ * candidate pairs: the two differ by rounding. */
 int libsupermesh_gpu_p1_mass(lsm_gpu_context *ctx, const lsm_gpu_mesh *a,
                              const lsm_gpu_mesh *b, const double *u_a,
                              const double *v_b, double *blocks, double *integral,

@@ -2467,7 +2467,7 @@ __global__ void __launch_bounds__(BLOCK, BPS) k_clip_tets_ix(
     const int4* __restrict__ chunks = nullptr) {
   // chunks (optional): the list is segmented; nlist then counts the table's
   // chunks and work counts the chunks taken
-  static_assert(ix_points(NP) <= 32, "pool indices are 5 bits");
+  static_assert(ix_points(NP) <= 32, "the last point byte leaves three bits for the plane");
   extern __shared__ double ix_mem[];
   uint2* table = reinterpret_cast<uint2*>(ix_mem);
   for (int i = threadIdx.x; i < 256; i += BLOCK) table[i] = g_clip_table.e[i];
@@ -4946,8 +4946,9 @@ __global__ void __launch_bounds__(128, 4) k_p1_mass(int64_t npairs, const int32_
 // have none and some four, so a lane that integrates its own pair's triangles
 // waits three quarters of the time; here a warp clips 32 pairs (clip_tri_c),
 // queues their triangles and takes 32 at a time from the queue's end.  9.5 M
-// candidate pairs: 1206 us by k_p1_mass with the walking clip, 610 here (160
-// threads at 96 registers; 638 with 192 at 80, 640 with 128 at 120), bound by
+// candidate pairs: 1206 us by k_p1_mass with the walking clip, 617 here
+// (threads and registers, without a profiler: 160 at 96 610 us, 192 at 80 638,
+// 128 at 120 640), bound by
 // L1 and shared wavefronts (72 %) and instructions.  Error of the integral
 // against 80-bit arithmetic as before or smaller (at most 2e-16 of the sum of
 // the terms' sizes).
