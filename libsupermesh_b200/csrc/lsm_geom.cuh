@@ -176,7 +176,8 @@ __device__ __forceinline__ void poly_lines(const double* v, double* nx, double* 
 // v1.  bnd = 64u L^3 (+ an absolute term for subnormal results) bounds it
 // with room to spare: if v1 clears tol by bnd the outcome of v4 >= tol is
 // known; otherwise v4 is computed and compared as the reference does.
-// Overflow or NaN make both quick comparisons false and take the exact path.
+// Overflow or NaN make both quick comparisons false and take the exact path
+// (v1 - bnd, not tol + bnd: with both infinite the difference is NaN).
 __device__ __forceinline__ bool final_tet_keep(const Tet& t, double tol, double& v1) {
   const double e1x = t.x[1] - t.x[0], e1y = t.y[1] - t.y[0], e1z = t.z[1] - t.z[0];
   const double e2x = t.x[2] - t.x[0], e2y = t.y[2] - t.y[0], e2z = t.z[2] - t.z[0];
@@ -189,7 +190,7 @@ __device__ __forceinline__ bool final_tet_keep(const Tet& t, double tol, double&
   const double l3 = (fabs(e3x) + fabs(e3y)) + fabs(e3z);
   const double L = fmax(l1, fmax(l2, l3));
   const double bnd = 0x1p-47 * (L * L * L) + 0x1p-1016;
-  if (v1 >= tol + bnd) return true;
+  if (v1 - bnd >= tol) return true;
   if (v1 < tol - bnd) return false;
   return tet_volume_v4(t) >= tol;
 }

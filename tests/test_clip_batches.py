@@ -120,6 +120,22 @@ def test_volumes_that_overflow(gpu_ctx, exponent):
     assert (out["elems"][n] == 7.0).all() and out["parent_a"][n] == -7 and out["parent_b"][n] == -7
 
 
+@pytest.mark.parametrize("exponent", [342, 343, 344, 345, 348, 352, 400, 500])
+def test_volumes_that_overflow_against_one_launch(gpu_ctx, exponent):
+    """The keep test's shortcut (vertex-1 volume) where it and its bound are
+    infinite: the vertex-4 volume decides, as in the one-launch clipper."""
+    A, B = M.grid3d(4, 3, 0.2), M.grid3d(5, 2, 0.2)
+    A, B = (A[0] * 2.0 ** exponent, A[1]), (B[0] * 2.0 ** exponent, B[1])
+    cand = gpu_ctx.find_candidates(A, B)
+    gpu_ctx.clip_candidates()
+    ip, ind = gpu_ctx.get_candidates(len(A[1]), cand)
+    m, k = gpu_ctx.pair_results(cand)
+    ra = np.repeat(np.arange(len(A[1])), np.diff(ip))
+    rm, rk, _ = _small(gpu_ctx, A[0][A[1]][ra], B[0][B[1]][ind])
+    assert np.array_equal(k, rk)
+    assert np.array_equal(m, rm, equal_nan=True)
+
+
 @pytest.mark.parametrize("value", [None, np.nan, np.inf, 1e200])
 def test_tet_hexahedron_batches(gpu_ctx, value):
     """The depth-first clipper's split table, six planes: batches of 2048 and
