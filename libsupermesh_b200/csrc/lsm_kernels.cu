@@ -3280,7 +3280,8 @@ __global__ void k_setup_pairs3(int64_t n, const double* __restrict__ tet_a, cons
 // passes wrote 428 bytes of setup per pair and read them back: 1,048,576
 // pairs, of which a third survive, 0.32 -> 0.15 ms.  A's faces enter the second
 // test as they come from the cross product: a direction need not be of unit
-// length there, only the margins scaled (kept clear of underflow).
+// length there, only the margins scaled (kept clear of underflow and, as the
+// cross product is of the coordinates' square, of overflow).
 __global__ void __launch_bounds__(256, 2) k_pairs_early(int64_t n, const double* __restrict__ tet_a,
                                                         const double* __restrict__ tet_b, double* setup,
                                                         double* tol_a, double* measure, int32_t* nout, int4* survivors,
@@ -3351,9 +3352,9 @@ __global__ void __launch_bounds__(256, 2) k_pairs_early(int64_t n, const double*
               h = fmax(h, (nx * t.x[k] + ny * t.y[k]) + nz * t.z[k]);
               m = fmin(m, (nx * u.x[k] + ny * u.y[k]) + nz * u.z[k]);
             }
-            // (a bound that is not finite, from coordinates that are not, proves nothing)
-            const double bound = size * margin;
-            reject = reject || (size > 0x1p-800 && bound < DBL_MAX && m - h >= bound);
+            // (size * Mp bounds every partial sum of the projections: where they, or
+            // the margin, might overflow, nothing is proven)
+            reject = reject || (size > 0x1p-800 && size * fmax(Mp, margin) < 0x1p1020 && m - h >= size * margin);
           }
         }
       }

@@ -84,6 +84,18 @@ def test_p1_blocks_match_oracle(gpu_ctx, oracle_mod, na, nb, ja, jb, scale):
     assert np.array_equal(blocks, ref.reshape(blocks.shape))
 
 
+@pytest.mark.parametrize("exponent", [-40, 300, 339, 340, 341, 342, 343, 344, 346, 352])
+def test_pairs_whose_projections_overflow(gpu_ctx, exponent):
+    """Explicit pairs at the scales where products of three coordinates leave
+    the range: the second early-out's projections then prove nothing."""
+    a, b = _pairs(4001, 12)
+    a, b = a * 2.0 ** exponent, b * 2.0 ** exponent
+    (m, k, _), (rm, rk, _) = gpu_ctx.intersect_pairs(3, a, b), _small(gpu_ctx, a, b)
+    assert (rk > 0).sum() > 100
+    assert np.array_equal(k, rk)
+    assert np.array_equal(m, rm, equal_nan=True)
+
+
 @pytest.mark.parametrize("exponent", [343, 344, 345, 348, 400, 500])
 def test_volumes_that_overflow(gpu_ctx, exponent):
     """Coordinates whose volumes' products overflow: a kept tet of NaN volume
