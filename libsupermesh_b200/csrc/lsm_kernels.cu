@@ -3327,8 +3327,10 @@ __global__ void __launch_bounds__(256, 2) k_pairs_early(int64_t n, const double*
       if (!reject && second) {
         double g, tau, MB;
         tet_screen_factors(u, P, g, tau, MB);
-        if (g < DBL_MAX) {  // B's planes bound a proper tet
-          const double Mp = fmax(M, MB);
+        // B's planes bound a proper tet, and no partial sum of a projection (at
+        // most 24 Mp^3) leaves the range
+        const double Mp = fmax(M, MB);
+        if (g < DBL_MAX && Mp < 0x1p330) {
           const double e = kEps + 128.0 * kEps * (1.0 + 2.0 * Mp);
           const double margin =
               1.01 * g * (tau + e) + 16.0 * kEps * (1.0 + Mp) + 128.0 * kEps * (1.0 + M);
@@ -3352,9 +3354,7 @@ __global__ void __launch_bounds__(256, 2) k_pairs_early(int64_t n, const double*
               h = fmax(h, (nx * t.x[k] + ny * t.y[k]) + nz * t.z[k]);
               m = fmin(m, (nx * u.x[k] + ny * u.y[k]) + nz * u.z[k]);
             }
-            // (size * Mp bounds every partial sum of the projections: where they, or
-            // the margin, might overflow, nothing is proven)
-            reject = reject || (size > 0x1p-800 && size * fmax(Mp, margin) < 0x1p1020 && m - h >= size * margin);
+            reject = reject || (size > 0x1p-800 && m - h >= size * margin);
           }
         }
       }
